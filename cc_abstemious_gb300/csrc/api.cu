@@ -209,12 +209,11 @@ void solve_surface_dense_fp64(Context& c, const Problem& p, const double2* d_rhs
     if (p.in.solver == 0) {
         c.w_flags.ensure(256);
         if (!reuse_lu) {
-            c.w_piv.ensure(sizeof(int32_t) * (size_t)n);
-            lu_factor_fp64(c, n, A, n, c.w_piv.as<int32_t>(), c.w_flags.as<int>() + 1);
+            c.w_piv.ensure(lu_aux_bytes(n));
+            lu_factor_fp64(c, n, A, n, c.w_piv.p, c.w_flags.as<int>() + 1);
         }
-        lu_solve_fp64(c, n, A, n, c.w_piv.as<int32_t>(), x);
-        int info = 0;
-        to_host(c, &info, c.w_flags.as<int>() + 1, sizeof(int));
+        lu_solve_fp64(c, n, A, n, c.w_piv.p, x);
+        const int info = lu_status(c);
         if (rep) rep->flag = 3;
         require(info == 0, "LU factorisation found a zero pivot (column " + std::to_string(info) + ")",
                 BEM_ERR_SINGULAR);
@@ -674,7 +673,7 @@ BEM_API bem_status bem_solve_lu(bem_ctx* ctx, int64_t n, const bem_cplx* A, int6
                                    mem == BEM_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                    c.stream));
         DevBuf piv, xb;
-        piv.ensure(sizeof(int32_t) * n);
+        piv.ensure(lu_aux_bytes(n));
         double2* dx;
         if (mem == BEM_MEM_DEVICE) dx = reinterpret_cast<double2*>(x);
         else {
@@ -682,10 +681,9 @@ BEM_API bem_status bem_solve_lu(bem_ctx* ctx, int64_t n, const bem_cplx* A, int6
             dx = xb.as<double2>();
         }
         c.w_flags.ensure(256);
-        lu_factor_fp64(c, n, W, n, piv.as<int32_t>(), c.w_flags.as<int>() + 1);
-        lu_solve_fp64(c, n, W, n, piv.as<int32_t>(), dx);
-        int info = 0;
-        to_host(c, &info, c.w_flags.as<int>() + 1, sizeof(int));
+        lu_factor_fp64(c, n, W, n, piv.p, c.w_flags.as<int>() + 1);
+        lu_solve_fp64(c, n, W, n, piv.p, dx);
+        const int info = lu_status(c);
         if (mem == BEM_MEM_HOST) to_host(c, x, dx, sizeof(double2) * n);
         require(info == 0, "LU factorisation found a zero pivot (column " + std::to_string(info) + ")",
                 BEM_ERR_SINGULAR);

@@ -224,7 +224,9 @@ struct Context {
     // every mixed solve)
     DevBuf w_gm, w_gmz, w_lu_F, w_lu_D, w_lu_W, w_lu_P, w_lu_H;
     DevBuf w_upload;  // mesh staging of problem construction
-    DevBuf w_piv;     // row pivots of the plain form's FP64 LU
+    DevBuf w_piv;     // the plain form's FP64 LU: row order, diagonal blocks' inverses
+    DevBuf w_lu64;    // its trailing update's digit images
+    int lu64_cluster = 0;  // largest cluster its panels run on (0: not asked yet)
     // results of the last bem_run
     std::vector<double> last_phi, last_vn;
     int64_t last_n = 0, last_nf = 0;
@@ -305,10 +307,16 @@ struct IncItem {
 void incident_batch(Context& ctx, const std::vector<IncItem>& items);
 void incident_field(Context& ctx, const Problem& p, double2* out);
 
+// Dense LU (lu64.cu): A is overwritten by its factors, `aux` (lu_aux_bytes(n)
+// bytes) receives what the substitutions need beside them; d_info, the word after
+// the device error word in w_flags, the first zero pivot's column + 1.
+size_t lu_aux_bytes(int64_t n);
+void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux, int* d_info);
+void lu_solve_fp64(Context& ctx, int64_t n, const double2* A, int64_t lda, const void* aux, double2* b);
+// Waits for the calls above; throws on a device error, returns d_info.
+int lu_status(Context& ctx);
+
 // Dense linear algebra (dense.cu)
-void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, int32_t* d_piv, int* d_info);
-void lu_solve_fp64(Context& ctx, int64_t n, const double2* A, int64_t lda, const int32_t* d_piv,
-                   double2* b);
 void gemv_fp64(Context& ctx, int64_t m, int64_t n, const double2* A, int64_t lda, const double2* x,
                double2* y, cd alpha, cd beta);
 double frob_norm_fp64(Context& ctx, int64_t m, int64_t n, const double2* A, int64_t lda);

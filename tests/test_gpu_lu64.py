@@ -1,0 +1,77 @@
+"""The FP64 LU (csrc/lu64.cu) at the sizes where its tiles, panels and clusters
+end: blocks of 32 columns, clusters of up to 16 CTAs with 32 rows each, narrower
+panels above 1024 rows, row blocks and column tiles of 64.
+
+The measure is the normwise backward error ||A x - b|| / (||A||_F ||x||), which
+for partial pivoting is at most a small multiple of n u (u = 2^-53); the bound
+below is 16 (n + 8) u, fixed beforehand (complex products count for 2 sqrt 2, the
+growth of random matrices for about n^(1/4))."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+bem = pytest.importorskip("cc_abstemious_gb300")
+U = 2.0 ** -53
+
+
+def matrix(n, seed, kind="plain"):
+    rng = np.random.default_rng(seed)
+    A = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    if kind == "graded":  # rows and columns over many orders of magnitude
+        A = 10.0 ** rng.uniform(-6, 6, n)[:, None] * A * 10.0 ** rng.uniform(-3, 3, n)[None, :]
+    elif kind == "tiny":  # products outside the range of normal numbers
+        A = A * 1e-160
+    elif kind == "pivots":  # every pivot is the last row
+        A = A + 1e3 * np.eye(n)[::-1]
+    return A, rng.normal(size=n) + 1j * rng.normal(size=n)
+
+
+def backward(A, x, b):
+    return np.linalg.norm(A @ x - b) / (np.linalg.norm(A) * np.linalg.norm(x))
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 95, 97, 127, 129, 161, 255, 257, 511, 513, 545, 1023,
+                               1025, 1057, 1217, 2433])
+def test_sizes(n):
+    A, b = matrix(n, n)
+    assert backward(A, bem.solve_lu(A, b), b) <= 16 * (n + 8) * U
+
+
+@pytest.mark.parametrize("kind", ["graded", "tiny", "pivots"])
+@pytest.mark.parametrize("n", [33, 97, 300, 1100])
+def test_scales_and_exchanges(n, kind):
+    A, b = matrix(n, 7 * n, kind)
+    s = 1.0 if kind != "tiny" else 1e160
+    x = bem.solve_lu(A, b * (1e-160 if kind == "tiny" else 1.0))
+    assert backward(A * s, x, b) <= 16 * (n + 8) * U
+
+
+def test_graded_rows_keep_their_digits():
+    """Row by row: a row scaled by 1e-9 has the residual of its own scale."""
+    A, b = matrix(300, 3)
+    d = 10.0 ** np.random.default_rng(4).uniform(-9, 0, 300)
+    x = bem.solve_lu(d[:, None] * A, d * b)
+    r = np.abs(A @ x - b) / (np.linalg.norm(A, axis=1) * np.linalg.norm(x))
+    assert r.max() <= 16 * 308 * U
+
+
+def test_zero_pivot_is_singular_and_nothing_sticks():
+    A, b = matrix(200, 1)
+    A[:, 77] = 0
+    with pytest.raises(bem.BemError):
+        bem.solve_lu(A, b)
+    A, b = matrix(200, 1)
+    assert backward(A, bem.solve_lu(A, b), b) <= 16 * 208 * U
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_non_finite_entries_end_in_non_finite_results(value):
+    A, b = matrix(150, 2)
+    A[140, 3] = value
+    try:
+        x = bem.solve_lu(A, b)
+    except bem.BemError:
+        return
+    assert not np.all(np.isfinite(x))
+    A, b = matrix(150, 2)
+    assert backward(A, bem.solve_lu(A, b), b) <= 16 * 158 * U
