@@ -17,36 +17,6 @@
 
 namespace bem {
 
-// influence_matrix.rs:12-37.  (x, e_x): source point and its normal; (y, e_y):
-// observation point and its normal.  Returns g and h without the wt*area scale.
-__device__ __forceinline__ void greens64(double k, int bm, double beta_im, double xx, double xy, double xz,
-                                         double exx, double exy, double exz, double yx, double yy, double yz,
-                                         double eyx, double eyy, double eyz, z2& g, z2& h) {
-    double rx = xx - yx, ry = xy - yy, rz = xz - yz;
-    double r = sqrt(rx * rx + ry * ry + rz * rz);
-    double inv = 1.0 / r;
-    double erx = rx * inv, ery = ry * inv, erz = rz * inv;
-    double s, c;
-    sincos(k * r, &s, &c);
-    double q = inv * (1.0 / (4.0 * PI_D));
-    g = make_double2(c * q, s * q);
-    z2 f1 = make_double2(-inv, k);
-    double rdoty = erx * eyx + ery * eyy + erz * eyz;
-    z2 gf1 = cmul(g, f1);
-    h = cscale(gf1, -rdoty);
-    if (bm) {
-        double rdotx = erx * exx + ery * exy + erz * exz;
-        double nxy = eyx * exx + eyy * exy + eyz * exz;
-        z2 dg = cscale(gf1, rdotx);
-        z2 t1 = cscale(cneg(f1), nxy);
-        z2 t2 = cscale(cscale(make_double2(k * k * r + 3.0 * f1.x, 3.0 * f1.y), rdotx), rdoty);
-        z2 dh = cmul(cscale(g, inv), csub(t1, t2));
-        // beta = i * beta_im
-        g = cadd(g, make_double2(-beta_im * dg.y, beta_im * dg.x));
-        h = cadd(h, make_double2(-beta_im * dh.y, beta_im * dh.x));
-    }
-}
-
 struct TileGeo64 {
     // columns: x y z ex ey ez wa area wt ; rows: x y z ex ey ez
     double cx[TILE], cy[TILE], cz[TILE], cex[TILE], cey[TILE], cez[TILE], cwa[TILE], carea[TILE], cwt[TILE];
@@ -77,7 +47,12 @@ __device__ __forceinline__ bool stage_tile64(TileGeo64& t, uint64_t* bar, const 
 // MODE 0: write H and G (get_dense_surface_matrices).
 // MODE 1: write A = alpha H + beta G; optional per-column-tile partial row sums
 //         of gamma H + delta G (the uniform-BC right-hand side of solve.rs:35-69).
-template <int MODE>
+// A = alpha H + beta G skips the products with alpha = 1 and beta = 0.
+// Bound by the FP64 pipe (two multiply-adds per clock and SM): 45 FP64
+// instructions per Burton-Miller pair in MODE 0 against about 115 with root,
+// phase, sine and cosine on that pipe.  4002 triangles, both matrices: 2.82 ->
+// 1.22 ms; 6144 quads, one operator: 6.87 -> 3.31 ms.
+template <int MODE, bool BM>
 __global__ void __launch_bounds__(ASM_THREADS) assemble64_kernel(
     int64_t n, int64_t npad, const double* __restrict__ geo, KParams kp, double2* __restrict__ H,
     double2* __restrict__ G, int64_t ld, z2 alpha, z2 beta, z2 gamma, z2 delta, double2* __restrict__ part,
@@ -91,6 +66,10 @@ __global__ void __launch_bounds__(ASM_THREADS) assemble64_kernel(
         mbar_wait_bounded(&bar, 0);
         return;
     }
+    // the weights of the columns carry the kernel's 1 / (4 pi)
+    if (threadIdx.x < TILE) t.cwa[threadIdx.x] *= 1.0 / (4.0 * PI_D);
+    __syncthreads();
+    const bool alpha_one = alpha.x == 1.0 && alpha.y == 0.0, beta_zero = beta.x == 0.0 && beta.y == 0.0;
     const int tx = threadIdx.x & (TILE - 1), ty = threadIdx.x >> 6;
     const int64_t i = I0 + tx;
     const double yx = t.rx[tx], yy = t.ry[tx], yz = t.rz[tx];
@@ -104,19 +83,16 @@ __global__ void __launch_bounds__(ASM_THREADS) assemble64_kernel(
         if (i == j) {
             self_term64(t.carea[jj], t.cwt[jj], kp.bm, kp.beta_im, kp.hdiag, kp.gdiag_im, g, h);
         } else {
-            greens64(kp.k, kp.bm, kp.beta_im, t.cx[jj], t.cy[jj], t.cz[jj], t.cex[jj], t.cey[jj], t.cez[jj], yx, yy,
-                     yz, eyx, eyy, eyz, g, h);
-            double wa = t.cwa[jj];
-            g = cscale(g, wa);
-            h = cscale(h, wa);
+            pair64<BM>(kp, t.cwa[jj], t.cx[jj] - yx, t.cy[jj] - yy, t.cz[jj] - yz, eyx, eyy, eyz,
+                       t.cex[jj], t.cey[jj], t.cez[jj], g, h);
         }
         if (i < n && j < n) {
             if (MODE == 0) {
                 H[j * ld + i] = h;
                 G[j * ld + i] = g;
             } else {
-                z2 a = cmul(alpha, h);
-                cfma(a, beta, g);
+                z2 a = alpha_one ? h : cmul(alpha, h);
+                if (!beta_zero) cfma(a, beta, g);
                 H[j * ld + i] = a;
                 if (part) {
                     cfma(acc, gamma, h);
@@ -171,8 +147,10 @@ void assemble_surface_fp64(Context& ctx, const Problem& p, double2* H, double2* 
     BEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx.stream));
     dim3 grid((unsigned)(p.geo.npad / TILE), (unsigned)(p.geo.npad / TILE));
     z2 zero = make_double2(0, 0);
-    assemble64_kernel<0><<<grid, ASM_THREADS, 0, ctx.stream>>>(p.n, p.geo.npad, p.geo.arr(0), kparams(p), H, G, ld,
-                                                              zero, zero, zero, zero, nullptr, err);
+    const KParams kp = kparams(p);
+    auto kernel = kp.bm ? assemble64_kernel<0, true> : assemble64_kernel<0, false>;
+    kernel<<<grid, ASM_THREADS, 0, ctx.stream>>>(p.n, p.geo.npad, p.geo.arr(0), kp, H, G, ld, zero, zero, zero, zero,
+                                                 nullptr, err);
     BEM_CHECK_LAUNCH(&ctx);
     check_device_err(ctx);
 }
@@ -188,8 +166,10 @@ void assemble_system_fp64(Context& ctx, const Problem& p, double2* A, int64_t ld
         part = ctx.w_part.as<double2>();
     }
     dim3 grid((unsigned)ntiles, (unsigned)ntiles);
-    assemble64_kernel<1><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-        p.n, p.geo.npad, p.geo.arr(0), kparams(p), A, nullptr, ld, make_double2(alpha.re, alpha.im),
+    const KParams kp = kparams(p);
+    auto kernel = kp.bm ? assemble64_kernel<1, true> : assemble64_kernel<1, false>;
+    kernel<<<grid, ASM_THREADS, 0, ctx.stream>>>(
+        p.n, p.geo.npad, p.geo.arr(0), kp, A, nullptr, ld, make_double2(alpha.re, alpha.im),
         make_double2(beta.re, beta.im), make_double2(gamma.re, gamma.im), make_double2(delta.re, delta.im), part, err);
     BEM_CHECK_LAUNCH(&ctx);
     if (rowsum) {
@@ -219,12 +199,7 @@ __global__ void row_or_column_kernel(int64_t npad, const double* __restrict__ ge
             g.y += kp.gdiag_im;
         }
     } else {
-        greens64(kp.k, kp.bm, kp.beta_im, geo[GX * npad + j], geo[GY * npad + j], geo[GZ * npad + j],
-                 geo[GEX * npad + j], geo[GEY * npad + j], geo[GEZ * npad + j], geo[GX * npad + i], geo[GY * npad + i],
-                 geo[GZ * npad + i], geo[GEX * npad + i], geo[GEY * npad + i], geo[GEZ * npad + i], g, h);
-        double wa = geo[GWA * npad + j];
-        g = cscale(g, wa);
-        h = cscale(h, wa);
+        pair64_at(kp, npad, geo, i, j, g, h);
     }
     z2 a = cmul(beta, g);
     cfma(a, alpha, h);
@@ -247,45 +222,56 @@ void row_or_column(Context& ctx, const Problem& p, const int64_t* dI, int64_t ni
 // Field matrices (influence_matrix.rs:101-127): classical kernel, the field
 // point as x and the element as y with its normal.  M, L are nfp x n.
 __global__ void field_matrices_kernel(int64_t nfp, int64_t fpad, const double* __restrict__ fp, int64_t n,
-                                      int64_t npad, const double* __restrict__ geo, double k,
+                                      int64_t npad, const double* __restrict__ geo, KParams kp,
                                       double2* __restrict__ M, double2* __restrict__ L, int64_t ld) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t j = blockIdx.y;
     if (i >= nfp) return;
     z2 g, h;
-    greens64(k, 0, 0.0, fp[i], fp[fpad + i], fp[2 * fpad + i], 0, 0, 0, geo[GX * npad + j], geo[GY * npad + j],
-             geo[GZ * npad + j], geo[GEX * npad + j], geo[GEY * npad + j], geo[GEZ * npad + j], g, h);
-    double wa = geo[GWA * npad + j];
-    M[j * ld + i] = cscale(h, wa);
-    L[j * ld + i] = cscale(g, wa);
+    pair64<false>(kp, geo[GWA * npad + j] * (1.0 / (4.0 * PI_D)), fp[i] - geo[GX * npad + j],
+                  fp[fpad + i] - geo[GY * npad + j], fp[2 * fpad + i] - geo[GZ * npad + j], geo[GEX * npad + j],
+                  geo[GEY * npad + j], geo[GEZ * npad + j], 0, 0, 0, g, h);
+    M[j * ld + i] = h;
+    L[j * ld + i] = g;
 }
 
 void field_matrices_fp64(Context& ctx, const Problem& p, double2* M, double2* L, int64_t ld) {
     if (p.nfp == 0) return;
     dim3 grid((unsigned)((p.nfp + 127) / 128), (unsigned)p.n);
     field_matrices_kernel<<<grid, 128, 0, ctx.stream>>>(p.nfp, p.nfp_pad, p.d_fp.as<double>(), p.n, p.geo.npad,
-                                                       p.geo.arr(0), p.wavenumber(), M, L, ld);
+                                                       p.geo.arr(0), kparams(p), M, L, ld);
     BEM_CHECK_LAUNCH(&ctx);
 }
 
 // Fused field evaluation: out_i = [inc_i] - sum_j M_ij phi_j + sum_j L_ij vn_j
 // without storing M and L.  One CTA per field point, fixed-order reduction.
+// A term is g (vn - c (1 / r - i k) phi) with g the Green's function and c the
+// direction cosine: 23 FP64 instructions against 33 with M and L formed and
+// about 95 with the phase and the root on the FP64 pipe too.  6144 elements x
+// 20000 points: 16.1 ms so, 6.0 ms with pair64, 5.3 ms now, bound by that pipe.
 constexpr int FIELD_THREADS = 256;
 __global__ void __launch_bounds__(FIELD_THREADS) evaluate_field_kernel(
     int64_t nfp, int64_t fpad, const double* __restrict__ fp, int64_t n, int64_t npad,
-    const double* __restrict__ geo, double k, const double2* __restrict__ phi, const double2* __restrict__ vn,
+    const double* __restrict__ geo, KParams kp, const double2* __restrict__ phi, const double2* __restrict__ vn,
     const double2* __restrict__ inc, double2* __restrict__ out) {
     __shared__ z2 red[FIELD_THREADS];
     int64_t i = blockIdx.x;
-    double px = fp[i], py = fp[fpad + i], pz = fp[2 * fpad + i];
+    const double px = fp[i], py = fp[fpad + i], pz = fp[2 * fpad + i];
     z2 acc = make_double2(0, 0);
     for (int64_t j = threadIdx.x; j < n; j += FIELD_THREADS) {
-        z2 g, h;
-        greens64(k, 0, 0.0, px, py, pz, 0, 0, 0, geo[GX * npad + j], geo[GY * npad + j], geo[GZ * npad + j],
-                 geo[GEX * npad + j], geo[GEY * npad + j], geo[GEZ * npad + j], g, h);
-        double wa = geo[GWA * npad + j];
-        cfma(acc, cscale(h, -wa), phi[j]);
-        cfma(acc, cscale(g, wa), vn[j]);
+        const double dx = px - geo[GX * npad + j], dy = py - geo[GY * npad + j], dz = pz - geo[GZ * npad + j];
+        double inv, r, c, s;
+        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        if (!wave_int(r2, kp.turn, kp.turn_exp, inv, r, c, s)) {
+            root64(r2, inv, r);
+            phase64(kp.k, r, c, s);
+        }
+        const double q = inv * geo[GWA * npad + j];
+        const double cy =
+            fma(dx, geo[GEX * npad + j], fma(dy, geo[GEY * npad + j], dz * geo[GEZ * npad + j])) * inv;
+        const z2 f = phi[j], v = vn[j], e = make_double2(cy * inv, -(cy * kp.k));
+        const z2 w = make_double2(fma(-e.x, f.x, fma(e.y, f.y, v.x)), fma(-e.x, f.y, fma(-e.y, f.x, v.y)));
+        cfma(acc, make_double2(c * q, s * q), w);
     }
     red[threadIdx.x] = acc;
     __syncthreads();
@@ -293,14 +279,17 @@ __global__ void __launch_bounds__(FIELD_THREADS) evaluate_field_kernel(
         if (threadIdx.x < s) red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + s]);
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[i] = inc ? cadd(inc[i], red[0]) : red[0];
+    if (threadIdx.x == 0) {
+        const z2 v = cscale(red[0], 1.0 / (4.0 * PI_D));  // (left out of every weight)
+        out[i] = inc ? cadd(inc[i], v) : v;
+    }
 }
 
 void evaluate_field(Context& ctx, const Problem& p, const double2* phi, const double2* vn, const double2* inc,
                     double2* out) {
     if (p.nfp == 0) return;
     evaluate_field_kernel<<<(unsigned)p.nfp, FIELD_THREADS, 0, ctx.stream>>>(
-        p.nfp, p.nfp_pad, p.d_fp.as<double>(), p.n, p.geo.npad, p.geo.arr(0), p.wavenumber(), phi, vn, inc, out);
+        p.nfp, p.nfp_pad, p.d_fp.as<double>(), p.n, p.geo.npad, p.geo.arr(0), kparams(p), phi, vn, inc, out);
     BEM_CHECK_LAUNCH(&ctx);
 }
 

@@ -248,6 +248,8 @@ struct KParams {
     int bm;          // Burton-Miller
     double hdiag;    // -0.5 exterior, 0 interior
     double gdiag_im; // BM: 0.5/k
+    unsigned long long turn;  // k / (2 pi) = turn 2^(turn_exp - 64), the top bit set
+    int turn_exp;
 };
 KParams kparams(const Problem& p);
 void lhs_factors(const Problem& p, cd& a, cd& b);

@@ -189,6 +189,20 @@ KParams kparams(const Problem& p) {
     kp.beta_im = kp.bm ? 1.0 / kp.k : 0.0;   // preprocess.rs:58 beta = i/k
     kp.hdiag = p.in.problem_type == 1 ? -0.5 : 0.0;  // preprocess.rs:60-66
     kp.gdiag_im = kp.bm ? 0.5 * (1.0 / kp.k) : 0.0;  // preprocess.rs:68-74
+    // k / (2 pi) to 64 bits (long double has at least 64 on x86-64 and aarch64);
+    // an exponent out of every range where there is no such number
+    kp.turn = 0;
+    kp.turn_exp = 1 << 20;
+    const long double turns = (long double)kp.k / 6.28318530717958647692528676655900577L;
+    if (std::isfinite(kp.k) && kp.k > 0) {
+        int e = 0;
+        const long double m = std::frexp(turns, &e);
+        const long double t = std::ldexp(m, 64);
+        if (t < 18446744073709551615.0L) {
+            kp.turn = (unsigned long long)t;
+            kp.turn_exp = e;
+        }
+    }
     return kp;
 }
 
