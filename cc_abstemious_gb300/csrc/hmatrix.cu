@@ -67,35 +67,7 @@ __device__ __forceinline__ z2 gen_entry(const GenParams& g, int64_t i, int64_t j
     if (i == j) {
         self_term64(geo[GAREA * np + j], geo[GWT * np + j], g.kp.bm, g.kp.beta_im, g.kp.hdiag, g.kp.gdiag_im, gg, hh);
     } else {
-        // source x = element j, observation y = collocation point i
-        double rx = geo[GX * np + j] - geo[GX * np + i], ry = geo[GY * np + j] - geo[GY * np + i],
-               rz = geo[GZ * np + j] - geo[GZ * np + i];
-        double r = sqrt(rx * rx + ry * ry + rz * rz);
-        double inv = 1.0 / r;
-        double erx = rx * inv, ery = ry * inv, erz = rz * inv;
-        double s, c;
-        sincos(g.kp.k * r, &s, &c);
-        double q = inv * (1.0 / (4.0 * PI_D));
-        gg = make_double2(c * q, s * q);
-        z2 f1 = make_double2(-inv, g.kp.k);
-        double eyx = geo[GEX * np + i], eyy = geo[GEY * np + i], eyz = geo[GEZ * np + i];
-        double rdoty = erx * eyx + ery * eyy + erz * eyz;
-        z2 gf1 = cmul(gg, f1);
-        hh = cscale(gf1, -rdoty);
-        if (g.kp.bm) {
-            double exx = geo[GEX * np + j], exy = geo[GEY * np + j], exz = geo[GEZ * np + j];
-            double rdotx = erx * exx + ery * exy + erz * exz;
-            double nxy = eyx * exx + eyy * exy + eyz * exz;
-            z2 dg = cscale(gf1, rdotx);
-            z2 t1 = cscale(cneg(f1), nxy);
-            z2 t2 = cscale(cscale(make_double2(g.kp.k * g.kp.k * r + 3.0 * f1.x, 3.0 * f1.y), rdotx), rdoty);
-            z2 dh = cmul(cscale(gg, inv), csub(t1, t2));
-            gg = cadd(gg, make_double2(-g.kp.beta_im * dg.y, g.kp.beta_im * dg.x));
-            hh = cadd(hh, make_double2(-g.kp.beta_im * dh.y, g.kp.beta_im * dh.x));
-        }
-        double wa = geo[GWA * np + j];
-        gg = cscale(gg, wa);
-        hh = cscale(hh, wa);
+        pair64_at(g.kp, np, geo, i, j, gg, hh);
     }
     z2 a = cmul(g.beta, gg);
     cfma(a, g.alpha, hh);
@@ -190,12 +162,26 @@ __device__ __forceinline__ z2 bsum2(z2 v, double* sh) {
 }
 
 // Sum of a complex value over the 32 lanes of a warp (every lane gets it).
+// The parts part ways in the first step: five FP64 additions, not ten (each
+// occupies the FP64 pipe of the SM quarter for 65 clocks).
 __device__ __forceinline__ z2 wsum2(z2 v) {
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-    return v;
+    const bool odd = threadIdx.x & 1;
+    double s = odd ? v.y : v.x;
+    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+    for (int o = 2; o <= 16; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return make_double2(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 1));
+}
+// Two complex values at once: six additions.
+__device__ __forceinline__ void wsum4(z2& a, z2& b) {
+    const bool odd = threadIdx.x & 1, up = threadIdx.x & 2;
+    double x = odd ? a.y : a.x, y = odd ? b.y : b.x;
+    x += __shfl_xor_sync(0xffffffffu, odd ? a.x : a.y, 1);
+    y += __shfl_xor_sync(0xffffffffu, odd ? b.x : b.y, 1);
+    double s = up ? y : x;
+    s += __shfl_xor_sync(0xffffffffu, up ? x : y, 2);
+    for (int o = 4; o <= 16; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    a = make_double2(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 1));
+    b = make_double2(__shfl_sync(0xffffffffu, s, 2), __shfl_sync(0xffffffffu, s, 3));
 }
 
 __device__ __forceinline__ double wsum(double v) {
@@ -204,12 +190,33 @@ __device__ __forceinline__ double wsum(double v) {
 }
 
 // argmax of |v[t]| over t not excluded; first index wins ties (aca.rs:256-268).
+// Moduli (hypot, about 25 FP64 instructions) only of the entries whose square
+// is within a few rounding errors of the largest square, which decides the
+// others.
 __device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t len, double* sh, int64_t* shi) {
+    const long long inf = 0x7ff0000000000000ll;
+    auto square = [&](int64_t t) {  // as the bits of a non-negative double; -1: excluded or NaN
+        if (excl[t]) return -1ll;
+        const long long k = __double_as_longlong(cnorm2(v[t]));
+        return k > inf ? -1ll : k;
+    };
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    long long top = -1;
+    for (int64_t t = threadIdx.x; t < len; t += blockDim.x) top = max(top, square(t));
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    __syncthreads();
+    if (l == 0) shi[w] = top;
+    __syncthreads();
+    top = l < nw ? (long long)shi[l] : -1ll;
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    // 2^-47 below the largest (zero where squares underflow: every entry)
+    const long long floor_ = top < 0 ? 0 : top < (64ll << 52) ? 0 : top == inf ? inf : top - 64;
     double best = -1.0;
     int64_t bi = len;
     for (int64_t t = threadIdx.x; t < len; t += blockDim.x) {
-        if (excl[t]) continue;
-        double a = hypot(v[t].x, v[t].y);
+        const long long k = square(t);
+        if (k < 0 || k < floor_) continue;
+        const double a = hypot(v[t].x, v[t].y);
         if (best < a) { best = a; bi = t; }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -217,12 +224,10 @@ __device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t le
         int64_t oi = __shfl_down_sync(0xffffffffu, bi, o);
         if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
     }
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     __syncthreads();
     if (l == 0) { sh[w] = best; shi[w] = bi; }
     __syncthreads();
     if (w == 0) {
-        int nw = blockDim.x >> 5;
         best = l < nw ? sh[l] : -1.0;
         bi = l < nw ? shi[l] : len;
         for (int o = 16; o > 0; o >>= 1) {
@@ -237,6 +242,7 @@ __device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t le
 }
 
 constexpr int LEAF_THREADS = 256;
+constexpr int JACOBI_SMEM = 32;  // ranks up to this run the Jacobi sweeps in shared memory
 
 // Dense (inadmissible) leaves: one CTA per leaf, entries column-major m x n.
 __global__ void __launch_bounds__(LEAF_THREADS) hm_dense_fill_kernel(const HLeaf* __restrict__ leaves,
@@ -282,7 +288,7 @@ __device__ __forceinline__ double bnsq(const double2* a, int64_t len, double* sh
 }
 
 // Partially pivoted ACA (aca.rs:57-136) of every admissible leaf.
-__global__ void __launch_bounds__(LEAF_THREADS) hm_aca_kernel(HLeaf* __restrict__ leaves,
+__global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restrict__ leaves,
                                                               const int32_t* __restrict__ list,
                                                               const int64_t* __restrict__ rows,
                                                               const int64_t* __restrict__ cols, GenParams g,
@@ -432,139 +438,165 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_aca_kernel(HLeaf* __restrict_
 // one-sided Jacobi, truncation at s < tol * cumulative sum (+1, at least 1),
 // then U <- Q_u W Sigma and V <- Q_v Z with Z = (V^H)^T (plain transpose, the
 // factors pair as u v^T).
-__device__ void house_qr_dev(double2* A, int64_t m, int r, double2* R, double2* tau, double* sh) {
-    // A: m x r column-major; on exit the reflectors v_k (v_k[k] = 1 implied
-    // by storing the full vector) are kept in A below and on the diagonal.
-    // Column k's reflector comes from two block reductions; its application
-    // to the later columns runs one warp per column (warp reductions, one
-    // barrier per k).
+__device__ void house_qr_dev(double2* A, int64_t m, int r, double2* R, double2* tau) {
+    // A: m x r column-major; on exit the reflectors v_k = x - alpha e_k are
+    // kept in A below and on the diagonal.  Warp 0 forms column k's reflector
+    // (|v_k|^2 = 2 |x| (|x| + |x_0|), no second reduction), every warp applies
+    // it to its share of the later columns: two barriers per k.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __shared__ double2 s_alpha, s_tau;
+    __shared__ double s_tau;
     for (int k = 0; k < r; ++k) {
         double2* a = A + (size_t)k * m;
-        double nx2 = 0;
-        for (int64_t i = k + threadIdx.x; i < m; i += blockDim.x) nx2 += cnorm2(a[i]);
-        double nx = sqrt(bsum(nx2, sh));
-        if (threadIdx.x == 0) {
-            z2 x0 = a[k];
-            double ax0 = hypot(x0.x, x0.y);
-            z2 ph = ax0 == 0 ? make_double2(1.0, 0.0) : make_double2(x0.x / ax0, x0.y / ax0);
-            s_alpha = cscale(cneg(ph), nx);
+        if (warp == 0) {
+            const z2 x0 = a[k];
+            double nx2 = 0;
+            for (int64_t i = k + lane; i < m; i += 32) nx2 = fma(a[i].x, a[i].x, fma(a[i].y, a[i].y, nx2));
+            const double nx = sqrt(wsum(nx2)), ax0 = sqrt(cnorm2(x0));
+            const double inv0 = ax0 == 0 ? 0.0 : 1.0 / ax0;
+            const z2 ph = ax0 == 0 ? make_double2(1.0, 0.0) : make_double2(x0.x * inv0, x0.y * inv0);
+            const z2 alpha = make_double2(-ph.x * nx, -ph.y * nx);
+            const double half = nx * (nx + ax0), tk = half == 0 ? 0.0 : 1.0 / half;
+            __syncwarp();
+            if (lane == 0) {
+                a[k] = csub(x0, alpha);
+                R[(size_t)k * r + k] = alpha;
+                tau[k] = make_double2(tk, 0.0);
+                s_tau = tk;
+            }
         }
         __syncthreads();
-        // v = x - alpha e_k (stored in a[k..m))
-        if (threadIdx.x == 0) a[k] = csub(a[k], s_alpha);
-        __syncthreads();
-        double vn2 = 0;
-        for (int64_t i = k + threadIdx.x; i < m; i += blockDim.x) vn2 += cnorm2(a[i]);
-        vn2 = bsum(vn2, sh);
-        if (threadIdx.x == 0) s_tau = make_double2(vn2 == 0 ? 0.0 : 2.0 / vn2, 0.0);
-        __syncthreads();
-        const double tk = s_tau.x;
-        // apply H_k to columns j > k, one warp per column
+        const double tk = s_tau;
         for (int j = k + 1 + warp; j < r; j += nw) {
             double2* c = A + (size_t)j * m;
             z2 d = make_double2(0, 0);
             for (int64_t i = k + lane; i < m; i += 32) cfma(d, cconj(a[i]), c[i]);
-            d = cscale(wsum2(d), tk);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(c[i], cneg(a[i]), d);
+            d = cscale(wsum2(d), -tk);
+            for (int64_t i = k + lane; i < m; i += 32) cfma(c[i], a[i], d);
         }
-        if (threadIdx.x == 0) tau[k] = make_double2(tk, 0.0);
-        for (int i = threadIdx.x; i < r; i += blockDim.x)
-            R[(size_t)k * r + i] = i == k ? s_alpha : make_double2(0, 0);
         __syncthreads();
     }
-    // R above the diagonal lives in rows < k of columns k (read after the loop)
-    for (int j = 0; j < r; ++j)
-        for (int i = threadIdx.x; i < j; i += blockDim.x) R[(size_t)j * r + i] = A[(size_t)j * m + i];
+    // R above the diagonal lives in rows < k of columns k
+    for (int t = threadIdx.x; t < r * r; t += blockDim.x) {
+        const int i = t % r, j = t / r;
+        if (i != j) R[t] = i < j ? A[(size_t)j * m + i] : make_double2(0, 0);
+    }
     __syncthreads();
 }
 
-// out (m x c) = Q [B; 0] where Q = H_0 ... H_{r-1} (reflectors in A), B r x c;
-// one warp per output column for each reflector.
+// out (m x c) = Q [B; 0] where Q = H_0 ... H_{r-1} (reflectors in A), B r x c.
+// A warp carries its columns through all reflectors; the columns do not meet.
 __device__ void house_apply_dev(const double2* A, int64_t m, int r, const double2* tau, const double2* B, int c,
-                                double2* out, double* sh) {
-    (void)sh;
+                                double2* out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int j = 0; j < c; ++j)
-        for (int64_t i = threadIdx.x; i < m; i += blockDim.x)
-            out[(size_t)j * m + i] = i < r ? B[(size_t)j * r + i] : make_double2(0, 0);
-    __syncthreads();
-    for (int k = r - 1; k >= 0; --k) {
-        const double2* v = A + (size_t)k * m;
-        const double tk = tau[k].x;
-        if (tk == 0.0) continue;
-        for (int j = warp; j < c; j += nw) {
-            double2* o = out + (size_t)j * m;
+    for (int j = warp; j < c; j += nw) {
+        double2* o = out + (size_t)j * m;
+        for (int64_t i = lane; i < m; i += 32) o[i] = i < r ? B[(size_t)j * r + i] : make_double2(0, 0);
+        __syncwarp();
+        for (int k = r - 1; k >= 0; --k) {
+            const double2* v = A + (size_t)k * m;
+            const double tk = tau[k].x;
+            if (tk == 0.0) continue;
             z2 d = make_double2(0, 0);
             for (int64_t i = k + lane; i < m; i += 32) cfma(d, cconj(v[i]), o[i]);
-            d = cscale(wsum2(d), tk);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(o[i], cneg(v[i]), d);
+            d = cscale(wsum2(d), -tk);
+            for (int64_t i = k + lane; i < m; i += 32) cfma(o[i], v[i], d);
+            __syncwarp();
         }
-        __syncthreads();
     }
+    __syncthreads();
 }
 
-// One-sided Jacobi SVD of the r x r matrix M (overwritten): M = W S Vh with S
-// descending.  Each sweep visits every column pair once in the round-robin
-// order: r' - 1 steps (r' = r rounded up to even) of r' / 2 disjoint pairs,
-// one warp per pair, one barrier per step.
-__device__ void jacobi_svd_dev(double2* M, double2* Vm, int r, double* S, int* perm, double* sh) {
-    (void)sh;
+// One-sided Jacobi on the columns of the r x r matrix M (overwritten by W Sigma):
+// each sweep visits every column pair once in the round-robin order, r' - 1
+// steps (r' = r rounded up to even) of r' / 2 disjoint pairs, until a sweep
+// finds no pair further than 1e-15 from orthogonal.
+//
+// Bound by FP64 issue (65 clocks per warp instruction however few lanes are
+// active), so a pair takes only as many lanes as fill the warps (16 columns:
+// one warp, four lanes per pair) and the rotation's angle comes from FP32: it
+// only has to be near, the next sweep corrects it; what is kept to FP64 is that
+// the rotation is unitary (its cosine and the phase, each one FP32 seed and a
+// third-order correction).  The right factor is not accumulated; the caller
+// forms it from W Sigma and the original matrix.  2560 triangles, leaf 32, eta 4:
+// the whole recompression 24.7 -> 7.8 ms, with the QR's reflectors formed by one
+// warp and the reductions' additions halved.
+// 1 / sqrt(v) for 0 < v (normal numbers).
+__device__ __forceinline__ double near_rsqrt(double v) {
+    const int e = (((__double2hiint(v) >> 20) & 0x7ff) - 1023) & ~1;  // even
+    const double s = wide(rsqrtf(near_float(v, e))) * __hiloint2double((1023 - e / 2) << 20, 0);
+    const double c = fma(-(v * s), s, 1.0);
+    return fma(s * c, fma(0.375, c, 0.5), s);
+}
+
+__device__ void jacobi_dev(double2* M, int r, double* S, int* perm) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int j = 0; j < r; ++j)
-        for (int i = threadIdx.x; i < r; i += blockDim.x) Vm[(size_t)j * r + i] = make_double2(i == j, 0.0);
-    __syncthreads();
-    __shared__ unsigned long long s_off;  // largest |cos angle| of a sweep, as the bits of a positive double
-    const int rr = r + (r & 1);           // players of the round robin (index r: a bye when r is odd)
-    for (int sweep = 0; sweep < 60; ++sweep) {
-        if (threadIdx.x == 0) s_off = 0ull;
-        __syncthreads();
-        for (int step = 0; step < rr - 1; ++step) {
-            for (int pi = warp; pi < rr / 2; pi += nw) {
-                // circle method: player 0 fixed, the others rotate by `step`
-                const int a0 = pi == 0 ? 0 : 1 + (pi - 1 + step) % (rr - 1);
-                const int b0 = 1 + (rr - 2 - pi + step) % (rr - 1);
-                const int p = min(a0, b0), q = max(a0, b0);
-                if (q >= r) continue;  // the bye
-                double2* up = M + (size_t)p * r;
-                double2* uq = M + (size_t)q * r;
-                double a = 0, b = 0;
-                z2 cc = make_double2(0, 0);
-                for (int i = lane; i < r; i += 32) {
-                    a += cnorm2(up[i]);
-                    b += cnorm2(uq[i]);
-                    cfma(cc, cconj(up[i]), uq[i]);
+    const int rr = r + (r & 1), pairs = rr / 2;  // players of the round robin (index r: a bye when r is odd)
+    const int warps = r <= 16 ? 1 : r <= 32 ? 2 : r <= 48 ? 4 : 8;
+    int lpp = 32;  // lanes per pair
+    while (lpp > 1 && lpp * pairs > 32 * warps) lpp >>= 1;
+    __shared__ int s_turned;
+    if (warp < warps) {
+        auto together = [&]() {
+            if (warps == 1) __syncwarp();
+            else asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
+        };
+        const int groups = 32 * warps / lpp, grp = (warp * 32 + lane) / lpp, g = lane & (lpp - 1);
+        for (int sweep = 0; sweep < 60 && r > 1; ++sweep) {
+            together();
+            if (threadIdx.x == 0) s_turned = 0;
+            together();
+            for (int step = 0; step < rr - 1; ++step) {
+                for (int p0 = 0; p0 < pairs; p0 += groups) {
+                    // circle method: player 0 fixed, the others rotate by `step`
+                    const int pi = p0 + grp;
+                    const int a0 = pi == 0 ? 0 : 1 + (pi - 1 + step) % (rr - 1);
+                    const int b0 = 1 + (rr - 2 - pi + step) % (rr - 1);
+                    const int p = min(a0, b0), q = max(a0, b0);
+                    const bool on = pi < pairs && q < r;  // (q = r: the bye)
+                    double2* up = M + (size_t)p * r;
+                    double2* uq = M + (size_t)q * r;
+                    double a = 0, b = 0;
+                    z2 cc = make_double2(0, 0);
+                    if (on)
+                        for (int i = g; i < r; i += lpp) {
+                            const z2 x = up[i], y = uq[i];
+                            a = fma(x.x, x.x, fma(x.y, x.y, a));
+                            b = fma(y.x, y.x, fma(y.y, y.y, b));
+                            cfma(cc, cconj(x), y);
+                        }
+                    for (int o = 1; o < lpp; o <<= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, o);
+                        b += __shfl_xor_sync(0xffffffffu, b, o);
+                        cc.x += __shfl_xor_sync(0xffffffffu, cc.x, o);
+                        cc.y += __shfl_xor_sync(0xffffffffu, cc.y, o);
+                    }
+                    const double n2 = cnorm2(cc);
+                    const bool turn = on && n2 > 1e-290 && n2 > 1e-30 * (a * b);
+                    if (!__any_sync(0xffffffffu, turn)) continue;
+                    if (lane == 0) s_turned = 1;
+                    if (!turn) continue;
+                    // tan of the angle from FP32, everything relative to max(a, b)
+                    const int e = ((__double2hiint(fmax(a, b)) >> 20) & 0x7ff) - 1023;
+                    const double ri = near_rsqrt(n2);
+                    const float d = near_float(b, e) - near_float(a, e), f = 2.0f * near_float(n2 * ri, e);
+                    const double t = (double)copysignf(__fdividef(f, fmaxf(fabsf(d) + sqrtf(fmaf(d, d, f * f)), 1e-37f)), d);
+                    const double cs = near_rsqrt(fma(t, t, 1.0)), sn = cs * t;
+                    const z2 se = cscale(cc, ri * sn);
+                    for (int i = g; i < r; i += lpp) {
+                        const z2 x = up[i], y = uq[i];
+                        up[i] = make_double2(fma(cs, x.x, -fma(se.x, y.x, se.y * y.y)),
+                                             fma(cs, x.y, -fma(se.x, y.y, -se.y * y.x)));
+                        uq[i] = make_double2(fma(cs, y.x, fma(se.x, x.x, -se.y * x.y)),
+                                             fma(cs, y.y, fma(se.x, x.y, se.y * x.x)));
+                    }
                 }
-                a = wsum(a);
-                b = wsum(b);
-                cc = wsum2(cc);
-                const double ac = hypot(cc.x, cc.y);
-                if (ac == 0 || ac <= 1e-15 * sqrt(a * b)) continue;
-                if (lane == 0) atomicMax(&s_off, (unsigned long long)__double_as_longlong(ac / sqrt(a * b)));
-                const double zeta = (b - a) / (2.0 * ac);
-                const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                const double cs = 1.0 / sqrt(1.0 + t * t), sn = cs * t;
-                const z2 e = make_double2(cc.x / ac, cc.y / ac);
-                const z2 se = cscale(e, sn), sce = cscale(cconj(e), sn);
-                double2* vp = Vm + (size_t)p * r;
-                double2* vq = Vm + (size_t)q * r;
-                for (int i = lane; i < r; i += 32) {
-                    z2 x = up[i], y = uq[i];
-                    up[i] = csub(cscale(x, cs), cmul(sce, y));
-                    uq[i] = cadd(cmul(se, x), cscale(y, cs));
-                    z2 vx = vp[i], vy = vq[i];
-                    vp[i] = csub(cscale(vx, cs), cmul(sce, vy));
-                    vq[i] = cadd(cmul(se, vx), cscale(vy, cs));
-                }
+                together();
             }
-            __syncthreads();
+            if (*(volatile int*)&s_turned == 0) break;
         }
-        const double off = __longlong_as_double((long long)s_off);
-        __syncthreads();
-        if (off < 1e-15) break;
     }
-    // singular values, descending order (stable)
+    __syncthreads();
+    // singular values and their descending order
     for (int j = warp; j < r; j += nw) {
         double v = 0;
         for (int i = lane; i < r; i += 32) v += cnorm2(M[(size_t)j * r + i]);
@@ -572,11 +604,10 @@ __device__ void jacobi_svd_dev(double2* M, double2* Vm, int r, double* S, int* p
         if (lane == 0) S[j] = sqrt(v);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 0; j < r; ++j) perm[j] = j;
-        for (int a = 0; a < r; ++a)
-            for (int b = a + 1; b < r; ++b)
-                if (S[perm[b]] > S[perm[a]]) { int t = perm[a]; perm[a] = perm[b]; perm[b] = t; }
+    for (int j = threadIdx.x; j < r; j += blockDim.x) {
+        int at = 0;
+        for (int i = 0; i < r; ++i) at += S[i] > S[j] || (S[i] == S[j] && i < j);
+        perm[at] = j;
     }
     __syncthreads();
 }
@@ -587,7 +618,7 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
                                                                      double2* __restrict__ scr,
                                                                      const int64_t* __restrict__ scr2_off,
                                                                      double tol) {
-    __shared__ double sh[48];
+    __shared__ double2 sM[JACOBI_SMEM * JACOBI_SMEM];
     HLeaf& L = leaves[list[blockIdx.x]];
     const int r = L.rank;
     const int64_t m = L.m, n = L.n;
@@ -597,25 +628,27 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
     double2* Ru = w;
     double2* Rv = Ru + (size_t)r * r;
     double2* RR = Rv + (size_t)r * r;
-    double2* Vm = RR + (size_t)r * r;
-    double2* B = Vm + (size_t)r * r;
+    double2* M = RR + (size_t)r * r;
+    double2* B = M + (size_t)r * r;
+    if (r <= JACOBI_SMEM) M = sM;
     double2* tauu = B + (size_t)r * r;
     double2* tauv = tauu + r;
     double2* outU = tauv + r;             // m x r
     double2* outV = outU + (size_t)m * r; // n x r
     double* S = reinterpret_cast<double*>(outV + (size_t)n * r);
     int* perm = reinterpret_cast<int*>(S + r);
-    house_qr_dev(U, m, r, Ru, tauu, sh);
-    house_qr_dev(V, n, r, Rv, tauv, sh);
+    house_qr_dev(U, m, r, Ru, tauu);
+    house_qr_dev(V, n, r, Rv, tauv);
     // RR = R_u R_v^T
     for (int t = threadIdx.x; t < r * r; t += blockDim.x) {
         int i = t % r, j = t / r;
         z2 acc = make_double2(0, 0);
         for (int l = 0; l < r; ++l) cfma(acc, Ru[(size_t)l * r + i], Rv[(size_t)l * r + j]);
         RR[(size_t)j * r + i] = acc;
+        M[(size_t)j * r + i] = acc;
     }
     __syncthreads();
-    jacobi_svd_dev(RR, Vm, r, S, perm, sh);
+    jacobi_dev(M, r, S, perm);
     // truncation (aca.rs:162-171)
     __shared__ int s_keep;
     if (threadIdx.x == 0) {
@@ -633,43 +666,54 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
     }
     __syncthreads();
     const int keep = s_keep;
-    // U_new = Q_u (W Sigma): W column t = RR column perm[t] / S (so W S = RR col)
+    // U_new = Q_u (W Sigma)
     for (int t = 0; t < keep; ++t)
-        for (int i = threadIdx.x; i < r; i += blockDim.x) B[(size_t)t * r + i] = RR[(size_t)perm[t] * r + i];
+        for (int i = threadIdx.x; i < r; i += blockDim.x) B[(size_t)t * r + i] = M[(size_t)perm[t] * r + i];
     __syncthreads();
-    house_apply_dev(U, m, r, tauu, B, keep, outU, sh);
-    // V_new = Q_v Z, Z column t = (Vh row t)^T = conj(Vm column perm[t])
-    for (int t = 0; t < keep; ++t)
-        for (int i = threadIdx.x; i < r; i += blockDim.x) B[(size_t)t * r + i] = cconj(Vm[(size_t)perm[t] * r + i]);
+    house_apply_dev(U, m, r, tauu, B, keep, outU);
+    // V_new = Q_v Z with Z the transpose of Sigma^-1 W^H (R_u R_v^T) =
+    // Sigma^-2 (W Sigma)^H (R_u R_v^T)
+    for (int t = threadIdx.x; t < keep * r; t += blockDim.x) {
+        const int c = t / r, i = t % r;
+        const double2* wt = M + (size_t)perm[c] * r;
+        const double sv = S[perm[c]], s2 = sv > 0 ? 1.0 / (sv * sv) : 0.0;
+        z2 acc = make_double2(0, 0);
+        for (int l = 0; l < r; ++l) cfma(acc, cconj(wt[l]), RR[(size_t)i * r + l]);
+        B[t] = cscale(acc, s2);
+    }
     __syncthreads();
-    house_apply_dev(V, n, r, tauv, B, keep, outV, sh);
+    house_apply_dev(V, n, r, tauv, B, keep, outV);
     for (int t = 0; t < keep; ++t) {
         for (int64_t i = threadIdx.x; i < m; i += blockDim.x) U[(size_t)t * m + i] = outU[(size_t)t * m + i];
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) V[(size_t)t * n + i] = outV[(size_t)t * n + i];
     }
     __syncthreads();
-    // calculate_norm_estimate (aca.rs:212-222): for each rank a, its products
-    // with the earlier ranks one warp each, summed in rank order by one thread
-    __shared__ double s_prod[256];  // keep <= kmax <= 256
-    double tot = 0;
+    // calculate_norm_estimate (aca.rs:212-222): |u_a|^2 |v_a|^2 and twice the
+    // products of every pair of ranks, one warp per pair
+    __shared__ double s_tot[LEAF_THREADS / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int a = 0; a < keep; ++a) {
-        double nu = bnsq(U + (size_t)a * m, m, sh), nv = bnsq(V + (size_t)a * n, n, sh);
-        for (int b = warp; b < a; b += nw) {
-            z2 du = make_double2(0, 0), dv = make_double2(0, 0);
+    double sum = 0;
+    for (int t = warp; t < keep * (keep + 1) / 2; t += nw) {
+        int a = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+        while (a * (a + 1) / 2 > t) --a;
+        while ((a + 1) * (a + 2) / 2 <= t) ++a;
+        const int b = t - a * (a + 1) / 2;
+        z2 du = make_double2(0, 0), dv = make_double2(0, 0);
+        if (a == b) {
+            for (int64_t i = lane; i < m; i += 32) du.x += cnorm2(U[(size_t)a * m + i]);
+            for (int64_t j = lane; j < n; j += 32) dv.x += cnorm2(V[(size_t)a * n + j]);
+        } else {
             for (int64_t i = lane; i < m; i += 32) cfma(du, U[(size_t)a * m + i], U[(size_t)b * m + i]);
             for (int64_t j = lane; j < n; j += 32) cfma(dv, V[(size_t)a * n + j], V[(size_t)b * n + j]);
-            du = wsum2(du);
-            dv = wsum2(dv);
-            if (lane == 0) s_prod[b] = 2.0 * hypot(du.x, du.y) * hypot(dv.x, dv.y);
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tot += nu * nv;
-            for (int b = 0; b < a; ++b) tot += s_prod[b];
-        }
-        __syncthreads();
+        wsum4(du, dv);
+        sum += a == b ? du.x * dv.x : 2.0 * sqrt(cnorm2(du) * cnorm2(dv));
     }
+    if (lane == 0) s_tot[warp] = sum;
+    __syncthreads();
+    double tot = 0;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < nw; ++i) tot += s_tot[i];
     if (threadIdx.x == 0) {
         L.rank = keep;
         L.norm = sqrt(tot);
