@@ -3,8 +3,8 @@
 // different sizes (ragged layout, per-system offsets in GmSys).
 //
 // One iteration is the fixed launch sequence
-//   apply(START) -> start -> apply(Q) -> [Gram-Schmidt x 2] -> arnoldi -> apply(CHECK) -> check
-// where every kernel reads the per-system state and returns immediately when
+//   [precondition] -> apply(Q) -> Gram-Schmidt and rotations -> apply(CHECK) -> check
+// after one apply(START) -> start, where every kernel reads the per-system state and returns immediately when
 // it has nothing to do.  The sequence can therefore be issued step by step
 // (plain form, host reads the state after each step) or captured into a CUDA
 // graph covering several iterations of every system (batched form).
@@ -27,6 +27,10 @@ constexpr int MV_ROWS_PER_THREAD = 2;
 constexpr int MV_THREADS = 256;
 constexpr int MV_ROWS = MV_ROWS_PER_THREAD * MV_THREADS;  // 512
 constexpr int MV_COLS = 512;
+// row block of the small-batch product, and the tickets that a row block of
+// MV_ROWS holds for it
+constexpr int SMALL_ROWS = 64;
+constexpr int TICKETS = MV_ROWS / SMALL_ROWS;
 constexpr int AR_THREADS = 1024;
 // largest Krylov vector kept in the Arnoldi kernel's shared memory (n <= 12800)
 constexpr size_t AR_SMEM_CAP = 200 * 1024;
@@ -234,6 +238,218 @@ __global__ void __launch_bounds__(MV_THREADS) gm_apply_kernel(GmBatch bt, int mo
     }
 }
 
+// The same product cut finer, for batches whose MV_ROWS x MV_COLS tiles are too
+// few to fill the SMs: a CTA of eight warps takes SMALL_ROWS rows of a column
+// chunk, the warps share its columns.  Latency bounds such a batch, so what
+// counts is loads in flight on every SM (four systems of n = 1280: 36 wide tiles
+// 37 us, 240 of these 11 us).
+//
+// The sums keep their order.  In the FAST scheme the warps take the groups of U
+// columns in turn and leave each group's FP32 sum in shared memory; a thread
+// per row and component folds them in column order, so that the result is the
+// same bits as the wide tile's.  In the others a warp accumulates its own
+// columns and the eight sums are added in FP64.
+constexpr int SMALL_WARPS = 8;
+template <typename T, int EXACT, int U>
+constexpr size_t small_smem() {
+    return sizeof(T) == sizeof(float2) && !EXACT ? sizeof(float2) * (MV_COLS / U) * SMALL_ROWS
+                                                 : sizeof(double2) * SMALL_WARPS * SMALL_ROWS;
+}
+
+template <typename T, int EXACT, int U>
+__global__ void __launch_bounds__(32 * SMALL_WARPS) gm_apply_small_kernel(GmBatch bt, int mode) {
+    static_assert(MV_COLS % (U * SMALL_WARPS) == 0, "every warp takes the same number of column groups");
+    constexpr bool F32 = sizeof(T) == sizeof(float2);
+    int s, bx, by;
+    if (bt.sys) {
+        const int64_t t = blockIdx.x;
+        int lo = 0, hi = bt.nsys - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (bt.sys[mid].tile64 <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        s = lo;
+        const int64_t local = t - bt.sys[s].tile64;
+        const int64_t rbs = (bt.sys[s].n + SMALL_ROWS - 1) / SMALL_ROWS;
+        bx = (int)(local % rbs);
+        by = (int)(local / rbs);
+    } else {
+        s = blockIdx.z;
+        bx = blockIdx.x;
+        by = blockIdx.y;
+    }
+    if (!gm_apply_active(bt, bt.st[s], mode)) return;
+    const GmView g = gm_view(bt, s);
+    const int64_t n = g.n, lda = g.lda;
+    const double2* kv = bt.Z ? bt.Z : bt.Q;
+    const double2* v = (mode == MV_Q) ? kv + g.q + (size_t)bt.st[s].k * n : bt.X + g.v;
+    __shared__ float2 xh[F32 ? MV_COLS : 1], xl[F32 && EXACT ? MV_COLS : 1];
+    __shared__ double2 xd[F32 ? 1 : MV_COLS];
+    __shared__ int last;
+    extern __shared__ double2 sums[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t j0 = (int64_t)by * MV_COLS;
+    const int jn = (int)min((int64_t)MV_COLS, n - j0);
+    for (int t = tid; t < MV_COLS; t += 32 * SMALL_WARPS) {
+        const double2 x = t < jn ? v[j0 + t] : make_double2(0, 0);
+        if (F32) {
+            const float hx = (float)x.x, hy = (float)x.y;
+            xh[t] = make_float2(hx, hy);
+            if (EXACT) xl[t] = make_float2((float)(x.x - (double)hx), (float)(x.y - (double)hy));
+        } else {
+            xd[t] = x;
+        }
+    }
+    __syncthreads();
+    const int64_t b0 = (int64_t)bx * SMALL_ROWS;
+    double2* part = bt.part + g.p + (size_t)by * g.n_pad;
+    if (F32 && !EXACT) {
+        float2* gs = reinterpret_cast<float2*>(sums);  // [group][row]
+        const int64_t i0 = b0 + 2 * lane;
+        if (i0 < n) {
+            const bool pair = i0 + 1 < n;
+            const float2* A = reinterpret_cast<const float2*>(bt.A) + g.a + i0;
+            for (int q0 = warp * U; q0 < jn; q0 += SMALL_WARPS * U) {
+                float4 a[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int q = q0 + u;
+                    if (q < jn) {
+                        const float2* col = A + (j0 + q) * lda;
+                        if (pair) a[u] = __ldcs(reinterpret_cast<const float4*>(col));
+                        else { float2 t = col[0]; a[u] = make_float4(t.x, t.y, 0.f, 0.f); }
+                    } else {
+                        a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+                float b0_ = 0, b1 = 0, b2 = 0, b3 = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float2 H = xh[q0 + u];
+                    const float4 w = a[u];
+                    b0_ = fmaf(w.x, H.x, fmaf(-w.y, H.y, b0_));
+                    b1 = fmaf(w.x, H.y, fmaf(w.y, H.x, b1));
+                    b2 = fmaf(w.z, H.x, fmaf(-w.w, H.y, b2));
+                    b3 = fmaf(w.z, H.y, fmaf(w.w, H.x, b3));
+                }
+                reinterpret_cast<float4*>(gs)[(q0 / U) * (SMALL_ROWS / 2) + lane] = make_float4(b0_, b1, b2, b3);
+            }
+        }
+        __syncthreads();
+        if (tid < 2 * SMALL_ROWS && b0 + (tid >> 1) < n) {
+            const float* f = reinterpret_cast<const float*>(gs) + tid;
+            const int groups = (jn + U - 1) / U;
+            float h = 0, l = 0, e, t;
+#pragma unroll 4
+            for (int q = 0; q < groups; ++q) {
+                two_sum(h, f[(size_t)q * 2 * SMALL_ROWS], t, e);
+                h = t;
+                l += e;
+            }
+            reinterpret_cast<double*>(part + b0)[tid] = (double)h + (double)l;
+        }
+    } else {
+        double2 r0 = make_double2(0, 0), r1 = make_double2(0, 0);
+        if (F32) {
+            const int64_t i0 = b0 + 2 * lane;
+            if (i0 < n) {
+                const bool pair = i0 + 1 < n;
+                const float2* A = reinterpret_cast<const float2*>(bt.A) + g.a + i0;
+                float h0 = 0, l0 = 0, h1 = 0, l1 = 0, h2 = 0, l2 = 0, h3 = 0, l3 = 0;
+                for (int q0 = warp * U; q0 < jn; q0 += SMALL_WARPS * U) {
+                    float4 a[U], z[EXACT == 2 ? U : 1];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int q = q0 + u;
+                        const float2* col = A + (j0 + (q < jn ? q : 0)) * lda;
+                        if (q >= jn) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        else if (pair) a[u] = __ldcs(reinterpret_cast<const float4*>(col));
+                        else { float2 t = col[0]; a[u] = make_float4(t.x, t.y, 0.f, 0.f); }
+                        if (EXACT == 2) {
+                            const float2* cl = col + bt.split_lo;
+                            if (q >= jn) z[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            else if (pair) z[u] = __ldcs(reinterpret_cast<const float4*>(cl));
+                            else { float2 t = cl[0]; z[u] = make_float4(t.x, t.y, 0.f, 0.f); }
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const float2 H = xh[q0 + u], L = xl[q0 + u];
+                        const float4 w = a[u];
+                        ff_acc(h0, l0, w.x, H.x); ff_acc(h0, l0, -w.y, H.y);
+                        ff_acc(h1, l1, w.x, H.y); ff_acc(h1, l1, w.y, H.x);
+                        ff_acc(h2, l2, w.z, H.x); ff_acc(h2, l2, -w.w, H.y);
+                        ff_acc(h3, l3, w.z, H.y); ff_acc(h3, l3, w.w, H.x);
+                        l0 = fmaf(w.x, L.x, fmaf(-w.y, L.y, l0));
+                        l1 = fmaf(w.x, L.y, fmaf(w.y, L.x, l1));
+                        l2 = fmaf(w.z, L.x, fmaf(-w.w, L.y, l2));
+                        l3 = fmaf(w.z, L.y, fmaf(w.w, L.x, l3));
+                        if (EXACT == 2) {
+                            const float4 y = z[EXACT == 2 ? u : 0];
+                            l0 = fmaf(y.x, H.x, fmaf(-y.y, H.y, l0));
+                            l1 = fmaf(y.x, H.y, fmaf(y.y, H.x, l1));
+                            l2 = fmaf(y.z, H.x, fmaf(-y.w, H.y, l2));
+                            l3 = fmaf(y.z, H.y, fmaf(y.w, H.x, l3));
+                        }
+                    }
+                }
+                r0 = make_double2((double)h0 + (double)l0, (double)h1 + (double)l1);
+                r1 = make_double2((double)h2 + (double)l2, (double)h3 + (double)l3);
+            }
+            sums[warp * SMALL_ROWS + 2 * lane] = r0;
+            sums[warp * SMALL_ROWS + 2 * lane + 1] = r1;
+        } else {
+            // (rows lane and lane + 32: each load of a warp is 512 bytes in one piece)
+            const int64_t i0 = b0 + lane;
+            const bool in0 = i0 < n, in1 = i0 + 32 < n;
+            const double2* A = reinterpret_cast<const double2*>(bt.A) + g.a + i0;
+            for (int q0 = warp * U; q0 < jn; q0 += SMALL_WARPS * U) {
+                double2 a0[U], a1[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int q = q0 + u;
+                    const double2* col = A + (j0 + (q < jn ? q : 0)) * lda;
+                    a0[u] = (q < jn && in0) ? __ldcs(col) : make_double2(0, 0);
+                    a1[u] = (q < jn && in1) ? __ldcs(col + 32) : make_double2(0, 0);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const double2 xv = xd[q0 + u];
+                    cfma(r0, a0[u], xv);
+                    cfma(r1, a1[u], xv);
+                }
+            }
+            sums[warp * SMALL_ROWS + lane] = r0;
+            sums[warp * SMALL_ROWS + lane + 32] = r1;
+        }
+        __syncthreads();
+        if (tid < 2 * SMALL_ROWS && b0 + (tid >> 1) < n) {
+            const double* f = reinterpret_cast<const double*>(sums) + tid;
+            double t = f[0];
+#pragma unroll
+            for (int w = 1; w < SMALL_WARPS; ++w) t += f[w * 2 * SMALL_ROWS];
+            reinterpret_cast<double*>(part + b0)[tid] = t;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        int* tk = bt.tickets + g.t + bx;
+        last = (atomicAdd(tk, 1) == g.cb - 1);
+        if (last) *tk = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (tid < 2 * SMALL_ROWS && b0 + (tid >> 1) < n) {
+        const double* p = reinterpret_cast<const double*>(bt.part + g.p + b0) + tid;
+        double acc = 0;
+        for (int c = 0; c < g.cb; ++c) acc += p[(size_t)c * 2 * g.n_pad];
+        reinterpret_cast<double*>(bt.W + g.v + b0)[tid] = acc;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Block-wide FP64 reductions (1024 threads).
 __device__ __forceinline__ double block_sum(double v, double* sh) {
@@ -280,7 +496,16 @@ __device__ double vec_norm(const double2* v, int64_t n, double* sh) {
     return sqrt(block_sum(s, sh));
 }
 
-// Cycle start (gmres.rs:84-106): r = b - A x, q_0 = r / ||r||, beta_0 = ||r||.
+// Krylov state of a cycle that starts with residual norm rn (one thread).
+__device__ __forceinline__ void gm_cycle_state(const GmBatch& bt, int s, double rn) {
+    GmSmall sm = gm_small(bt, s);
+    for (int i = 0; i <= bt.m; ++i) sm.beta[i] = make_double2(0, 0);
+    for (int i = 0; i < bt.m; ++i) { sm.cs[i] = make_double2(0, 0); sm.sn[i] = make_double2(0, 0); }
+    sm.beta[0] = make_double2(rn, 0.0);
+    bt.st[s].k = 0;
+}
+
+// Start of the first cycle (gmres.rs:84-106; gm_check_kernel starts the others): r = b - A x, q_0 = r / ||r||, beta_0 = ||r||.
 __global__ void __launch_bounds__(AR_THREADS) gm_start_kernel(GmBatch bt) {
     const int s = blockIdx.x;
     GmState& st = bt.st[s];
@@ -305,13 +530,9 @@ __global__ void __launch_bounds__(AR_THREADS) gm_start_kernel(GmBatch bt) {
     }
     double xn = vec_norm(bt.X + g.v, n, sh);
     if (threadIdx.x == 0) {
-        GmSmall sm = gm_small(bt, s);
-        for (int i = 0; i <= bt.m; ++i) sm.beta[i] = make_double2(0, 0);
-        for (int i = 0; i < bt.m; ++i) { sm.cs[i] = make_double2(0, 0); sm.sn[i] = make_double2(0, 0); }
-        sm.beta[0] = make_double2(rn, 0.0);
         st.xnorm = xn;
         st.error = rn / (st.anorm * xn + st.bnorm);
-        st.k = 0;
+        gm_cycle_state(bt, s, rn);
         st.need_start = 0;
         st.check = 0;
         st.num_mv += zero_x ? 0 : 1;
@@ -321,16 +542,35 @@ __global__ void __launch_bounds__(AR_THREADS) gm_start_kernel(GmBatch bt) {
 // ---------------------------------------------------------------------------
 // Gram-Schmidt of the mixed and refined forms across the whole GPU: classical
 // Gram-Schmidt applied twice (the second pass re-orthogonalises; as accurate
-// as the modified form), in FP64.  Every CTA owns a chunk of GS_ROWS rows of
-// one system: the dots kernel forms its chunk's contribution to q_i^H w for
-// every i <= k (a warp per basis vector), the update kernel adds the chunks'
-// contributions in chunk order and subtracts Q h from its rows (and, after
-// the second pass, leaves the squared norm of its rows).  Systems pending a
+// as the modified form), in FP64.  Every CTA owns a chunk of rows of one
+// system: the dots kernel forms its chunk's contribution to q_i^H w for every
+// i <= k, the update kernel adds the chunks' contributions in a fixed order and
+// subtracts Q h from its rows (and, after the second pass, leaves the squared
+// norm of its rows).  Systems pending a
 // Krylov step only (the Arnoldi kernel's predicate).
+//
+// FP64 instructions bound both (65 clocks per warp instruction and SM quarter),
+// so a small batch is cut into chunks of down to 64 rows until the CTAs cover
+// the SMs, and a basis vector takes eight lanes: a reduction over 32 lanes
+// would cost as much as the products of 64 rows.  (Four systems of n = 1280, 12
+// chunks of 512 rows and a warp per vector: 10.5 us per kernel; 80 chunks of 64:
+// 3.7 and 5.3 us.)
 constexpr int GS_ROWS = 512, GS_THREADS = 256;
 
 __device__ __forceinline__ bool gm_arnoldi_active(const GmState& st) {
     return !(st.done || st.need_start || st.check);
+}
+
+// Sum over the eight lanes of a group (every lane gets it): the parts part ways
+// in the first step, three additions.
+__device__ __forceinline__ double2 sum8(double2 v) {
+    const bool odd = threadIdx.x & 1;
+    double s = odd ? v.y : v.x;
+    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    const int base = threadIdx.x & 24;
+    return make_double2(__shfl_sync(0xffffffffu, s, base), __shfl_sync(0xffffffffu, s, base + 1));
 }
 
 __global__ void __launch_bounds__(GS_THREADS) gm_gs_dots_kernel(GmBatch bt) {
@@ -338,25 +578,24 @@ __global__ void __launch_bounds__(GS_THREADS) gm_gs_dots_kernel(GmBatch bt) {
     const GmState& st = bt.st[s];
     if (!gm_arnoldi_active(st)) return;
     const GmView g = gm_view(bt, s);
-    const int64_t r0 = (int64_t)c * GS_ROWS;
+    const int64_t r0 = (int64_t)c * bt.gs_rows;
     if (r0 >= g.n) return;
-    const int rows = (int)min((int64_t)GS_ROWS, g.n - r0);
+    const int rows = (int)min((int64_t)bt.gs_rows, g.n - r0);
     __shared__ double2 ws[GS_ROWS];
     const double2* W = bt.W + g.v + r0;
     for (int l = threadIdx.x; l < rows; l += GS_THREADS) ws[l] = W[l];
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = threadIdx.x >> 3, lane = threadIdx.x & 7;
     const double2* Q = bt.Q + g.q + r0;
     double2* part = bt.gs_part + ((size_t)s * bt.gs_chunks + c) * (bt.m + 1);
-    for (int i = warp; i <= st.k; i += GS_THREADS / 32) {
-        const double2* qi = Q + (size_t)i * g.n;
+    for (int i0 = 0; i0 <= st.k; i0 += GS_THREADS / 8) {
+        const int i = i0 + grp;
+        if (i0 + (grp & ~3) > st.k) break;  // (a whole warp)
+        const double2* qi = Q + (size_t)min(i, st.k) * g.n;
         double2 acc = make_double2(0, 0);
-        for (int l = lane; l < rows; l += 32) cfma(acc, cconj(qi[l]), ws[l]);
-        for (int o = 16; o > 0; o >>= 1) {
-            acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-            acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
-        }
-        if (lane == 0) part[i] = acc;
+        for (int l = lane; l < rows; l += 8) cfma(acc, cconj(qi[l]), ws[l]);
+        acc = sum8(acc);
+        if (lane == 0 && i <= st.k) part[i] = acc;
     }
 }
 
@@ -366,32 +605,53 @@ __global__ void __launch_bounds__(GS_THREADS) gm_gs_update_kernel(GmBatch bt, in
     const GmState& st = bt.st[s];
     if (!gm_arnoldi_active(st)) return;
     const GmView g = gm_view(bt, s);
-    const int64_t r0 = (int64_t)c * GS_ROWS;
+    const int64_t r0 = (int64_t)c * bt.gs_rows;
     if (r0 >= g.n) return;
-    const int rows = (int)min((int64_t)GS_ROWS, g.n - r0);
+    const int rows = (int)min((int64_t)bt.gs_rows, g.n - r0);
     const int k = st.k;
-    const int nch = (int)((g.n + GS_ROWS - 1) / GS_ROWS);
+    const int nch = (int)((g.n + bt.gs_rows - 1) / bt.gs_rows);
     extern __shared__ double2 hsum[];  // k + 1 coefficients
+    __shared__ double2 partial[GS_THREADS];
     __shared__ double red[GS_THREADS / 32];
     const double2* part = bt.gs_part + (size_t)s * bt.gs_chunks * (bt.m + 1);
-    for (int i = threadIdx.x; i <= k; i += GS_THREADS) {
+    const int grp = threadIdx.x >> 3, lane = threadIdx.x & 7;
+    for (int i0 = 0; i0 <= k; i0 += GS_THREADS / 8) {
+        const int i = i0 + grp;
+        if (i0 + (grp & ~3) > k) break;
         double2 h = make_double2(0, 0);
-        for (int cc = 0; cc < nch; ++cc) h = cadd(h, part[(size_t)cc * (bt.m + 1) + i]);
-        hsum[i] = h;
+        for (int cc = lane; cc < nch; cc += 8) h = cadd(h, part[(size_t)cc * (bt.m + 1) + min(i, k)]);
+        h = sum8(h);
+        if (lane == 0 && i <= k) hsum[i] = h;
     }
     __syncthreads();
-    if (c == 0 && threadIdx.x == 0) {
+    if (c == 0) {
         GmSmall sm = gm_small(bt, s);
-        for (int i = 0; i <= k; ++i) sm.hk1[i] = pass == 0 ? hsum[i] : cadd(sm.hk1[i], hsum[i]);
+        for (int i = threadIdx.x; i <= k; i += GS_THREADS) sm.hk1[i] = pass == 0 ? hsum[i] : cadd(sm.hk1[i], hsum[i]);
     }
     double2* W = bt.W + g.v + r0;
     const double2* Q = bt.Q + g.q + r0;
     double nn = 0;
-    for (int l = threadIdx.x; l < rows; l += GS_THREADS) {
-        double2 a = W[l];
-        for (int i = 0; i <= k; ++i) cfma(a, cneg(hsum[i]), Q[(size_t)i * g.n + l]);
-        W[l] = a;
-        nn += a.x * a.x + a.y * a.y;
+    // rows x groups of coefficients: with fewer than 256 rows the threads share
+    // a row's coefficients
+    const int wide = min(bt.gs_rows, GS_THREADS), groups = GS_THREADS / wide;
+    const int lr = threadIdx.x % wide, kg = threadIdx.x / wide;
+    for (int l0 = 0; l0 < rows; l0 += wide) {
+        const int l = l0 + lr;
+        double2 a = make_double2(0, 0);
+        if (l < rows) {
+            if (kg == 0) a = W[l];
+            for (int i = kg; i <= k; i += groups) cfma(a, cneg(hsum[i]), Q[(size_t)i * g.n + l]);
+        }
+        if (groups > 1) {
+            partial[threadIdx.x] = a;
+            __syncthreads();
+            if (kg == 0)
+                for (int q = 1; q < groups; ++q) a = cadd(a, partial[q * wide + lr]);
+        }
+        if (l < rows && kg == 0) {
+            W[l] = a;
+            nn = fma(a.x, a.x, fma(a.y, a.y, nn));
+        }
     }
     if (pass == 1) {
         for (int o = 16; o > 0; o >>= 1) nn += __shfl_down_sync(0xffffffffu, nn, o);
@@ -399,9 +659,164 @@ __global__ void __launch_bounds__(GS_THREADS) gm_gs_update_kernel(GmBatch bt, in
         __syncthreads();
         if (threadIdx.x == 0) {
             double t = 0;
-            for (int w = 0; w < GS_THREADS / 32; ++w) t += red[w];
+            for (int w = 0; w < wide / 32; ++w) t += red[w];
             bt.gs_norm[(size_t)s * bt.gs_chunks + c] = t;
         }
+    }
+}
+
+// The rest of an Arnoldi step after the Gram-Schmidt kernels: Givens rotations
+// (gmres.rs:178-202), residual estimate and, when the estimate passes or the
+// cycle ends, y = H_k^{-1} beta_k (gmres.rs:146-157); q_{k+1} = w / |w| and
+// x += Z_k y by chunks of rows.  Every CTA of a system does the small part for
+// itself (so that nothing but the chunks' results has to travel); the last one
+// of a system to finish records it.
+//
+// The chain bounds it: two dependent FP64 multiply-adds (130 clocks) and a
+// shuffle per earlier rotation, the other products of a rotation off the chain,
+// one lane per unknown in the triangular solve.  (One thread doing all of it
+// took 36 us per step at n = 1280, k up to 30, and x += Z y another 40 us on
+// one SM; now 12.5 us on average with the update.)
+constexpr int GV_STEP_THREADS = 256;
+constexpr size_t givens_smem(int m) { return sizeof(double2) * 4 * (size_t)(m + 1); }
+__global__ void __launch_bounds__(GV_STEP_THREADS) gm_givens_kernel(GmBatch bt, int chunks) {
+    const int s = blockIdx.y;
+    GmState& st = bt.st[s];
+    if (!gm_arnoldi_active(st)) return;
+    extern __shared__ double2 sh2[];
+    const GmView g = gm_view(bt, s);
+    const int64_t n = g.n;
+    const int k = st.k, m = bt.m, tid = threadIdx.x, lane = tid & 31;
+    const double anorm = st.anorm, xnorm = st.xnorm, bnorm = st.bnorm, tol = st.tol;
+    const int last_k = st.m - 1;
+    GmSmall sm = gm_small(bt, s);
+    double2 *h = sh2, *a = h + (m + 1), *cs = a + (m + 1), *sn = cs + (m + 1);
+    double2 *dinv = a, *y = cs;  // (in the triangular solve)
+    __shared__ double scale_s, error_s;
+    __shared__ double2 cs_k, sn_k, beta_k, beta_k1;
+    __shared__ int chk_s, last;
+    for (int i = tid; i <= k; i += GV_STEP_THREADS) h[i] = sm.hk1[i];
+    for (int i = tid; i < k; i += GV_STEP_THREADS) {
+        cs[i] = sm.cs[i];
+        sn[i] = sm.sn[i];
+    }
+    __syncthreads();
+    if (tid < 32) {
+        double nn = 0;
+        const int nch = (int)((n + bt.gs_rows - 1) / bt.gs_rows);  // this system's chunks (ragged batches)
+        for (int c = lane; c < nch; c += 32) nn += bt.gs_norm[(size_t)s * bt.gs_chunks + c];
+        for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
+        // a_i = the entry rotation i meets: a_0 = h_0, a_{i+1} = -conj(sn_i) a_i + cs_i h_{i+1}
+        // (lane 0 the real, lane 1 the imaginary part)
+        double2 cur = h[0];
+        for (int i = 0; i < k; ++i) {
+            if (lane == 0) a[i] = cur;
+            const double2 cc = cs[i], ss = sn[i], b = h[i + 1];
+            const double base = lane ? b.y : b.x, p = lane ? cur.y : cur.x, q = lane ? -cur.x : cur.y;
+            const double v = fma(-ss.y, q, fma(-ss.x, p, cc.x * base));
+            cur.x = __shfl_sync(0xffffffffu, v, 0);
+            cur.y = __shfl_sync(0xffffffffu, v, 1);
+        }
+        __syncwarp();
+        // the rotated entries, off the chain
+        for (int i = lane; i < k; i += 32) {
+            const double2 t = cadd(make_double2(cs[i].x * a[i].x, cs[i].x * a[i].y), cmul(sn[i], h[i + 1]));
+            a[i] = t;  // (held until every lane has read h)
+        }
+        __syncwarp();
+        for (int i = lane; i < k; i += 32) h[i] = a[i];
+        // new rotation (LAWN 148): v1 = cur, v2 = |w| real.  The roots and the
+        // quotients are taken side by side, a lane each: one costs 600 clocks.
+        const double c2 = cnorm2(cur);
+        double rt = sqrt(lane == 0 ? nn : lane == 1 ? c2 : c2 + nn);
+        if (lane == 1 && !(c2 > 1e-280)) rt = cabs_(cur);
+        const double hn = __shfl_sync(0xffffffffu, rt, 0), a1 = __shfl_sync(0xffffffffu, rt, 1),
+                     r = __shfl_sync(0xffffffffu, rt, 2);
+        const double qt = (lane == 0 ? cur.x : lane == 1 ? cur.y : lane == 2 ? a1 : lane == 3 ? hn : 1.0) /
+                          (lane < 2 ? a1 : lane < 4 ? r : hn);
+        double2 signf = make_double2(__shfl_sync(0xffffffffu, qt, 0), __shfl_sync(0xffffffffu, qt, 1));
+        const double c0 = __shfl_sync(0xffffffffu, qt, 2), t0 = __shfl_sync(0xffffffffu, qt, 3),
+                     sc = __shfl_sync(0xffffffffu, qt, 4);
+        if (cur.x == 0.0 && cur.y == 0.0) signf = make_double2(1.0, 0.0);
+        const double2 s0 = make_double2(signf.x * t0, signf.y * t0);
+        const double2 bk = sm.beta[k];
+        const double2 b1 = cmul(cneg(cconj(s0)), bk), b0 = make_double2(bk.x * c0, bk.y * c0);
+        if (lane == 0) {
+            h[k] = cadd(make_double2(c0 * cur.x, c0 * cur.y), make_double2(s0.x * hn, s0.y * hn));
+            scale_s = sc;
+            cs_k = make_double2(c0, 0.0);
+            sn_k = s0;
+            beta_k = b0;
+            beta_k1 = b1;
+            error_s = cabs_(b1) / (anorm * xnorm + bnorm);
+            chk_s = (error_s < tol) || (k == last_k);
+        }
+    }
+    __syncthreads();
+    if (chk_s) {
+        // column by column from the last: y_i, then its multiple off the rest
+        if (tid <= k) dinv[tid] = cdiv(make_double2(1.0, 0.0), tid == k ? h[k] : sm.H[(size_t)tid * (m + 1) + tid]);
+        for (int i = tid + GV_STEP_THREADS; i <= k; i += GV_STEP_THREADS)
+            dinv[i] = cdiv(make_double2(1.0, 0.0), i == k ? h[k] : sm.H[(size_t)i * (m + 1) + i]);
+        for (int i = tid; i <= k; i += GV_STEP_THREADS) y[i] = i == k ? beta_k : sm.beta[i];
+        __syncthreads();
+        if (tid < 32)
+            for (int i = k; i >= 0; --i) {
+                const double2 yi = cmul(y[i], dinv[i]);
+                __syncwarp();
+                if (lane == 0) y[i] = yi;
+                for (int r = lane; r < i; r += 32) {
+                    const double2 e = i == k ? h[r] : sm.H[(size_t)i * (m + 1) + r];
+                    y[r] = csub(y[r], cmul(e, yi));
+                }
+                __syncwarp();
+            }
+        __syncthreads();
+    }
+    // this CTA's rows
+    const int64_t per = (n + chunks - 1) / chunks, l0 = (int64_t)blockIdx.x * per, l1 = min(n, l0 + per);
+    const double sc = scale_s;
+    const double2* Wg = bt.W + g.v;
+    double2* Q = bt.Q + g.q;
+    double2* qk1 = Q + (size_t)(k + 1) * n;
+    for (int64_t l = l0 + tid; l < l1; l += GV_STEP_THREADS) {
+        const double2 w = Wg[l];
+        qk1[l] = make_double2(w.x * sc, w.y * sc);
+    }
+    if (chk_s) {
+        // x += Q_k y, or Z_k y with flexible right preconditioning
+        double2* x = bt.X + g.v;
+        const double2* Zs = bt.Z ? bt.Z + g.q : Q;
+        for (int64_t l = l0 + tid; l < l1; l += GV_STEP_THREADS) {
+            double2 v = x[l];
+            for (int j = 0; j <= k; ++j) cfma(v, Zs[(size_t)j * n + l], y[j]);
+            x[l] = v;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        int* tk = bt.tickets + g.t;  // (between the products' launches: zero)
+        last = atomicAdd(tk, 1) == chunks - 1;
+        if (last) *tk = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    for (int i = tid; i <= k; i += GV_STEP_THREADS) {
+        sm.H[(size_t)k * (m + 1) + i] = h[i];
+        if (chk_s) sm.y[i] = y[i];
+    }
+    if (tid == 0) {
+        sm.H[(size_t)k * (m + 1) + k + 1] = make_double2(0, 0);
+        sm.cs[k] = cs_k;
+        sm.sn[k] = sn_k;
+        sm.beta[k] = beta_k;
+        sm.beta[k + 1] = beta_k1;
+        st.error = error_s;
+        st.num_mv += 1;
+        st.iterations += 1;
+        st.check = chk_s;
+        if (!chk_s) st.k = k + 1;
     }
 }
 
@@ -426,47 +841,31 @@ __global__ void __launch_bounds__(AR_THREADS) gm_arnoldi_kernel(GmBatch bt, int 
     double2* w = w_in_smem ? wsh : Wg;
     GmSmall sm = gm_small(bt, s);
     double2* qk1 = Q + (size_t)(k + 1) * n;
-    double hn;
-    if (bt.gs_part && !bt.ref_dotc) {
-        // orthogonalised across the GPU (gm_gs_dots_kernel /
-        // gm_gs_update_kernel): h_{:,k} is in hk1[0..k], w in W; its norm
-        // from the chunks' partial squares
-        double nn = 0;
-        const int nch = (int)((n + GS_ROWS - 1) / GS_ROWS);  // this system's chunks (ragged batches)
-        for (int c = 0; c < nch; ++c) nn += bt.gs_norm[(size_t)s * bt.gs_chunks + c];
-        hn = sqrt(nn);
-        const double sc = 1.0 / hn;
+    if (w_in_smem)
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) w[i] = Wg[i];
+    __syncthreads();
+    // modified Gram-Schmidt
+    for (int i = 0; i <= k; ++i) {
+        const double2* qi = Q + (size_t)i * n;
+        double2 acc = make_double2(0, 0);
         for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-            const double2 a = Wg[l];
-            qk1[l] = make_double2(a.x * sc, a.y * sc);
+            double2 a = w[l], q = qi[l];
+            if (bt.ref_dotc) cfma(acc, cconj(a), q);  // nalgebra dotc(qk1, q_i) = sum conj(qk1) q_i
+            else cfma(acc, cconj(q), a);             // q_i^H w
         }
-    } else {
-        if (w_in_smem)
-            for (int64_t i = threadIdx.x; i < n; i += blockDim.x) w[i] = Wg[i];
+        double2 h = block_sum2(acc, sh);
+        for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
+            double2 a = w[l];
+            cfma(a, cneg(h), qi[l]);
+            w[l] = a;
+        }
+        if (threadIdx.x == 0) sm.hk1[i] = h;
         __syncthreads();
-        // modified Gram-Schmidt
-        for (int i = 0; i <= k; ++i) {
-            const double2* qi = Q + (size_t)i * n;
-            double2 acc = make_double2(0, 0);
-            for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-                double2 a = w[l], q = qi[l];
-                if (bt.ref_dotc) cfma(acc, cconj(a), q);  // nalgebra dotc(qk1, q_i) = sum conj(qk1) q_i
-                else cfma(acc, cconj(q), a);             // q_i^H w
-            }
-            double2 h = block_sum2(acc, sh);
-            for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-                double2 a = w[l];
-                cfma(a, cneg(h), qi[l]);
-                w[l] = a;
-            }
-            if (threadIdx.x == 0) sm.hk1[i] = h;
-            __syncthreads();
-        }
-        hn = vec_norm(w, n, sh);
-        // scale = 1 / hk1[k+1] as a complex division (gmres.rs:172)
-        double2 scale = cdiv(make_double2(1.0, 0.0), make_double2(hn, 0.0));
-        for (int64_t l = threadIdx.x; l < n; l += blockDim.x) qk1[l] = cmul(w[l], scale);
     }
+    const double hn = vec_norm(w, n, sh);
+    // scale = 1 / hk1[k+1] as a complex division (gmres.rs:172)
+    double2 scale = cdiv(make_double2(1.0, 0.0), make_double2(hn, 0.0));
+    for (int64_t l = threadIdx.x; l < n; l += blockDim.x) qk1[l] = cmul(w[l], scale);
     if (threadIdx.x == 0) {
         sm.hk1[k + 1] = make_double2(hn, 0.0);
         // apply previous rotations
@@ -520,12 +919,15 @@ __global__ void __launch_bounds__(AR_THREADS) gm_arnoldi_kernel(GmBatch bt, int 
     }
 }
 
-// True residual check (gmres.rs:122-138).
+// True residual check (gmres.rs:122-138), and the start of the next cycle
+// (gmres.rs:84-106) where the check ends one: x has not changed since, so its
+// residual is the one at hand.
 __global__ void __launch_bounds__(AR_THREADS) gm_check_kernel(GmBatch bt) {
     const int s = blockIdx.x;
     GmState& st = bt.st[s];
     if (st.done || !st.check) return;
     __shared__ double sh[80];
+    __shared__ int restart;
     const GmView g = gm_view(bt, s);
     const int64_t n = g.n;
     const double2* b = bt.B + g.v;
@@ -542,6 +944,7 @@ __global__ void __launch_bounds__(AR_THREADS) gm_check_kernel(GmBatch bt) {
         st.xnorm = xn;
         st.error = rn / (st.anorm * xn + st.bnorm);
         st.check = 0;
+        restart = 0;
         if (st.error < st.tol) {
             st.done = 1;
             st.converged = 1;
@@ -552,10 +955,22 @@ __global__ void __launch_bounds__(AR_THREADS) gm_check_kernel(GmBatch bt) {
             // Krylov correction to x a second time at the next check.
             st.restarts += 1;
             if (st.restarts >= st.max_restarts) st.done = 1;
-            else st.need_start = 1;
+            else restart = 1;
         } else {
             st.k += 1;
         }
+    }
+    __syncthreads();
+    if (!restart) return;
+    // the next cycle starts from the residual that was just formed
+    double2* Q = bt.Q + g.q;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const double2 r = csub(b[i], W[i]);
+        Q[i] = make_double2(r.x / rn, r.y / rn);
+    }
+    if (threadIdx.x == 0) {
+        gm_cycle_state(bt, s, rn);
+        st.num_mv += 1;  // (A x counts for the check and for the start)
     }
 }
 
@@ -637,12 +1052,23 @@ void arnoldi_allow_smem(int device) {
     // a failed set throws out of call_once, which leaves the flag unset so the
     // next call tries again
     std::call_once(g_ar_smem_once[device], [] {
-        cudaError_t err = cudaFuncSetAttribute(gm_arnoldi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)AR_SMEM_CAP);
-        if (err != cudaSuccess)
-            throw Error(BEM_ERR_CUDA,
-                        std::string("cudaFuncSetAttribute(gm_arnoldi_kernel): ") + cudaGetErrorString(err));
+        auto allow = [](const void* kernel, size_t bytes, const char* name) {
+            cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (err != cudaSuccess)
+                throw Error(BEM_ERR_CUDA, std::string("cudaFuncSetAttribute(") + name + "): " + cudaGetErrorString(err));
+        };
+        allow((const void*)gm_arnoldi_kernel, AR_SMEM_CAP, "gm_arnoldi_kernel");
+        allow((const void*)gm_givens_kernel, AR_SMEM_CAP, "gm_givens_kernel");
+        allow((const void*)gm_gs_update_kernel, AR_SMEM_CAP, "gm_gs_update_kernel");
+        allow((const void*)gm_apply_small_kernel<float2, 0, 4>, small_smem<float2, 0, 4>(), "gm_apply_small_kernel");
     });
+}
+
+// Rows per Gram-Schmidt chunk: halved from 512 until the chunks cover the SMs.
+static int gs_rows_for(const GmWorkspace& ws, int nsys, int64_t n) {
+    int rows = GS_ROWS;
+    while (rows > 64 && (n + rows - 1) / rows * nsys < ws.sms) rows /= 2;
+    return rows;
 }
 
 GmWorkspace::~GmWorkspace() {
@@ -651,6 +1077,7 @@ GmWorkspace::~GmWorkspace() {
 
 void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const void* A, int64_t lda,
                 size_t mat_stride, bool fp32, bool ref_dotc) {
+    BEM_CUDA(cudaDeviceGetAttribute(&ws.sms, cudaDevAttrMultiProcessorCount, ctx.device));
     GmBatch& bt = ws.bt;
     bt.nsys = nsys;
     bt.n = n;
@@ -667,6 +1094,7 @@ void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const
     ws.cb = cb;
     bt.rb = rb;
     bt.cb = cb;
+    bt.tpr = TICKETS;
     bt.sys = nullptr;
     bt.ntiles = 0;
     ws.sys_host.clear();
@@ -675,12 +1103,13 @@ void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const
     auto carve = [&](size_t b) { size_t o = bytes; bytes += (b + 255) / 256 * 256; return o; };
     size_t oX = carve(sizeof(double2) * nsys * n), oB = carve(sizeof(double2) * nsys * n);
     size_t oQ = carve(sizeof(double2) * nsys * bt.qstride), oW = carve(sizeof(double2) * nsys * n);
-    size_t oP = carve(sizeof(double2) * nsys * cb * bt.n_pad), oT = carve(sizeof(int) * nsys * rb);
+    size_t oP = carve(sizeof(double2) * nsys * cb * bt.n_pad), oT = carve(sizeof(int) * nsys * rb * TICKETS);
     size_t oS = carve(sizeof(double2) * nsys * small), oSt = carve(sizeof(GmState) * nsys);
     size_t oN = carve(sizeof(double) * nsys * 1024 + sizeof(double) * nsys);
     ws.w_in_smem = (n * sizeof(double2) <= AR_SMEM_CAP);
     // partial sums of the whole-GPU Gram-Schmidt (forms other than the reference's)
-    const int gsc = ref_dotc ? 0 : (int)((n + GS_ROWS - 1) / GS_ROWS);
+    bt.gs_rows = gs_rows_for(ws, nsys, n);
+    const int gsc = ref_dotc ? 0 : (int)((n + bt.gs_rows - 1) / bt.gs_rows);
     size_t oG = gsc ? carve(sizeof(double2) * nsys * gsc * (m + 1)) : 0;
     size_t oGn = gsc ? carve(sizeof(double) * nsys * gsc) : 0;
     ws.memb().ensure(bytes);
@@ -699,8 +1128,8 @@ void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const
     bt.st = reinterpret_cast<GmState*>(base + oSt);
     ws.norm_part = reinterpret_cast<double*>(base + oN);
     ws.anorm = ws.norm_part + (size_t)nsys * 1024;
-    BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * nsys * rb, ctx.stream));
-    if (ws.w_in_smem) arnoldi_allow_smem(ctx.device);
+    BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * nsys * rb * TICKETS, ctx.stream));
+    arnoldi_allow_smem(ctx.device);
     if (ws.graph_exec) {
         cudaGraphExecDestroy(ws.graph_exec);
         ws.graph_exec = nullptr;
@@ -724,6 +1153,7 @@ size_t gm_prepare_external(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, i
     size_t oS = carve(sizeof(double2) * nsys * small), oSt = carve(sizeof(GmState) * nsys);
     size_t oN = carve(sizeof(double) * nsys * 1024 + sizeof(double) * nsys);
     if (bytes > capacity) return bytes;
+    BEM_CUDA(cudaDeviceGetAttribute(&ws.sms, cudaDevAttrMultiProcessorCount, ctx.device));
     GmBatch& bt = ws.bt;
     bt.nsys = nsys;
     bt.n = n;
@@ -739,6 +1169,7 @@ size_t gm_prepare_external(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, i
     ws.cb = cb;
     bt.rb = rb;
     bt.cb = cb;
+    bt.tpr = 1;  // caller memory: no finer tiling
     bt.sys = nullptr;
     bt.ntiles = 0;
     ws.sys_host.clear();
@@ -773,7 +1204,7 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     std::vector<GmSys>& sys = ws.sys_host;
     sys.assign(nsys, GmSys{});
     size_t v = 0, q = 0, p = 0, t = 0;
-    int64_t tiles = 0, nmax = 0, npmax = 0;
+    int64_t tiles = 0, tiles64 = 0, nmax = 0, npmax = 0;
     for (int s = 0; s < nsys; ++s) {
         GmSys& d = sys[s];
         d.n = ns[s];
@@ -791,11 +1222,14 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
         v += (size_t)d.n;
         q += (size_t)d.n * (m + 1);
         p += (size_t)d.cb * d.n_pad;
-        t += (size_t)d.rb;
+        t += (size_t)d.rb * TICKETS;
+        d.tile64 = tiles64;
+        tiles64 += (d.n + SMALL_ROWS - 1) / SMALL_ROWS * d.cb;
         tiles += (int64_t)d.rb * d.cb;
         nmax = std::max(nmax, d.n);
         npmax = std::max(npmax, d.n_pad);
     }
+    BEM_CUDA(cudaDeviceGetAttribute(&ws.sms, cudaDevAttrMultiProcessorCount, ctx.device));
     GmBatch& bt = ws.bt;
     bt.nsys = nsys;
     bt.n = nmax;
@@ -808,6 +1242,8 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     bt.qstride = 0;
     bt.rb = bt.cb = 0;
     bt.ntiles = tiles;
+    bt.ntiles64 = tiles64;
+    bt.tpr = TICKETS;
     ws.fp32 = fp32;
     ws.rb = ws.cb = 0;
     const size_t small = gm_small_size(m);
@@ -821,7 +1257,8 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     size_t oD = carve(sizeof(GmSys) * nsys);
     ws.w_in_smem = (nmax * sizeof(double2) <= AR_SMEM_CAP);
     // partial sums of the whole-GPU Gram-Schmidt
-    const int gsc = (int)((nmax + GS_ROWS - 1) / GS_ROWS);
+    bt.gs_rows = gs_rows_for(ws, nsys, nmax);
+    const int gsc = (int)((nmax + bt.gs_rows - 1) / bt.gs_rows);
     size_t oG = carve(sizeof(double2) * nsys * gsc * (m + 1));
     size_t oGn = carve(sizeof(double) * nsys * gsc);
     ws.memb().ensure(bytes);
@@ -844,7 +1281,7 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     BEM_CUDA(cudaMemcpyAsync(dsys, sys.data(), sizeof(GmSys) * nsys, cudaMemcpyHostToDevice, ctx.stream));
     bt.sys = dsys;
     BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * t, ctx.stream));
-    if (ws.w_in_smem) arnoldi_allow_smem(ctx.device);
+    arnoldi_allow_smem(ctx.device);
     if (ws.graph_exec) {
         cudaGraphExecDestroy(ws.graph_exec);
         ws.graph_exec = nullptr;
@@ -913,35 +1350,63 @@ void gm_init_each(Context& ctx, GmWorkspace& ws, const std::vector<double>& tol,
     ctx.sync();  // the host arrays are pageable and owned by the caller
 }
 
+// Finer tiles where they were the faster ones.  FP64: at every size (us per
+// product, wide -> finer: n = 2048 263 -> 39, 6144 312 -> 269, 16384 1820 -> 1749;
+// the wide tiles remain for caller-provided memory, which has no room for the
+// tickets).  FP32: below 1.5 wide tiles per SM (Krylov products, us of eight, wide ->
+// finer: 36 tiles 295 -> 92, 144 384 -> 373, 196 751 -> 568, 288 822 -> 870, 1152
+// 2447 -> 3069; beyond, memory bounds them and the longer columns of the wide
+// tiles read it better).
+
 static void launch_apply(Context& ctx, GmWorkspace& ws, int mode) {
     if (ws.hook) {
         ws.hook(ctx, ws, mode, ws.hook_user);
         return;
     }
-    dim3 grid = ws.bt.sys ? dim3((unsigned)ws.bt.ntiles) : dim3((unsigned)ws.rb, (unsigned)ws.cb, (unsigned)ws.bt.nsys);
-    if (ws.bt.split_lo) {
-        gm_apply_kernel<float2, 2, 4><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
+    const GmBatch& bt = ws.bt;
+    // (hooks and launches alike read the sizes from ws.bt: the same for every
+    // mode of a solve, so the three modes sum in one order)
+    const int64_t tiles = bt.sys ? bt.ntiles : (int64_t)ws.rb * ws.cb * bt.nsys;
+    const bool small = bt.tpr == TICKETS && (!ws.fp32 || 2 * tiles < 3 * ws.sms);
+    const dim3 grid = bt.sys ? dim3((unsigned)(small ? bt.ntiles64 : bt.ntiles))
+                             : dim3((unsigned)(small ? (bt.n + SMALL_ROWS - 1) / SMALL_ROWS : ws.rb),
+                                    (unsigned)ws.cb, (unsigned)bt.nsys);
+#define BEM_APPLY(T, E, U)                                                                              \
+    do {                                                                                                \
+        if (small)                                                                                      \
+            gm_apply_small_kernel<T, E, U>                                                              \
+                <<<grid, 32 * SMALL_WARPS, small_smem<T, E, U>(), ctx.stream>>>(bt, mode);              \
+        else                                                                                            \
+            gm_apply_kernel<T, E, U><<<grid, MV_THREADS, 0, ctx.stream>>>(bt, mode);                    \
+    } while (0)
+    if (bt.split_lo) {
+        BEM_APPLY(float2, 2, 4);
     } else if (ws.fp32) {
         if (mode == MV_Q) {
             // columns per load batch (loads in flight per thread), tuned per size
-            const int u = ctx.tuning.pick("gm_apply_fp32", "unroll", ws.bt.n, ws.bt.nsys, MV_UNROLL);
-            if (u == 4) gm_apply_kernel<float2, 0, 4><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
-            else if (u == 16) gm_apply_kernel<float2, 0, 16><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
-            else gm_apply_kernel<float2, 0, 8><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
+            const int u = ctx.tuning.pick("gm_apply_fp32", "unroll", bt.n, bt.nsys, MV_UNROLL);
+            if (u == 4) BEM_APPLY(float2, 0, 4);
+            else if (u == 16) BEM_APPLY(float2, 0, 16);
+            else BEM_APPLY(float2, 0, 8);
         } else {
-            gm_apply_kernel<float2, 1><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
+            BEM_APPLY(float2, 1, MV_UNROLL);
         }
     } else {
-        gm_apply_kernel<double2, 1><<<grid, MV_THREADS, 0, ctx.stream>>>(ws.bt, mode);
+        BEM_APPLY(double2, 1, MV_UNROLL);
     }
+#undef BEM_APPLY
+    BEM_CHECK_LAUNCH(&ctx);
+}
+
+void gm_launch_start(Context& ctx, GmWorkspace& ws) {
+    // outside the reference-faithful mode the residual of x = 0 is b itself
+    if (ws.bt.ref_dotc) launch_apply(ctx, ws, MV_START);
+    gm_start_kernel<<<ws.bt.nsys, AR_THREADS, 0, ctx.stream>>>(ws.bt);
     BEM_CHECK_LAUNCH(&ctx);
 }
 
 void gm_launch_iteration(Context& ctx, GmWorkspace& ws, cudaEvent_t ev_q0, cudaEvent_t ev_q1) {
-    int nsys = ws.bt.nsys;
-    launch_apply(ctx, ws, MV_START);
-    gm_start_kernel<<<nsys, AR_THREADS, 0, ctx.stream>>>(ws.bt);
-    BEM_CHECK_LAUNCH(&ctx);
+    const int nsys = ws.bt.nsys;
     if (ws.precond) {
         if (ws.ev_p0) BEM_CUDA(cudaEventRecord(ws.ev_p0, ctx.stream));
         ws.precond(ctx, ws, MV_Q, ws.precond_user);
@@ -950,8 +1415,7 @@ void gm_launch_iteration(Context& ctx, GmWorkspace& ws, cudaEvent_t ev_q0, cudaE
     if (ev_q0) BEM_CUDA(cudaEventRecord(ev_q0, ctx.stream));
     launch_apply(ctx, ws, MV_Q);
     if (ev_q1) BEM_CUDA(cudaEventRecord(ev_q1, ctx.stream));
-    const bool gs = ws.bt.gs_part && !ws.bt.ref_dotc;
-    if (gs) {
+    if (ws.bt.gs_part && !ws.bt.ref_dotc) {
         const dim3 grid((unsigned)ws.bt.gs_chunks, (unsigned)nsys);
         const size_t hsm = sizeof(double2) * (size_t)(ws.bt.m + 1);
         for (int pass = 0; pass < 2; ++pass) {
@@ -960,9 +1424,14 @@ void gm_launch_iteration(Context& ctx, GmWorkspace& ws, cudaEvent_t ev_q0, cudaE
             gm_gs_update_kernel<<<grid, GS_THREADS, hsm, ctx.stream>>>(ws.bt, pass);
             BEM_CHECK_LAUNCH(&ctx);
         }
+        const int chunks = (int)std::max<int64_t>(
+            1, std::min<int64_t>((ws.bt.n + GV_STEP_THREADS - 1) / GV_STEP_THREADS, 2 * ws.sms / nsys));
+        gm_givens_kernel<<<dim3((unsigned)chunks, (unsigned)nsys), GV_STEP_THREADS, givens_smem(ws.bt.m),
+                           ctx.stream>>>(ws.bt, chunks);
+    } else {
+        const size_t dyn = ws.w_in_smem ? (size_t)ws.bt.n * sizeof(double2) : 0;
+        gm_arnoldi_kernel<<<nsys, AR_THREADS, dyn, ctx.stream>>>(ws.bt, ws.w_in_smem ? 1 : 0);
     }
-    size_t dyn = (!gs && ws.w_in_smem) ? (size_t)ws.bt.n * sizeof(double2) : 0;
-    gm_arnoldi_kernel<<<nsys, AR_THREADS, dyn, ctx.stream>>>(ws.bt, (!gs && ws.w_in_smem) ? 1 : 0);
     BEM_CHECK_LAUNCH(&ctx);
     launch_apply(ctx, ws, MV_CHECK);
     gm_check_kernel<<<nsys, AR_THREADS, 0, ctx.stream>>>(ws.bt);
@@ -1065,6 +1534,7 @@ void gm_run(Context& ctx, GmWorkspace& ws, int chunk, int64_t max_total_iteratio
             }
         }
         gm_read_states(ctx, ws, prev);
+        gm_launch_start(ctx, ws);
         for (;;) {
             gm_launch_iteration(ctx, ws, e0, e1);
             ++issued;
@@ -1108,6 +1578,7 @@ void gm_run(Context& ctx, GmWorkspace& ws, int chunk, int64_t max_total_iteratio
         ws.graph_chunk = chunk;
         ws.graph_rounds = max_rounds;
     }
+    gm_launch_start(ctx, ws);
     if (ws.graph_loop) {
         int rounds = 0;
         BEM_CUDA(cudaMemsetAsync(ws.rounds.p, 0, sizeof(int), ctx.stream));

@@ -19,9 +19,10 @@ struct GmSys {
     size_t v_off;   // X, B, W
     size_t q_off;   // Q, Z
     size_t p_off;   // column-chunk partial sums
-    size_t t_off;   // last-CTA tickets
+    size_t t_off;   // last-CTA tickets (one per 64 rows)
     int64_t tile0;  // first CTA of this system in the flattened mat-vec grid
     int rb, cb;     // row blocks, column chunks
+    int64_t tile64; // first CTA of this system in the flattened grid of 64-row blocks
 };
 
 struct GmBatch {
@@ -48,6 +49,9 @@ struct GmBatch {
     double2* gs_part = nullptr;
     double* gs_norm = nullptr;
     int gs_chunks = 0;
+    int gs_rows = 0;     // rows per chunk
+    int tpr = 1;         // tickets per row block
+    int64_t ntiles64 = 0;  // ragged: CTAs of the flattened grid of 64-row blocks
     // split FP64 operators (refined form): every system's FP32 matrix (the
     // operator rounded to FP32, leading dimension lda) is followed, split_lo
     // float2 entries further on, by the FP32 rounding of the remainder, and
@@ -80,7 +84,7 @@ __host__ __device__ __forceinline__ GmView gm_view(const GmBatch& bt, int s) {
     } else {
         v.n = bt.n; v.lda = bt.lda; v.n_pad = bt.n_pad;
         v.a = (size_t)s * bt.mat_stride; v.v = (size_t)s * bt.n; v.q = (size_t)s * bt.qstride;
-        v.p = (size_t)s * bt.cb * bt.n_pad; v.t = (size_t)s * bt.rb;
+        v.p = (size_t)s * bt.cb * bt.n_pad; v.t = (size_t)s * bt.rb * bt.tpr;
         v.rb = bt.rb; v.cb = bt.cb;
     }
     return v;
@@ -135,6 +139,7 @@ struct GmWorkspace {
     bool fp32 = false;
     bool w_in_smem = false;
     int rb = 0, cb = 0;
+    int sms = 0;  // SMs of the device
     double* norm_part = nullptr;
     double* anorm = nullptr;
     // operator applied through `hook`: bytes streamed per system and mat-vec
@@ -166,6 +171,8 @@ void gm_init(Context& ctx, GmWorkspace& ws, double tol, int64_t max_restarts);
 // Per-system tolerance, restart count and restart length (m[s] <= batch m).
 void gm_init_each(Context& ctx, GmWorkspace& ws, const std::vector<double>& tol,
                   const std::vector<int64_t>& max_restarts, const std::vector<int>& m);
+// Start of the first cycle; once, before the iterations.
+void gm_launch_start(Context& ctx, GmWorkspace& ws);
 void gm_launch_iteration(Context& ctx, GmWorkspace& ws, cudaEvent_t ev_q0, cudaEvent_t ev_q1);
 void gm_read_states(Context& ctx, GmWorkspace& ws, std::vector<GmState>& out);
 void gm_run(Context& ctx, GmWorkspace& ws, int chunk, int64_t max_total_iterations);

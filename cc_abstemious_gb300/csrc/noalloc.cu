@@ -82,6 +82,7 @@ BEM_API bem_status bem_gmres_solve_noalloc(bem_ctx* ctx, int64_t n, const bem_cp
         gm_init(c, ws, tol, restarts);
         GmState st{};
         const int64_t limit = restarts * (int64_t)m + 1;
+        gm_launch_start(c, ws);
         for (int64_t it = 0; it < limit; ++it) {
             gm_launch_iteration(c, ws, nullptr, nullptr);
             BEM_CUDA(cudaMemcpyAsync(&st, ws.bt.st, sizeof(GmState), cudaMemcpyDeviceToHost, c.stream));

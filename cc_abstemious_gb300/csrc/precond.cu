@@ -134,6 +134,12 @@ void near_pattern(const Forest& F, int body, NearPattern& P, bool diag_only, boo
 // ---------------------------------------------------------------------------
 // Exact inverse of every diagonal leaf block, [A_cc | I] reduced by
 // Gauss-Jordan with partial pivoting in FP32, one CTA per (block, system).
+// Shared memory bounds it (each of the b steps reads and writes the block): a
+// warp owns eight rows and a lane four columns, so that the pivot row stays in
+// registers over the rows, and a step has two barriers.  (With a thread per
+// element, two divisions to find it and one thread searching the pivot: 324 us
+// for 80 blocks of 64, now 137.)  Which product of a pair is rounded is spelt out: the
+// inverse's last bits steer the iterates, so they do not depend on the compiler.
 struct PcDev {
     const int64_t *cl_off, *cl_idx, *nb_blk;
     const int32_t *nb_off, *nb_d;
@@ -166,8 +172,6 @@ __global__ void __launch_bounds__(256) pc_diag_inverse_kernel(const T* __restric
                                                               const GmSys* __restrict__ sys, PcDev pc,
                                                               float2* __restrict__ M) {
     extern __shared__ float2 aug[];  // b x 2b, row-major
-    __shared__ int s_piv;
-    __shared__ float2 fcol[PC_LEAF];  // elimination factors of the current column
     const int s = blockIdx.y;
     const int c = pc_leaf(pc, s, blockIdx.x);
     if (c < 0) return;
@@ -184,43 +188,69 @@ __global__ void __launch_bounds__(256) pc_diag_inverse_kernel(const T* __restric
         aug[i * w + j] = make_float2((float)v.x, (float)v.y);
         aug[i * w + b + j] = make_float2(i == j ? 1.f : 0.f, 0.f);
     }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int RPW = PC_LEAF / 8, CPL = 2 * PC_LEAF / 32;  // rows of a warp, columns of a lane
     __syncthreads();
     for (int col = 0; col < b; ++col) {
-        if (threadIdx.x == 0) {
-            int best = col;
-            float bv = -1.f;
-            for (int r = col; r < b; ++r) {
-                float v = fabsf(aug[r * w + col].x) + fabsf(aug[r * w + col].y);
-                if (v > bv) { bv = v; best = r; }
+        // the pivot, found by every warp for itself: largest |re| + |im|, the
+        // first of equals (a NaN is never taken)
+        int pr = col;
+        unsigned top = 0;
+        for (int q = 0; q < PC_LEAF / 32; ++q) {
+            const int r = lane + 32 * q;
+            unsigned key = 0;
+            if (r >= col && r < b) {
+                const float v = fabsf(aug[r * w + col].x) + fabsf(aug[r * w + col].y);
+                if (v >= 0.f) key = __float_as_uint(v) + 1;
             }
-            s_piv = best;
+            const unsigned m = __reduce_max_sync(0xffffffffu, key);
+            if (m > top) {
+                top = m;
+                pr = 32 * q + __ffs(__ballot_sync(0xffffffffu, key == m)) - 1;
+            }
         }
-        __syncthreads();
-        const int pr = s_piv;
-        if (pr != col)
-            for (int t = threadIdx.x; t < w; t += blockDim.x) {
-                float2 a = aug[col * w + t];
-                aug[col * w + t] = aug[pr * w + t];
-                aug[pr * w + t] = a;
-            }
-        __syncthreads();
-        const float2 d = aug[col * w + col];
-        const float dn = d.x * d.x + d.y * d.y;
+        const float2 d = aug[pr * w + col];
+        const float dn = __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y));
         const float2 inv = dn > 0.f ? make_float2(d.x / dn, -d.y / dn) : make_float2(0.f, 0.f);
-        __syncthreads();
-        for (int t = threadIdx.x; t < w; t += blockDim.x) aug[col * w + t] = fmul(aug[col * w + t], inv);
-        for (int r = threadIdx.x; r < b; r += blockDim.x) fcol[r] = aug[r * w + col];
-        __syncthreads();
-        for (int t = threadIdx.x; t < b * w; t += blockDim.x) {
-            int r = t / w, j = t % w;
-            if (r == col) continue;
-            float2 f = fcol[r];
-            float2 v = aug[r * w + j];
-            float2 u = aug[col * w + j];
-            aug[r * w + j] = make_float2(v.x - (f.x * u.x - f.y * u.y), v.y - (f.x * u.y + f.y * u.x));
+        // the new row col (u), the row that moves to pr, this warp's factors;
+        // columns up to col are not read again
+        float2 u[CPL], moved[CPL], f[RPW];
+#pragma unroll
+        for (int q = 0; q < CPL; ++q) {
+            const int j = lane + 32 * q;
+            u[q] = moved[q] = make_float2(0.f, 0.f);
+            if (j > col && j < w) {
+                const float2 a = aug[pr * w + j];
+                u[q] = make_float2(__fmaf_rn(a.x, inv.x, -__fmul_rn(a.y, inv.y)),
+                                   __fmaf_rn(a.x, inv.y, __fmul_rn(a.y, inv.x)));
+                moved[q] = aug[col * w + j];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < RPW; ++q) {
+            const int r = warp + 8 * q;
+            f[q] = r < b ? aug[(r == pr ? col : r) * w + col] : make_float2(0.f, 0.f);
         }
         __syncthreads();
-        // the pivot column of the other rows was consumed; zero it for clarity
+#pragma unroll
+        for (int q = 0; q < RPW; ++q) {
+            const int r = warp + 8 * q;
+            if (r >= b) break;
+#pragma unroll
+            for (int e = 0; e < CPL; ++e) {
+                const int j = lane + 32 * e;
+                if (j <= col || j >= w) continue;
+                if (r == col) {
+                    aug[r * w + j] = u[e];
+                } else {
+                    const float2 v = r == pr ? moved[e] : aug[r * w + j];
+                    aug[r * w + j] =
+                        make_float2(v.x - __fmaf_rn(f[q].x, u[e].x, -__fmul_rn(f[q].y, u[e].y)),
+                                    v.y - __fmaf_rn(f[q].y, u[e].x, __fmul_rn(f[q].x, u[e].y)));
+                }
+            }
+        }
+        __syncthreads();
     }
     float2* Mo = M + pc_moff(pc, s) + pc.nb_blk[pc.nb_off[c]];  // first neighbour is the block itself
     for (int t = threadIdx.x; t < b * b; t += blockDim.x) {
@@ -229,54 +259,86 @@ __global__ void __launch_bounds__(256) pc_diag_inverse_kernel(const T* __restric
     }
 }
 
-// z[rows of c] = sum over near d of M_cd q[rows of d]; one CTA per (leaf, system).
-__device__ __forceinline__ void pc_block_apply(int c, const int64_t* cl_off, const int64_t* cl_idx,
+// z[rows of c] = sum over near d of M_cd q[rows of d]; two CTAs per (leaf,
+// system), 32 rows each, whose eight warps share the columns of every block.
+//
+// FP64 instructions bound it (65 clocks per warp and SM quarter), so the
+// widening of M is done in bits and the columns are spread over the quarters
+// (80 blocks of 64: 17 us with one CTA of two warps per leaf and conversion
+// instructions, now 8).
+constexpr int PC_APPLY_THREADS = 256, PC_APPLY_ROWS = 32;
+
+// A float as a double, without the conversion instruction where it is normal.
+__device__ __forceinline__ double pc_wide(float f) {
+    const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xff;
+    if (e == 0 || e == 0xff) return (double)f;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023 - 127) << 20))),
+                            (int)(b << 29));
+}
+
+__device__ __forceinline__ void pc_block_apply(int c, int half, const int64_t* cl_off, const int64_t* cl_idx,
                                                const int32_t* nb_off, const int32_t* nb_d, const int64_t* nb_blk,
                                                const float2* Ms, const double2* q, double2* z, int use_offdiag) {
-    __shared__ double2 qs[PC_LEAF];
+    constexpr int WARPS = PC_APPLY_THREADS / 32, CPW = PC_LEAF / WARPS;  // columns of a warp
+    __shared__ double2 qs[WARPS][CPW];
+    __shared__ double2 sums[WARPS][PC_APPLY_ROWS];
     const int64_t oc = cl_off[c];
     const int bc = (int)(cl_off[c + 1] - oc);
+    const int r0 = half * PC_APPLY_ROWS;
+    if (r0 >= bc) return;
     double2 acc = make_double2(0, 0);
-    const int i = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = r0 + lane, j0 = warp * CPW;
     const int nend = use_offdiag ? nb_off[c + 1] : nb_off[c] + 1;
     for (int t = nb_off[c]; t < nend; ++t) {
         const int d = nb_d[t];
         const int64_t od = cl_off[d];
         const int bd = (int)(cl_off[d + 1] - od);
-        __syncthreads();
-        if (i < bd) qs[i] = q[cl_idx[od + i]];
-        __syncthreads();
-        if (i < bc) {
-            const float2* blk = Ms + nb_blk[t];
-            for (int j = 0; j < bd; ++j) {
-                float2 m = blk[(size_t)j * bc + i];
-                cfma(acc, make_double2(m.x, m.y), qs[j]);
-            }
-        }
+        const float2* blk = Ms + nb_blk[t];
+        float2 m[CPW];
+#pragma unroll
+        for (int j = 0; j < CPW; ++j)
+            m[j] = i < bc && j0 + j < bd ? blk[(size_t)(j0 + j) * bc + i] : make_float2(0.f, 0.f);
+        __syncwarp();
+        if (lane < CPW) qs[warp][lane] = j0 + lane < bd ? q[cl_idx[od + j0 + lane]] : make_double2(0, 0);
+        __syncwarp();
+        const int jn = min(CPW, bd - j0);
+#pragma unroll
+        for (int j = 0; j < CPW; ++j)
+            if (j < jn) cfma(acc, make_double2(pc_wide(m[j].x), pc_wide(m[j].y)), qs[warp][j]);
     }
-    if (i < bc) z[cl_idx[oc + i]] = acc;
+    sums[warp][lane] = acc;
+    __syncthreads();
+    if (threadIdx.x < 2 * PC_APPLY_ROWS) {
+        const int row = threadIdx.x >> 1;
+        const double* f = reinterpret_cast<const double*>(sums) + threadIdx.x;
+        double t = f[0];
+#pragma unroll
+        for (int g = 1; g < WARPS; ++g) t += f[g * 2 * PC_APPLY_ROWS];
+        if (r0 + row < bc) reinterpret_cast<double*>(z + cl_idx[oc + r0 + row])[threadIdx.x & 1] = t;
+    }
 }
 
-__global__ void __launch_bounds__(PC_LEAF) pc_apply_gmres_kernel(PcDev pc, GmBatch bt) {
+__global__ void __launch_bounds__(PC_APPLY_THREADS) pc_apply_gmres_kernel(PcDev pc, GmBatch bt) {
     const int s = blockIdx.y;
     const GmState& st = bt.st[s];
     if (!gm_apply_active(bt, st, MV_Q)) return;
-    const int c = pc_leaf(pc, s, blockIdx.x);
+    const int c = pc_leaf(pc, s, blockIdx.x >> 1);
     if (c < 0) return;
     const GmView g = gm_view(bt, s);
     const double2* q = bt.Q + g.q + (size_t)st.k * g.n;
     double2* z = bt.Z + g.q + (size_t)st.k * g.n;
     const int off = pc.offdiag && (!pc.sys_off || pc.sys_off[s]);
-    pc_block_apply(c, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s), q, z, off);
+    pc_block_apply(c, blockIdx.x & 1, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s), q, z,
+                   off);
 }
 
 // Probe form: Y[:, q] = M_s Z[:, q] for nprobe vectors (training).
-__global__ void __launch_bounds__(PC_LEAF) pc_apply_probes_kernel(PcDev pc, int s, const double2* __restrict__ Zp,
+__global__ void __launch_bounds__(PC_APPLY_THREADS) pc_apply_probes_kernel(PcDev pc, int s, const double2* __restrict__ Zp,
                                                                   double2* __restrict__ Yp, int64_t n) {
     const int q = blockIdx.y;
-    const int c = pc_leaf(pc, s, blockIdx.x);
+    const int c = pc_leaf(pc, s, blockIdx.x >> 1);
     if (c < 0) return;
-    pc_block_apply(c, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s),
+    pc_block_apply(c, blockIdx.x & 1, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s),
                    Zp + (size_t)q * n, Yp + (size_t)q * n, pc.offdiag);
 }
 
@@ -744,8 +806,8 @@ struct PcHookData {
 static void pc_hook(Context& c, GmWorkspace& ws, int mode, void* user) {
     (void)mode;
     PcHookData& h = *static_cast<PcHookData*>(user);
-    dim3 grid((unsigned)(h.data.multi ? h.data.nc_max : h.data.pat.nc), (unsigned)ws.bt.nsys);
-    pc_apply_gmres_kernel<<<grid, PC_LEAF, 0, c.stream>>>(h.data.dev(h.use_off ? 1 : 0), ws.bt);
+    dim3 grid((unsigned)(2 * (h.data.multi ? h.data.nc_max : h.data.pat.nc)), (unsigned)ws.bt.nsys);
+    pc_apply_gmres_kernel<<<grid, PC_APPLY_THREADS, 0, c.stream>>>(h.data.dev(h.use_off ? 1 : 0), ws.bt);
     BEM_CHECK_LAUNCH(&c);
 }
 
@@ -764,15 +826,15 @@ struct GateSys {
 };
 
 // Y = M_s Z for every system s (blockIdx.z) and probe (blockIdx.y).
-__global__ void __launch_bounds__(PC_LEAF) gate_apply_kernel(PcDev pc, const GateSys* __restrict__ gs,
-                                                             const double2* __restrict__ Z, double2* __restrict__ Y) {
+__global__ void __launch_bounds__(PC_APPLY_THREADS) gate_apply_kernel(PcDev pc, const GateSys* __restrict__ gs,
+                                                                      const double2* __restrict__ Z, double2* __restrict__ Y) {
     const int s = blockIdx.z, q = blockIdx.y;
-    const int c = pc_leaf(pc, s, blockIdx.x);
+    const int c = pc_leaf(pc, s, blockIdx.x >> 1);
     if (c < 0) return;
     const GateSys g = gs[s];
     const size_t v = (size_t)g.voff + (size_t)q * g.n;
-    pc_block_apply(c, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s), Z + v, Y + v,
-                   pc.offdiag);
+    pc_block_apply(c, blockIdx.x & 1, pc.cl_off, pc.cl_idx, pc.nb_off, pc.nb_d, pc.nb_blk, pc.M + pc_moff(pc, s), Z + v,
+                   Y + v, pc.offdiag);
 }
 
 // W = A_s Y and the residual partials |W - Z|^2, |Z|^2 of every system and
@@ -844,7 +906,8 @@ static int learned_gate(Context& c, PcData& d, GmWorkspace& ws, uint64_t seed) {
     BEM_CHECK_LAUNCH(&c);
     const int nleaf = d.multi ? d.nc_max : d.pat.nc;
     for (int use = 0; use < 2; ++use) {
-        gate_apply_kernel<<<dim3((unsigned)nleaf, (unsigned)GATE_PROBES, (unsigned)nsys), PC_LEAF, 0, c.stream>>>(
+        gate_apply_kernel<<<dim3((unsigned)(2 * nleaf), (unsigned)GATE_PROBES, (unsigned)nsys),
+                            PC_APPLY_THREADS, 0, c.stream>>>(
             d.dev(use), dgs.as<GateSys>(), Z.as<double2>(), Y.as<double2>());
         BEM_CHECK_LAUNCH(&c);
         gate_residual_kernel<<<dim3((unsigned)((nmax + 127) / 128), (unsigned)GATE_PROBES, (unsigned)nsys), 128, 0,
@@ -1143,7 +1206,7 @@ double learned_train(Context& c, std::vector<Problem*>& probs, int steps, int np
             probes_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, c.stream>>>(tot, seed * 104729 + (uint64_t)f,
                                                                                 Z.as<double2>());
             BEM_CHECK_LAUNCH(&c);
-            pc_apply_probes_kernel<<<dim3((unsigned)b.pc.pat.nc, (unsigned)nprobe), PC_LEAF, 0, c.stream>>>(
+            pc_apply_probes_kernel<<<dim3((unsigned)(2 * b.pc.pat.nc), (unsigned)nprobe), PC_APPLY_THREADS, 0, c.stream>>>(
                 b.pc.dev(1), f, Z.as<double2>(), Y.as<double2>(), n);
             BEM_CHECK_LAUNCH(&c);
             probe_matvec_kernel<<<dim3((unsigned)((n + 127) / 128), (unsigned)nprobe), 128, 0, c.stream>>>(
@@ -1185,7 +1248,7 @@ double learned_train(Context& c, std::vector<Problem*>& probs, int steps, int np
         probes_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, c.stream>>>(tot, seed * 7919 + (uint64_t)it,
                                                                             Z.as<double2>());
         BEM_CHECK_LAUNCH(&c);
-        pc_apply_probes_kernel<<<dim3((unsigned)b.pc.pat.nc, (unsigned)nprobe), PC_LEAF, 0, c.stream>>>(
+        pc_apply_probes_kernel<<<dim3((unsigned)(2 * b.pc.pat.nc), (unsigned)nprobe), PC_APPLY_THREADS, 0, c.stream>>>(
             b.pc.dev(1), f, Z.as<double2>(), Y.as<double2>(), n);
         BEM_CHECK_LAUNCH(&c);
         probe_matvec_kernel<<<dim3((unsigned)((n + 127) / 128), (unsigned)nprobe), 128, 0, c.stream>>>(
