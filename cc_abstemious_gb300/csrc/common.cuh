@@ -227,6 +227,7 @@ struct Context {
     DevBuf w_piv;     // the plain form's FP64 LU: row order, diagonal blocks' inverses
     DevBuf w_lu64;    // its trailing update's digit images
     int lu64_cluster = 0;  // largest cluster its panels run on (0: not asked yet)
+    int gm_cluster = 0;    // the same for the Arnoldi step of the reference's form
     // results of the last bem_run
     std::vector<double> last_phi, last_vn;
     int64_t last_n = 0, last_nf = 0;

@@ -17,6 +17,7 @@
 // orthogonalise across the whole GPU (classical Gram-Schmidt twice).
 #include <mutex>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "complex.cuh"
 #include "gmres.cuh"
@@ -32,7 +33,7 @@ constexpr int MV_COLS = 512;
 constexpr int SMALL_ROWS = 64;
 constexpr int TICKETS = MV_ROWS / SMALL_ROWS;
 constexpr int AR_THREADS = 1024;
-// largest Krylov vector kept in the Arnoldi kernel's shared memory (n <= 12800)
+// dynamic shared memory of the Arnoldi kernels
 constexpr size_t AR_SMEM_CAP = 200 * 1024;
 
 __device__ __forceinline__ bool mv_active(const GmState& s, int mode) {
@@ -665,6 +666,133 @@ __global__ void __launch_bounds__(GS_THREADS) gm_gs_update_kernel(GmBatch bt, in
     }
 }
 
+// The small part of an Arnoldi step, in shared memory: the new column h of H
+// turned by the earlier rotations, the new one, the residual estimate and, where
+// the step is checked, y (gmres.rs:146-157, 178-202).
+struct GmStep {
+    double2 *h, *a, *cs, *sn;  // k + 1 entries each
+    double2 *dinv, *y;         // of the triangular solve, in the place of a and cs
+    double2 *cs_k, *sn_k, *beta_k, *beta_k1;
+    double *scale, *error;
+    int* chk;
+};
+constexpr size_t gm_step_smem(int m) { return sizeof(double2) * 4 * (size_t)(m + 1); }
+#define GM_STEP_SHARED(name, smem)                                                                         \
+    __shared__ double2 name##_z[4];                                                                        \
+    __shared__ double name##_d[2];                                                                         \
+    __shared__ int name##_i;                                                                               \
+    GmStep name;                                                                                           \
+    name.h = smem; name.a = name.h + (bt.m + 1); name.cs = name.a + (bt.m + 1);                            \
+    name.sn = name.cs + (bt.m + 1); name.dinv = name.a; name.y = name.cs;                                  \
+    name.cs_k = name##_z; name.sn_k = name##_z + 1; name.beta_k = name##_z + 2; name.beta_k1 = name##_z + 3; \
+    name.scale = name##_d; name.error = name##_d + 1; name.chk = &name##_i
+
+// One warp; nn = |w|^2.
+__device__ __forceinline__ void gm_rotate(const GmStep& t, const GmState& st, const GmSmall& sm, double nn) {
+    const int k = st.k, lane = threadIdx.x & 31;
+    // a_i = the entry rotation i meets: a_0 = h_0, a_{i+1} = -conj(sn_i) a_i + cs_i h_{i+1}
+    // (lane 0 the real, lane 1 the imaginary part; cs_i h_{i+1} is laid down beforehand)
+    for (int i = lane; i < k; i += 32)
+        t.a[i + 1] = make_double2(t.cs[i].x * t.h[i + 1].x, t.cs[i].x * t.h[i + 1].y);
+    __syncwarp();
+    double2 cur = t.h[0];
+    for (int i = 0; i < k; ++i) {
+        const double2 ss = t.sn[i], b = t.a[i + 1];
+        if (lane == 0) t.a[i] = cur;
+        const double p = lane ? cur.y : cur.x, q = lane ? -cur.x : cur.y;
+        const double v = fma(-ss.y, q, fma(-ss.x, p, lane ? b.y : b.x));
+        cur.x = __shfl_sync(0xffffffffu, v, 0);
+        cur.y = __shfl_sync(0xffffffffu, v, 1);
+    }
+    __syncwarp();
+    // the rotated entries, off the chain
+    for (int i = lane; i < k; i += 32)
+        t.a[i] = cadd(make_double2(t.cs[i].x * t.a[i].x, t.cs[i].x * t.a[i].y), cmul(t.sn[i], t.h[i + 1]));
+    __syncwarp();
+    for (int i = lane; i < k; i += 32) t.h[i] = t.a[i];
+    // new rotation (LAWN 148): v1 = cur, v2 = |w| real.  The roots and the
+    // quotients are taken side by side, a lane each: one costs 600 clocks.
+    const double c2 = cnorm2(cur);
+    double rt = sqrt(lane == 0 ? nn : lane == 1 ? c2 : c2 + nn);
+    if (lane == 1 && !(c2 > 1e-280)) rt = cabs_(cur);
+    const double hn = __shfl_sync(0xffffffffu, rt, 0), a1 = __shfl_sync(0xffffffffu, rt, 1),
+                 r = __shfl_sync(0xffffffffu, rt, 2);
+    const double qt = (lane == 0 ? cur.x : lane == 1 ? cur.y : lane == 2 ? a1 : lane == 3 ? hn : 1.0) /
+                      (lane < 2 ? a1 : lane < 4 ? r : hn);
+    double2 signf = make_double2(__shfl_sync(0xffffffffu, qt, 0), __shfl_sync(0xffffffffu, qt, 1));
+    const double c0 = __shfl_sync(0xffffffffu, qt, 2), t0 = __shfl_sync(0xffffffffu, qt, 3),
+                 sc = __shfl_sync(0xffffffffu, qt, 4);
+    if (cur.x == 0.0 && cur.y == 0.0) signf = make_double2(1.0, 0.0);
+    const double2 s0 = make_double2(signf.x * t0, signf.y * t0);
+    const double2 bk = sm.beta[k];
+    const double2 b1 = cmul(cneg(cconj(s0)), bk), b0 = make_double2(bk.x * c0, bk.y * c0);
+    if (lane == 0) {
+        t.h[k] = cadd(make_double2(c0 * cur.x, c0 * cur.y), make_double2(s0.x * hn, s0.y * hn));
+        *t.scale = sc;
+        *t.cs_k = make_double2(c0, 0.0);
+        *t.sn_k = s0;
+        *t.beta_k = b0;
+        *t.beta_k1 = b1;
+        *t.error = cabs_(b1) / (st.anorm * st.xnorm + st.bnorm);
+        *t.chk = (*t.error < st.tol) || (k == st.m - 1);
+    }
+}
+
+// The whole CTA: y = H_k^{-1} beta_k, column by column from the last (H_k is
+// upper triangular after the rotations).
+__device__ __forceinline__ void gm_solve_y(const GmStep& t, const GmSmall& sm, int k, int m) {
+    for (int i = threadIdx.x; i <= k; i += blockDim.x)
+        t.dinv[i] = cdiv(make_double2(1.0, 0.0), i == k ? t.h[k] : sm.H[(size_t)i * (m + 1) + i]);
+    for (int i = threadIdx.x; i <= k; i += blockDim.x) t.y[i] = i == k ? *t.beta_k : sm.beta[i];
+    __syncthreads();
+    if (threadIdx.x < 32)
+        for (int i = k; i >= 0; --i) {
+            const double2 yi = cmul(t.y[i], t.dinv[i]);
+            __syncwarp();
+            if (threadIdx.x == 0) t.y[i] = yi;
+            for (int r = threadIdx.x; r < i; r += 32) {
+                const double2 e = i == k ? t.h[r] : sm.H[(size_t)i * (m + 1) + r];
+                t.y[r] = csub(t.y[r], cmul(e, yi));
+            }
+            __syncwarp();
+        }
+    __syncthreads();
+}
+
+// x += Q_k y, or Z_k y with flexible right preconditioning, rows l0 .. l1.
+__device__ __forceinline__ void gm_add_correction(const GmBatch& bt, const GmView& g, const double2* y, int k,
+                                                  int64_t l0, int64_t l1) {
+    double2* x = bt.X + g.v;
+    const double2* Zs = (bt.Z ? bt.Z : bt.Q) + g.q;
+    for (int64_t l = l0 + threadIdx.x; l < l1; l += blockDim.x) {
+        double2 v = x[l];
+        for (int j = 0; j <= k; ++j) cfma(v, Zs[(size_t)j * g.n + l], y[j]);
+        x[l] = v;
+    }
+}
+
+// One CTA, when every other one is done with the state.
+__device__ __forceinline__ void gm_record(const GmStep& t, GmState& st, const GmSmall& sm, int m) {
+    const int k = st.k;
+    for (int i = threadIdx.x; i <= k; i += blockDim.x) {
+        sm.H[(size_t)k * (m + 1) + i] = t.h[i];
+        if (*t.chk) sm.y[i] = t.y[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sm.H[(size_t)k * (m + 1) + k + 1] = make_double2(0, 0);
+        sm.cs[k] = *t.cs_k;
+        sm.sn[k] = *t.sn_k;
+        sm.beta[k] = *t.beta_k;
+        sm.beta[k + 1] = *t.beta_k1;
+        st.error = *t.error;
+        st.num_mv += 1;
+        st.iterations += 1;
+        st.check = *t.chk;
+        if (!*t.chk) st.k = k + 1;
+    }
+}
+
 // The rest of an Arnoldi step after the Gram-Schmidt kernels: Givens rotations
 // (gmres.rs:178-202), residual estimate and, when the estimate passes or the
 // cycle ends, y = H_k^{-1} beta_k (gmres.rs:146-157); q_{k+1} = w / |w| and
@@ -678,121 +806,42 @@ __global__ void __launch_bounds__(GS_THREADS) gm_gs_update_kernel(GmBatch bt, in
 // took 36 us per step at n = 1280, k up to 30, and x += Z y another 40 us on
 // one SM; now 12.5 us on average with the update.)
 constexpr int GV_STEP_THREADS = 256;
-constexpr size_t givens_smem(int m) { return sizeof(double2) * 4 * (size_t)(m + 1); }
 __global__ void __launch_bounds__(GV_STEP_THREADS) gm_givens_kernel(GmBatch bt, int chunks) {
     const int s = blockIdx.y;
     GmState& st = bt.st[s];
     if (!gm_arnoldi_active(st)) return;
     extern __shared__ double2 sh2[];
+    __shared__ int last;
+    GM_STEP_SHARED(t, sh2);
     const GmView g = gm_view(bt, s);
     const int64_t n = g.n;
-    const int k = st.k, m = bt.m, tid = threadIdx.x, lane = tid & 31;
-    const double anorm = st.anorm, xnorm = st.xnorm, bnorm = st.bnorm, tol = st.tol;
-    const int last_k = st.m - 1;
-    GmSmall sm = gm_small(bt, s);
-    double2 *h = sh2, *a = h + (m + 1), *cs = a + (m + 1), *sn = cs + (m + 1);
-    double2 *dinv = a, *y = cs;  // (in the triangular solve)
-    __shared__ double scale_s, error_s;
-    __shared__ double2 cs_k, sn_k, beta_k, beta_k1;
-    __shared__ int chk_s, last;
-    for (int i = tid; i <= k; i += GV_STEP_THREADS) h[i] = sm.hk1[i];
+    const int k = st.k, m = bt.m, tid = threadIdx.x;
+    const GmSmall sm = gm_small(bt, s);
+    for (int i = tid; i <= k; i += GV_STEP_THREADS) t.h[i] = sm.hk1[i];
     for (int i = tid; i < k; i += GV_STEP_THREADS) {
-        cs[i] = sm.cs[i];
-        sn[i] = sm.sn[i];
+        t.cs[i] = sm.cs[i];
+        t.sn[i] = sm.sn[i];
     }
     __syncthreads();
     if (tid < 32) {
         double nn = 0;
         const int nch = (int)((n + bt.gs_rows - 1) / bt.gs_rows);  // this system's chunks (ragged batches)
-        for (int c = lane; c < nch; c += 32) nn += bt.gs_norm[(size_t)s * bt.gs_chunks + c];
+        for (int c = tid; c < nch; c += 32) nn += bt.gs_norm[(size_t)s * bt.gs_chunks + c];
         for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
-        // a_i = the entry rotation i meets: a_0 = h_0, a_{i+1} = -conj(sn_i) a_i + cs_i h_{i+1}
-        // (lane 0 the real, lane 1 the imaginary part)
-        double2 cur = h[0];
-        for (int i = 0; i < k; ++i) {
-            if (lane == 0) a[i] = cur;
-            const double2 cc = cs[i], ss = sn[i], b = h[i + 1];
-            const double base = lane ? b.y : b.x, p = lane ? cur.y : cur.x, q = lane ? -cur.x : cur.y;
-            const double v = fma(-ss.y, q, fma(-ss.x, p, cc.x * base));
-            cur.x = __shfl_sync(0xffffffffu, v, 0);
-            cur.y = __shfl_sync(0xffffffffu, v, 1);
-        }
-        __syncwarp();
-        // the rotated entries, off the chain
-        for (int i = lane; i < k; i += 32) {
-            const double2 t = cadd(make_double2(cs[i].x * a[i].x, cs[i].x * a[i].y), cmul(sn[i], h[i + 1]));
-            a[i] = t;  // (held until every lane has read h)
-        }
-        __syncwarp();
-        for (int i = lane; i < k; i += 32) h[i] = a[i];
-        // new rotation (LAWN 148): v1 = cur, v2 = |w| real.  The roots and the
-        // quotients are taken side by side, a lane each: one costs 600 clocks.
-        const double c2 = cnorm2(cur);
-        double rt = sqrt(lane == 0 ? nn : lane == 1 ? c2 : c2 + nn);
-        if (lane == 1 && !(c2 > 1e-280)) rt = cabs_(cur);
-        const double hn = __shfl_sync(0xffffffffu, rt, 0), a1 = __shfl_sync(0xffffffffu, rt, 1),
-                     r = __shfl_sync(0xffffffffu, rt, 2);
-        const double qt = (lane == 0 ? cur.x : lane == 1 ? cur.y : lane == 2 ? a1 : lane == 3 ? hn : 1.0) /
-                          (lane < 2 ? a1 : lane < 4 ? r : hn);
-        double2 signf = make_double2(__shfl_sync(0xffffffffu, qt, 0), __shfl_sync(0xffffffffu, qt, 1));
-        const double c0 = __shfl_sync(0xffffffffu, qt, 2), t0 = __shfl_sync(0xffffffffu, qt, 3),
-                     sc = __shfl_sync(0xffffffffu, qt, 4);
-        if (cur.x == 0.0 && cur.y == 0.0) signf = make_double2(1.0, 0.0);
-        const double2 s0 = make_double2(signf.x * t0, signf.y * t0);
-        const double2 bk = sm.beta[k];
-        const double2 b1 = cmul(cneg(cconj(s0)), bk), b0 = make_double2(bk.x * c0, bk.y * c0);
-        if (lane == 0) {
-            h[k] = cadd(make_double2(c0 * cur.x, c0 * cur.y), make_double2(s0.x * hn, s0.y * hn));
-            scale_s = sc;
-            cs_k = make_double2(c0, 0.0);
-            sn_k = s0;
-            beta_k = b0;
-            beta_k1 = b1;
-            error_s = cabs_(b1) / (anorm * xnorm + bnorm);
-            chk_s = (error_s < tol) || (k == last_k);
-        }
+        gm_rotate(t, st, sm, nn);
     }
     __syncthreads();
-    if (chk_s) {
-        // column by column from the last: y_i, then its multiple off the rest
-        if (tid <= k) dinv[tid] = cdiv(make_double2(1.0, 0.0), tid == k ? h[k] : sm.H[(size_t)tid * (m + 1) + tid]);
-        for (int i = tid + GV_STEP_THREADS; i <= k; i += GV_STEP_THREADS)
-            dinv[i] = cdiv(make_double2(1.0, 0.0), i == k ? h[k] : sm.H[(size_t)i * (m + 1) + i]);
-        for (int i = tid; i <= k; i += GV_STEP_THREADS) y[i] = i == k ? beta_k : sm.beta[i];
-        __syncthreads();
-        if (tid < 32)
-            for (int i = k; i >= 0; --i) {
-                const double2 yi = cmul(y[i], dinv[i]);
-                __syncwarp();
-                if (lane == 0) y[i] = yi;
-                for (int r = lane; r < i; r += 32) {
-                    const double2 e = i == k ? h[r] : sm.H[(size_t)i * (m + 1) + r];
-                    y[r] = csub(y[r], cmul(e, yi));
-                }
-                __syncwarp();
-            }
-        __syncthreads();
-    }
+    if (*t.chk) gm_solve_y(t, sm, k, m);
     // this CTA's rows
     const int64_t per = (n + chunks - 1) / chunks, l0 = (int64_t)blockIdx.x * per, l1 = min(n, l0 + per);
-    const double sc = scale_s;
+    const double sc = *t.scale;
     const double2* Wg = bt.W + g.v;
-    double2* Q = bt.Q + g.q;
-    double2* qk1 = Q + (size_t)(k + 1) * n;
+    double2* qk1 = bt.Q + g.q + (size_t)(k + 1) * n;
     for (int64_t l = l0 + tid; l < l1; l += GV_STEP_THREADS) {
         const double2 w = Wg[l];
         qk1[l] = make_double2(w.x * sc, w.y * sc);
     }
-    if (chk_s) {
-        // x += Q_k y, or Z_k y with flexible right preconditioning
-        double2* x = bt.X + g.v;
-        const double2* Zs = bt.Z ? bt.Z + g.q : Q;
-        for (int64_t l = l0 + tid; l < l1; l += GV_STEP_THREADS) {
-            double2 v = x[l];
-            for (int j = 0; j <= k; ++j) cfma(v, Zs[(size_t)j * n + l], y[j]);
-            x[l] = v;
-        }
-    }
+    if (*t.chk) gm_add_correction(bt, g, t.y, k, l0, l1);
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -801,122 +850,150 @@ __global__ void __launch_bounds__(GV_STEP_THREADS) gm_givens_kernel(GmBatch bt, 
         if (last) *tk = 0;
     }
     __syncthreads();
-    if (!last) return;
-    for (int i = tid; i <= k; i += GV_STEP_THREADS) {
-        sm.H[(size_t)k * (m + 1) + i] = h[i];
-        if (chk_s) sm.y[i] = y[i];
-    }
-    if (tid == 0) {
-        sm.H[(size_t)k * (m + 1) + k + 1] = make_double2(0, 0);
-        sm.cs[k] = cs_k;
-        sm.sn[k] = sn_k;
-        sm.beta[k] = beta_k;
-        sm.beta[k + 1] = beta_k1;
-        st.error = error_s;
-        st.num_mv += 1;
-        st.iterations += 1;
-        st.check = chk_s;
-        if (!chk_s) st.k = k + 1;
-    }
+    if (last) gm_record(t, st, sm, m);
 }
 
-// Arnoldi step k with modified Gram-Schmidt (gmres.rs:158-176), Givens
-// update (gmres.rs:178-202), residual estimate and, when the estimate passes
-// or the cycle ends, the solution update x += Q_k H_k^{-1} beta_k
-// (gmres.rs:146-157).  The Krylov vector w lives in shared memory when it
-// fits (`w_in_smem`), else in the W buffer.
-__global__ void __launch_bounds__(AR_THREADS) gm_arnoldi_kernel(GmBatch bt, int w_in_smem) {
-    const int s = blockIdx.x;
+// Arnoldi step k of the reference's form: modified Gram-Schmidt (gmres.rs:158-176)
+// with its product conj(w)^T q, and the small part as above.  One cluster per
+// system; a CTA holds its share of w in shared memory where it fits
+// (`w_in_smem`), and every coefficient is one exchange: each warp sends its part
+// of the sum to all CTAs, which add the parts in one order.  Two slots by parity
+// are enough, since nobody sends for step i + 1 before it has read step i.
+//
+// FP64 instructions bound it: subtracting h_i q_i and the next product are one
+// pass over the rows, with q_{i+1} loaded before the wait.  (One CTA with two
+// block-wide reductions per coefficient: 23 us each at n = 6144; now 3.5 us, 16
+// steps 3.15 -> 0.50 ms.)
+constexpr int MG_THREADS = 128, MG_WARPS = MG_THREADS / 32, MG_UNROLL = 4;
+
+__global__ void __launch_bounds__(MG_THREADS) gm_arnoldi_kernel(GmBatch bt, int w_in_smem, int cluster) {
+    const int s = blockIdx.x / cluster, rank = blockIdx.x % cluster;
     GmState& st = bt.st[s];
-    if (st.done || st.need_start || st.check) return;
-    extern __shared__ double2 wsh[];
-    __shared__ double sh[80];
-    __shared__ double2 hsh;
+    if (!gm_arnoldi_active(st)) return;
+    extern __shared__ double2 sh2[];
+    __shared__ double2 slot[2][MAX_CLUSTER * MG_WARPS];
+    __shared__ uint64_t mb[2];
+    GM_STEP_SHARED(t, sh2);
     const GmView g = gm_view(bt, s);
     const int64_t n = g.n;
-    const int k = st.k;
-    const int m = bt.m;
-    double2* Q = bt.Q + g.q;
-    double2* Wg = bt.W + g.v;
-    double2* w = w_in_smem ? wsh : Wg;
-    GmSmall sm = gm_small(bt, s);
-    double2* qk1 = Q + (size_t)(k + 1) * n;
+    const int k = st.k, m = bt.m, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const GmSmall sm = gm_small(bt, s);
+    const int64_t per = (n + cluster - 1) / cluster, l0 = min(n, (int64_t)rank * per), l1 = min(n, l0 + per);
+    const int rows = (int)(l1 - l0);
+    const double2* Q = bt.Q + g.q + l0;
+    double2* Wg = bt.W + g.v + l0;
+    double2* w = w_in_smem ? sh2 + 4 * (m + 1) : Wg;
+    const uint32_t bytes = (uint32_t)(cluster * MG_WARPS * sizeof(double2));
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(mb), box = (uint32_t)__cvta_generic_to_shared(slot);
+    auto arm = [&](int p) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * p), "r"(bytes) : "memory");
+    };
+    if (tid == 0) {
+        for (int p = 0; p < 2; ++p)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * p) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        arm(0);
+        arm(1);
+    }
+    for (int i = tid; i < k; i += MG_THREADS) {
+        t.cs[i] = sm.cs[i];
+        t.sn[i] = sm.sn[i];
+    }
     if (w_in_smem)
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) w[i] = Wg[i];
-    __syncthreads();
-    // modified Gram-Schmidt
-    for (int i = 0; i <= k; ++i) {
-        const double2* qi = Q + (size_t)i * n;
-        double2 acc = make_double2(0, 0);
-        for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-            double2 a = w[l], q = qi[l];
-            if (bt.ref_dotc) cfma(acc, cconj(a), q);  // nalgebra dotc(qk1, q_i) = sum conj(qk1) q_i
-            else cfma(acc, cconj(q), a);             // q_i^H w
-        }
-        double2 h = block_sum2(acc, sh);
-        for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-            double2 a = w[l];
-            cfma(a, cneg(h), qi[l]);
-            w[l] = a;
-        }
-        if (threadIdx.x == 0) sm.hk1[i] = h;
-        __syncthreads();
-    }
-    const double hn = vec_norm(w, n, sh);
-    // scale = 1 / hk1[k+1] as a complex division (gmres.rs:172)
-    double2 scale = cdiv(make_double2(1.0, 0.0), make_double2(hn, 0.0));
-    for (int64_t l = threadIdx.x; l < n; l += blockDim.x) qk1[l] = cmul(w[l], scale);
-    if (threadIdx.x == 0) {
-        sm.hk1[k + 1] = make_double2(hn, 0.0);
-        // apply previous rotations
-        for (int i = 0; i < k; ++i) {
-            double2 t = cadd(cmul(sm.cs[i], sm.hk1[i]), cmul(sm.sn[i], sm.hk1[i + 1]));
-            sm.hk1[i + 1] = cadd(cmul(cneg(cconj(sm.sn[i])), sm.hk1[i]), cmul(sm.cs[i], sm.hk1[i + 1]));
-            sm.hk1[i] = t;
-        }
-        // new rotation (LAWN 148)
-        double2 v1 = sm.hk1[k], v2 = sm.hk1[k + 1];
-        double a1 = cabs_(v1);
-        double2 signf = (v1.x == 0.0 && v1.y == 0.0) ? make_double2(1.0, 0.0) : make_double2(v1.x / a1, v1.y / a1);
-        double r = sqrt(cnorm2(v1) + cnorm2(v2));
-        double2 cs = make_double2(a1 / r, 0.0);
-        double2 sn = cmul(signf, cconj(v2));
-        sn = make_double2(sn.x / r, sn.y / r);
-        sm.cs[k] = cs;
-        sm.sn[k] = sn;
-        sm.hk1[k] = cadd(cmul(cs, sm.hk1[k]), cmul(sn, sm.hk1[k + 1]));
-        sm.hk1[k + 1] = make_double2(0, 0);
-        for (int i = 0; i < k + 2; ++i) sm.H[(size_t)k * (m + 1) + i] = sm.hk1[i];
-        sm.beta[k + 1] = cmul(cneg(cconj(sn)), sm.beta[k]);
-        sm.beta[k] = cmul(sm.beta[k], cs);
-        st.error = cabs_(sm.beta[k + 1]) / (st.anorm * st.xnorm + st.bnorm);
-        st.num_mv += 1;
-        st.iterations += 1;
-        int chk = (st.error < st.tol) || (k == st.m - 1);
-        st.check = chk;
-        if (chk) {
-            // y = H_k^{-1} beta_k: H_k is upper triangular after the rotations
-            for (int i = k; i >= 0; --i) {
-                double2 v = sm.beta[i];
-                for (int q = i + 1; q <= k; ++q) v = csub(v, cmul(sm.H[(size_t)q * (m + 1) + i], sm.y[q]));
-                sm.y[i] = cdiv(v, sm.H[(size_t)i * (m + 1) + i]);
+        for (int l = tid; l < rows; l += MG_THREADS) w[l] = Wg[l];
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // (a thread's rows are its own from here on)
+    bool ok = true;
+    // this warp's part of step e's sum, to every CTA
+    auto send = [&](int e, double2 acc) {
+        const bool odd = lane & 1;
+        double v = odd ? acc.y : acc.x;
+        v += __shfl_xor_sync(0xffffffffu, odd ? acc.x : acc.y, 1);
+        for (int o = 2; o < 32; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+        acc = make_double2(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
+        const int p = e & 1;
+        if (lane < cluster)
+            st_async16(peer_addr(box + (uint32_t)sizeof(double2) * (p * MAX_CLUSTER * MG_WARPS + rank * MG_WARPS + warp),
+                                 lane),
+                       peer_addr(bar + 8 * p, lane), as_uint4(acc));
+    };
+    // the sum of step e, the same in every thread
+    auto collect = [&](int e) {
+        const int p = e & 1;
+        ok = ok && peers_arrived(&mb[p], (uint32_t)(e >> 1) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        const double* f = reinterpret_cast<const double*>(slot[p]);
+        double v = 0;
+        for (int q = lane; q < 2 * MG_WARPS * cluster; q += 32) v += f[q];
+        for (int o = 2; o < 32; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const double2 h = make_double2(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
+        // for step e + 2, whose parts come after everyone has step e + 1's
+        if (tid == 0) arm(p);
+        return h;
+    };
+    double2 acc = make_double2(0, 0);
+    for (int l = tid; l < rows; l += MG_THREADS) cfma(acc, cconj(w[l]), Q[l]);
+    for (int i = 0; i <= k && ok; ++i) {
+        send(i, acc);
+        const double2 *qi = Q + (size_t)i * n, *qn = Q + (size_t)(i + 1) * n;
+        const bool more = i < k;
+        double2 a[MG_UNROLL], b[MG_UNROLL];
+        auto load = [&](int base) {
+#pragma unroll
+            for (int u = 0; u < MG_UNROLL; ++u) {
+                const int l = base + u * MG_THREADS;
+                a[u] = l < rows ? qi[l] : make_double2(0, 0);
+                b[u] = l < rows && more ? qn[l] : make_double2(0, 0);
             }
-        } else {
-            st.k = k + 1;
+        };
+        load(tid);
+        const double2 h = collect(i);
+        if (tid == 0) t.h[i] = h;
+        acc = make_double2(0, 0);
+        for (int base = tid; base < rows; base += MG_UNROLL * MG_THREADS) {
+            double2 qa[MG_UNROLL], qb[MG_UNROLL];
+#pragma unroll
+            for (int u = 0; u < MG_UNROLL; ++u) {
+                qa[u] = a[u];
+                qb[u] = b[u];
+            }
+            load(base + MG_UNROLL * MG_THREADS);
+#pragma unroll
+            for (int u = 0; u < MG_UNROLL; ++u) {
+                const int l = base + u * MG_THREADS;
+                if (l < rows) {
+                    double2 v = w[l];
+                    cfma(v, cneg(h), qa[u]);
+                    w[l] = v;
+                    if (more) cfma(acc, cconj(v), qb[u]);
+                    else acc.x = fma(v.x, v.x, fma(v.y, v.y, acc.x));
+                }
+            }
         }
-        hsh.x = chk;
     }
-    __syncthreads();
-    if (hsh.x != 0.0) {
-        // x += Q_k y, or Z_k y with flexible right preconditioning
-        double2* x = bt.X + g.v;
-        const double2* Zs = bt.Z ? bt.Z + g.q : Q;
-        for (int64_t l = threadIdx.x; l < n; l += blockDim.x) {
-            double2 a = x[l];
-            for (int j = 0; j <= k; ++j) cfma(a, Zs[(size_t)j * n + l], sm.y[j]);
-            x[l] = a;
-        }
+    double nn = 0;
+    if (ok) {
+        send(k + 1, acc);
+        nn = collect(k + 1).x;
     }
+    ok = __syncthreads_and(ok);
+    if (ok) {
+        if (tid < 32) gm_rotate(t, st, sm, nn);
+        __syncthreads();
+        if (*t.chk) gm_solve_y(t, sm, k, m);
+        const double sc = *t.scale;
+        double2* qk1 = bt.Q + g.q + (size_t)(k + 1) * n + l0;
+        for (int l = tid; l < rows; l += MG_THREADS) qk1[l] = make_double2(w[l].x * sc, w[l].y * sc);
+        if (*t.chk) gm_add_correction(bt, g, t.y, k, l0, l1);
+    }
+    if (!ok && tid == 0) {  // a wait ran out: the system ends as not converged
+        st.done = 1;
+        __threadfence();
+    }
+    // nobody leaves while its shared memory may still be written, and the state
+    // changes when everyone has read it
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (ok && rank == 0) gm_record(t, st, sm, m);
 }
 
 // True residual check (gmres.rs:122-138), and the start of the next cycle
@@ -1038,16 +1115,16 @@ __global__ void finish_norms_kernel(const double* part, int nb, int nsys, double
 }
 
 // ---------------------------------------------------------------------------
-// The Arnoldi kernel keeps w in dynamic shared memory when it fits
-// (n * 16 B <= AR_SMEM_CAP).  The kernel attribute is process-wide, so it is
-// raised once per device to the cap and never lowered: a smaller solve on
-// another thread cannot shrink the limit under a larger one's launch or graph.
+// Kernel attributes are process-wide, so the limits of dynamic shared memory are
+// raised once per device to their caps and never lowered: a smaller solve on
+// another thread cannot shrink one under a larger one's launch or graph.
 namespace {
 constexpr int AR_MAX_DEVICES = 64;
 std::once_flag g_ar_smem_once[AR_MAX_DEVICES];
 }  // namespace
 
-void arnoldi_allow_smem(int device) {
+static void gm_kernel_attributes(Context& ctx) {
+    const int device = ctx.device;
     require(device >= 0 && device < AR_MAX_DEVICES, "device index out of range");
     // a failed set throws out of call_once, which leaves the flag unset so the
     // next call tries again
@@ -1058,10 +1135,12 @@ void arnoldi_allow_smem(int device) {
                 throw Error(BEM_ERR_CUDA, std::string("cudaFuncSetAttribute(") + name + "): " + cudaGetErrorString(err));
         };
         allow((const void*)gm_arnoldi_kernel, AR_SMEM_CAP, "gm_arnoldi_kernel");
+        BEM_CUDA(cudaFuncSetAttribute(gm_arnoldi_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         allow((const void*)gm_givens_kernel, AR_SMEM_CAP, "gm_givens_kernel");
         allow((const void*)gm_gs_update_kernel, AR_SMEM_CAP, "gm_gs_update_kernel");
         allow((const void*)gm_apply_small_kernel<float2, 0, 4>, small_smem<float2, 0, 4>(), "gm_apply_small_kernel");
     });
+    if (!ctx.gm_cluster) ctx.gm_cluster = max_cluster((const void*)gm_arnoldi_kernel, MG_THREADS, AR_SMEM_CAP);
 }
 
 // Rows per Gram-Schmidt chunk: halved from 512 until the chunks cover the SMs.
@@ -1106,7 +1185,6 @@ void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const
     size_t oP = carve(sizeof(double2) * nsys * cb * bt.n_pad), oT = carve(sizeof(int) * nsys * rb * TICKETS);
     size_t oS = carve(sizeof(double2) * nsys * small), oSt = carve(sizeof(GmState) * nsys);
     size_t oN = carve(sizeof(double) * nsys * 1024 + sizeof(double) * nsys);
-    ws.w_in_smem = (n * sizeof(double2) <= AR_SMEM_CAP);
     // partial sums of the whole-GPU Gram-Schmidt (forms other than the reference's)
     bt.gs_rows = gs_rows_for(ws, nsys, n);
     const int gsc = ref_dotc ? 0 : (int)((n + bt.gs_rows - 1) / bt.gs_rows);
@@ -1129,7 +1207,7 @@ void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const
     ws.norm_part = reinterpret_cast<double*>(base + oN);
     ws.anorm = ws.norm_part + (size_t)nsys * 1024;
     BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * nsys * rb * TICKETS, ctx.stream));
-    arnoldi_allow_smem(ctx.device);
+    gm_kernel_attributes(ctx);
     if (ws.graph_exec) {
         cudaGraphExecDestroy(ws.graph_exec);
         ws.graph_exec = nullptr;
@@ -1191,8 +1269,7 @@ size_t gm_prepare_external(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, i
     // the last-CTA tickets must start at zero; every other region is written
     // before it is read
     BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * nsys * rb, ctx.stream));
-    ws.w_in_smem = (n * sizeof(double2) <= AR_SMEM_CAP);
-    if (ws.w_in_smem) arnoldi_allow_smem(ctx.device);
+    gm_kernel_attributes(ctx);
     return bytes;
 }
 
@@ -1255,7 +1332,6 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     size_t oS = carve(sizeof(double2) * nsys * small), oSt = carve(sizeof(GmState) * nsys);
     size_t oN = carve(sizeof(double) * nsys * 1024 + sizeof(double) * nsys);
     size_t oD = carve(sizeof(GmSys) * nsys);
-    ws.w_in_smem = (nmax * sizeof(double2) <= AR_SMEM_CAP);
     // partial sums of the whole-GPU Gram-Schmidt
     bt.gs_rows = gs_rows_for(ws, nsys, nmax);
     const int gsc = (int)((nmax + bt.gs_rows - 1) / bt.gs_rows);
@@ -1281,7 +1357,7 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
     BEM_CUDA(cudaMemcpyAsync(dsys, sys.data(), sizeof(GmSys) * nsys, cudaMemcpyHostToDevice, ctx.stream));
     bt.sys = dsys;
     BEM_CUDA(cudaMemsetAsync(bt.tickets, 0, sizeof(int) * t, ctx.stream));
-    arnoldi_allow_smem(ctx.device);
+    gm_kernel_attributes(ctx);
     if (ws.graph_exec) {
         cudaGraphExecDestroy(ws.graph_exec);
         ws.graph_exec = nullptr;
@@ -1426,11 +1502,16 @@ void gm_launch_iteration(Context& ctx, GmWorkspace& ws, cudaEvent_t ev_q0, cudaE
         }
         const int chunks = (int)std::max<int64_t>(
             1, std::min<int64_t>((ws.bt.n + GV_STEP_THREADS - 1) / GV_STEP_THREADS, 2 * ws.sms / nsys));
-        gm_givens_kernel<<<dim3((unsigned)chunks, (unsigned)nsys), GV_STEP_THREADS, givens_smem(ws.bt.m),
+        gm_givens_kernel<<<dim3((unsigned)chunks, (unsigned)nsys), GV_STEP_THREADS, gm_step_smem(ws.bt.m),
                            ctx.stream>>>(ws.bt, chunks);
     } else {
-        const size_t dyn = ws.w_in_smem ? (size_t)ws.bt.n * sizeof(double2) : 0;
-        gm_arnoldi_kernel<<<nsys, AR_THREADS, dyn, ctx.stream>>>(ws.bt, ws.w_in_smem ? 1 : 0);
+        // 128 rows per CTA while the cluster reaches
+        int cs = 1;
+        while (cs < ctx.gm_cluster && (int64_t)cs * MG_THREADS < ws.bt.n) cs *= 2;
+        const size_t step = gm_step_smem(ws.bt.m), slice = sizeof(double2) * (size_t)((ws.bt.n + cs - 1) / cs);
+        const bool in_smem = step + slice <= AR_SMEM_CAP;
+        launch_cluster(ctx, gm_arnoldi_kernel, nsys * cs, cs, MG_THREADS, step + (in_smem ? slice : 0), ws.bt,
+                       in_smem ? 1 : 0, cs);
     }
     BEM_CHECK_LAUNCH(&ctx);
     launch_apply(ctx, ws, MV_CHECK);

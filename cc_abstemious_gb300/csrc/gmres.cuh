@@ -137,7 +137,6 @@ struct GmWorkspace {
     DevBuf init_args;
     std::vector<GmSys> sys_host;  // ragged layout (empty: uniform)
     bool fp32 = false;
-    bool w_in_smem = false;
     int rb = 0, cb = 0;
     int sms = 0;  // SMs of the device
     double* norm_part = nullptr;

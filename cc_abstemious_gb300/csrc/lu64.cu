@@ -46,6 +46,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "complex.cuh"
 #include "umma.cuh"
@@ -161,7 +162,6 @@ __device__ __forceinline__ int exp_above(double v) {
 // waits for every outstanding store, 1100 clocks.)
 constexpr int PANEL_WORKERS = 256, PANEL_THREADS = PANEL_WORKERS + 32, PANEL_WARPS = PANEL_WORKERS / 32;
 constexpr size_t PANEL_SMEM = 200 * 1024;  // beside 20 KB of static shared memory
-constexpr int MAX_CLUSTER = 16;
 constexpr unsigned NO_ROW = 0x7fffffffu;
 
 struct Cand {
@@ -209,35 +209,9 @@ __device__ __forceinline__ double2 recip(double2 d) {
     return make_double2(d.x * r, -d.y * r);
 }
 
-// 16 bytes into another CTA's shared memory, counted on a barrier there.
-__device__ __forceinline__ uint32_t peer_addr(uint32_t saddr, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_async16(uint32_t dst, uint32_t bar, uint4 v) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                     dst),
-                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ uint4 as_uint4(double2 v) {
-    return make_uint4((unsigned)__double2loint(v.x), (unsigned)__double2hiint(v.x), (unsigned)__double2loint(v.y),
-                      (unsigned)__double2hiint(v.y));
-}
 // Bounded wait for data written by other CTAs of the cluster.
 __device__ __forceinline__ void wait_peers(uint64_t* bar, uint32_t phase, int* err) {
-    for (uint32_t it = 0; it < (1u << 22); ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(phase)
-            : "memory");
-        if (ok) return;
-    }
-    atomicOr(err, DEVERR_MBAR_TIMEOUT);
+    if (!peers_arrived(bar, phase)) atomicOr(err, DEVERR_MBAR_TIMEOUT);
 }
 
 __global__ void __launch_bounds__(PANEL_THREADS, 1)
@@ -1129,41 +1103,6 @@ __global__ void __launch_bounds__(SOLVE_THREADS) lu64_solve_kernel(int64_t n, co
 }
 
 // ---------------------------------------------------------------------------
-// The largest cluster the device schedules with the panel's shared memory.
-int max_cluster(const void* kernel, int threads, size_t smem) {
-    for (int cs = MAX_CLUSTER; cs > 1; cs /= 2) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)cs);
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim = {(unsigned)cs, 1, 1};
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int num = 0;
-        if (cudaOccupancyMaxActiveClusters(&num, kernel, &cfg) == cudaSuccess && num >= 1) return cs;
-        cudaGetLastError();
-    }
-    return 1;
-}
-
-template <class... K, class... Args>
-void launch_cluster(Context& ctx, void (*kernel)(K...), int cs, int threads, size_t smem, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)cs);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim = {(unsigned)cs, 1, 1};
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    BEM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-    BEM_CHECK_LAUNCH(&ctx);
-}
-
 }  // namespace
 
 // What a factorization leaves beside the factors: the row order and the
@@ -1215,7 +1154,7 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
         require((size_t)rows_of(R) * w * sizeof(double2) <= PANEL_SMEM, "LU: matrix too large", BEM_ERR_OOM);
         for (int64_t c0 = b0; c0 < b0 + nb; c0 += w) {
             const int pw = (int)std::min<int64_t>(w, b0 + nb - c0), rpc = (int)rows_of(n - c0);
-            launch_cluster(ctx, lu64_panel_kernel, cs, PANEL_THREADS, sizeof(double2) * (size_t)rpc * pw, n, A, lda, c0,
+            launch_cluster(ctx, lu64_panel_kernel, cs, cs, PANEL_THREADS, sizeof(double2) * (size_t)rpc * pw, n, A, lda, c0,
                            pw, b0, nb, rpc, mv, cexp + b0, pinv, d_info, err);
             const int nc = (int)(b0 + nb - c0 - pw);
             if (nc > 0) {

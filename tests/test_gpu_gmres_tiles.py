@@ -1,6 +1,7 @@
 """GMRES (csrc/gmres.cu, csrc/precond.cu) at the sizes where its tiles end: row
 blocks of 64 and 512, column chunks of 512, Gram-Schmidt chunks of 64 to 512 rows,
-preconditioner blocks of up to 64 in halves of 32.
+preconditioner blocks of up to 64 in halves of 32, Arnoldi clusters of up to 16
+CTAs with 128 rows each.
 
 FP64: the stopping test gives ||r|| <= tol (||A||_F ||x|| + ||b||), so the error
 against a direct solution is at most tol ||A^-1|| (||A||_F + ||A||) ||x||; with the
@@ -16,7 +17,7 @@ bem = pytest.importorskip("cc_abstemious_gb300")
 from cc_abstemious_gb300 import workloads  # noqa: E402
 
 
-@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 129, 511, 512, 513, 577, 700])
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 129, 511, 512, 513, 577, 700, 1023, 1025, 2047, 2049, 2600])
 def test_fp64_sizes(n):
     rng = np.random.default_rng(n)
     A = 0.25 * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))) / np.sqrt(n) + 2 * np.eye(n)
@@ -30,7 +31,7 @@ def test_fp64_sizes(n):
     assert rep["flag"] == 1 or n <= 2
     if n <= 2:
         return
-    assert np.linalg.norm(x - ref) <= 1e-11 * np.linalg.norm(ref)
+    assert np.linalg.norm(x - ref) <= 2e-11 * np.linalg.norm(ref)
 
 
 @pytest.mark.parametrize("form", ["mixed", "refined"])
