@@ -47,6 +47,7 @@ struct HMatrixDev {
     std::vector<HLeaf> leaves;
     std::vector<int64_t> rows, cols;
     DevBuf d_leaves, d_rows, d_cols, d_store, d_scratch, d_y, d_rowptr, d_rowent, d_vec;
+    DevBuf d_order;  // leaves by the work of their product, largest first
     int64_t nadm = 0, ninadm = 0, stored = 0, rank_sum = 0;
 };
 
@@ -732,67 +733,158 @@ __global__ void hm_dense_norm_kernel(HLeaf* __restrict__ leaves, const int32_t* 
 // ---------------------------------------------------------------------------
 // Mat-vec: every leaf multiplies its gathered slice of x (alpha applied), the
 // row reduction adds the slices of each global row in leaf order.
-__global__ void __launch_bounds__(LEAF_THREADS) hm_leaf_mv_kernel(const HLeaf* __restrict__ leaves,
-                                                                  const int64_t* __restrict__ rows,
-                                                                  const int64_t* __restrict__ cols,
-                                                                  const double2* __restrict__ store, GmBatch bt,
-                                                                  int mode, const double2* __restrict__ xin,
-                                                                  z2 alpha, double2* __restrict__ y) {
-    __shared__ double sh[48];
-    __shared__ double2 tks[64];
+//
+// FP64 instructions bound it (65 clocks per warp and SM quarter), so the four
+// warps of a leaf's CTA, one per quarter, get equal shares: of the column range
+// in V^T x (eight lanes per rank, so that a sum costs four additions for four
+// ranks), of the rows or, in a leaf of few rows, of the columns in U t and D x.
+// The leaves are taken heaviest first.  (A block-wide reduction per rank and
+// threads without a row: 735 us at n = 10240 with 27 M stored entries, whose
+// products alone take 173 us; now 276 us.)
+constexpr int HMV_THREADS = 128, HMV_WARPS = HMV_THREADS / 32, HMV_CHUNK = 512;
+
+// Sum over eight lanes, the parts in the first two of them.
+__device__ __forceinline__ double sum8_parts(double2 v) {
+    const bool odd = threadIdx.x & 1;
+    double s = odd ? v.y : v.x;
+    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    return s;
+}
+
+// out[i] (+)= sum over k < nc of M[k m + i] c[k], M column-major in device
+// memory, c and `part` (HMV_THREADS entries) in shared memory; the whole CTA.
+__device__ __forceinline__ void leaf_columns(const double2* __restrict__ M, int64_t m, int nc, const double2* c,
+                                             double2* part, bool add, z2 alpha, double2* __restrict__ out) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int groups = m <= 32 ? HMV_WARPS : m <= 64 ? HMV_WARPS / 2 : 1;  // warps sharing a row
+    const int tiles = HMV_WARPS / groups, kg = warp / tiles;
+    const int per = (nc + groups - 1) / groups, ka = min(nc, kg * per), kb = min(nc, ka + per);
+    for (int64_t i0 = 0; i0 < m; i0 += 32 * tiles) {
+        const int64_t i = i0 + 32 * (warp % tiles) + lane;
+        z2 acc = make_double2(0, 0);
+        if (i < m) {
+            const double2* col = M + i;
+            int k = ka;
+            for (; k + 8 <= kb; k += 8) {
+                double2 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = __ldcs(col + (size_t)(k + u) * m);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) cfma(acc, v[u], c[k + u]);
+            }
+            for (; k < kb; ++k) cfma(acc, __ldcs(col + (size_t)k * m), c[k]);
+        }
+        if (groups > 1) {
+            part[threadIdx.x] = acc;
+            __syncthreads();
+            if (kg == 0)
+                for (int q = 1; q < groups; ++q) acc = cadd(acc, part[threadIdx.x + 32 * tiles * q]);
+        }
+        if (i < m && kg == 0) {
+            acc = cmul(alpha, acc);
+            out[i] = add ? cadd(out[i], acc) : acc;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(HMV_THREADS) hm_leaf_mv_kernel(const HLeaf* __restrict__ leaves,
+                                                                 const int32_t* __restrict__ order,
+                                                                 const int64_t* __restrict__ cols,
+                                                                 const double2* __restrict__ store, GmBatch bt,
+                                                                 int mode, const double2* __restrict__ xin, z2 alpha,
+                                                                 double2* __restrict__ y) {
+    __shared__ double2 xs[HMV_CHUNK], part[HMV_THREADS];
+    __shared__ double2 tw[HMV_WARPS][64], tk[64];
     const double2* x = xin;
     if (bt.st) {
         const GmState& st = bt.st[0];
         if (!gm_apply_active(bt, st, mode)) return;
         x = (mode == MV_Q) ? bt.Q + (size_t)st.k * bt.n : bt.X;
     }
-    const HLeaf L = leaves[blockIdx.x];
+    const HLeaf L = leaves[order[blockIdx.x]];
     const double2* D = store + L.store_off;
     double2* yo = y + L.y_off;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const z2 one = make_double2(1, 0);
     if (!L.adm) {
-        for (int64_t i = threadIdx.x; i < L.m; i += blockDim.x) {
-            z2 acc = make_double2(0, 0);
-            for (int64_t j = 0; j < L.n; ++j) cfma(acc, D[(size_t)j * L.m + i], x[cols[L.col_off + j]]);
-            yo[i] = cmul(alpha, acc);
+        for (int64_t j0 = 0; j0 < L.n; j0 += HMV_CHUNK) {
+            const int jn = (int)min((int64_t)HMV_CHUNK, L.n - j0);
+            if (j0) __syncthreads();
+            for (int j = tid; j < jn; j += HMV_THREADS) xs[j] = x[cols[L.col_off + j0 + j]];
+            __syncthreads();
+            leaf_columns(D + (size_t)j0 * L.m, L.m, jn, xs, part, j0 > 0, alpha, yo);
         }
         return;
     }
     const double2* U = D;
     const double2* V = U + (size_t)L.m * L.kmax;
-    for (int i = threadIdx.x; i < L.m; i += blockDim.x) yo[i] = make_double2(0, 0);
+    if (L.rank == 0)
+        for (int64_t i = tid; i < L.m; i += HMV_THREADS) yo[i] = make_double2(0, 0);
+    const int l8 = lane & 7;
     for (int k0 = 0; k0 < L.rank; k0 += 64) {
         const int kc = min(64, L.rank - k0);
-        for (int k = 0; k < kc; ++k) {
-            const double2* vk = V + (size_t)(k0 + k) * L.n;
-            z2 acc = make_double2(0, 0);
-            for (int64_t j = threadIdx.x; j < L.n; j += blockDim.x) cfma(acc, vk[j], x[cols[L.col_off + j]]);
-            acc = bsum2(acc, sh);
-            if (threadIdx.x == 0) tks[k] = cmul(alpha, acc);  // alpha * (v_k . x), aca.rs:187-193
+        for (int k = tid; k < HMV_WARPS * 64; k += HMV_THREADS) (&tw[0][0])[k] = make_double2(0, 0);
+        for (int64_t j0 = 0; j0 < L.n; j0 += HMV_CHUNK) {
+            const int jn = (int)min((int64_t)HMV_CHUNK, L.n - j0);
+            __syncthreads();
+            for (int j = tid; j < jn; j += HMV_THREADS) xs[j] = x[cols[L.col_off + j0 + j]];
+            __syncthreads();
+            // this warp's columns, a multiple of eight
+            const int per = ((jn + 8 * HMV_WARPS - 1) / (8 * HMV_WARPS)) * 8;
+            const int ja = min(jn, warp * per), jb = min(jn, ja + per);
+            for (int k = 0; k < kc; k += 4) {
+                const int kk = k + (lane >> 3);
+                const double2* vk = V + (size_t)(k0 + min(kk, kc - 1)) * L.n + j0;
+                z2 acc = make_double2(0, 0);
+                int j = ja + l8;
+                for (; j + 24 < jb; j += 32) {
+                    double2 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = __ldcs(vk + j + 8 * u);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) cfma(acc, v[u], xs[j + 8 * u]);
+                }
+                for (; j < jb; j += 8) cfma(acc, __ldcs(vk + j), xs[j]);
+                const double sum = sum8_parts(acc);
+                if (l8 < 2 && kk < kc) reinterpret_cast<double*>(&tw[warp][kk])[l8] += sum;
+            }
         }
         __syncthreads();
-        for (int64_t i = threadIdx.x; i < L.m; i += blockDim.x) {
-            z2 a = yo[i];
-            for (int k = 0; k < kc; ++k) cfma(a, U[(size_t)(k0 + k) * L.m + i], tks[k]);
-            yo[i] = a;
-        }
+        for (int k = tid; k < kc; k += HMV_THREADS)  // alpha * (v_k . x), aca.rs:187-193
+            tk[k] = cmul(alpha, cadd(cadd(tw[0][k], tw[1][k]), cadd(tw[2][k], tw[3][k])));
+        __syncthreads();
+        leaf_columns(U + (size_t)k0 * L.m, L.m, kc, tk, part, k0 > 0, one, yo);
         __syncthreads();
     }
 }
 
-// out[i] = beta * out[i] + sum over the leaves covering row i (fixed order).
-__global__ void hm_row_reduce_kernel(int64_t n, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ ent,
-                                     const double2* __restrict__ y, GmBatch bt, int mode, z2 beta,
-                                     double2* __restrict__ out) {
+// out[i] = beta * out[i] + sum over the leaves covering row i (fixed order): a
+// row's entries are gathered from all over y, so eight lanes share them (one
+// thread per row waits for one after another: 43 us at n = 10240, now 10).
+constexpr int ROW_LANES = 8, ROW_THREADS = 128;
+__global__ void __launch_bounds__(ROW_THREADS) hm_row_reduce_kernel(int64_t n, const int64_t* __restrict__ rowptr,
+                                                                    const int64_t* __restrict__ ent,
+                                                                    const double2* __restrict__ y, GmBatch bt,
+                                                                    int mode, z2 beta, double2* __restrict__ out) {
     if (bt.st) {
         const GmState& st = bt.st[0];
         if (!gm_apply_active(bt, st, mode)) return;
     }
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    z2 acc = (beta.x == 0.0 && beta.y == 0.0) ? make_double2(0, 0) : cmul(beta, out[i]);
-    for (int64_t t = rowptr[i]; t < rowptr[i + 1]; ++t) acc = cadd(acc, y[ent[t]]);
-    out[i] = acc;
+    const int64_t i = (blockIdx.x * (int64_t)ROW_THREADS + threadIdx.x) / ROW_LANES;
+    const int l8 = threadIdx.x & (ROW_LANES - 1);
+    z2 acc = make_double2(0, 0), b = acc;
+    if (i < n) {
+        if (beta.x != 0.0 || beta.y != 0.0) b = cmul(beta, out[i]);
+        for (int64_t t = rowptr[i] + l8; t < rowptr[i + 1]; t += ROW_LANES) acc = cadd(acc, y[ent[t]]);
+    }
+    const double s = sum8_parts(acc);  // (every lane has read out[i])
+    __syncwarp();
+    if (i < n && l8 < 2) reinterpret_cast<double*>(out + i)[l8] = (l8 ? b.y : b.x) + s;
 }
+
+static unsigned row_grid(int64_t n) { return (unsigned)((n * ROW_LANES + ROW_THREADS - 1) / ROW_THREADS); }
 
 // ---------------------------------------------------------------------------
 static GenParams gen_params(const Problem& p, int side) {
@@ -822,6 +914,16 @@ static std::shared_ptr<HTrees> build_trees(Context& c, const Problem& p) {
     T->F = build_forest(c, std::vector<const Problem*>{&p}, p.in.hm_leaf);
     T->bl = forest_block_leaves(c, *T->F, p.in.hm_eta);
     return T;
+}
+
+template <class Work>
+static std::vector<int32_t> heaviest_first(size_t count, Work work) {
+    std::vector<std::pair<int64_t, int32_t>> key(count);
+    for (size_t b = 0; b < count; ++b) key[b] = {-(int64_t)work(b), (int32_t)b};
+    std::sort(key.begin(), key.end());
+    std::vector<int32_t> order(count);
+    for (size_t b = 0; b < count; ++b) order[b] = key[b].second;
+    return order;
 }
 
 // trees: the problem's trees from an earlier build (several frequencies of
@@ -874,8 +976,13 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
                              c.stream));
     BEM_CUDA(cudaMemcpyAsync(H->d_cols.p, F.d_perm.p, sizeof(int64_t) * H->cols.size(), cudaMemcpyDeviceToDevice,
                              c.stream));
+    // the compressed leaves by size, then by the work their rank makes: a large
+    // one begun last would run alone
     std::vector<int32_t> adm_list, dense_list;
-    for (size_t b = 0; b < nl; ++b) (H->leaves[b].adm ? adm_list : dense_list).push_back((int32_t)b);
+    for (int32_t b : heaviest_first(nl, [&](size_t b) { return H->leaves[b].m + H->leaves[b].n; }))
+        if (H->leaves[(size_t)b].adm) adm_list.push_back(b);
+    for (size_t b = 0; b < nl; ++b)
+        if (!H->leaves[b].adm) dense_list.push_back((int32_t)b);
     DevBuf d_adm, d_dense;
     d_adm.ensure(sizeof(int32_t) * std::max<size_t>(adm_list.size(), 1));
     d_dense.ensure(sizeof(int32_t) * std::max<size_t>(dense_list.size(), 1));
@@ -906,6 +1013,15 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
         c.sync();
         require(herr == 0, "ACA rank exceeded the storage cap of " + std::to_string(ACA_RMAX),
                 BEM_ERR_NOT_CONVERGED);
+        std::stable_sort(adm_list.begin(), adm_list.end(), [&](int32_t a, int32_t b) {
+            auto work = [&](int32_t l) {
+                const HLeaf& L = H->leaves[(size_t)l];
+                return (int64_t)L.rank * L.rank * (L.m + L.n + 8 * L.rank);
+            };
+            return work(a) > work(b);
+        });
+        BEM_CUDA(cudaMemcpyAsync(d_adm.p, adm_list.data(), sizeof(int32_t) * adm_list.size(), cudaMemcpyHostToDevice,
+                                 c.stream));
         // recompression scratch sized by the ranks just found
         std::vector<int64_t> off(adm_list.size());
         int64_t tot = 0;
@@ -944,6 +1060,12 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
             H->stored += L.m * L.n;
         }
     }
+    const std::vector<int32_t> order = heaviest_first(nl, [&](size_t b) {
+        const HLeaf& L = H->leaves[b];
+        return L.adm ? L.rank * (L.m + L.n) : L.m * L.n;
+    });
+    H->d_order.ensure(sizeof(int32_t) * std::max<size_t>(nl, 1));
+    BEM_CUDA(cudaMemcpyAsync(H->d_order.p, order.data(), sizeof(int32_t) * nl, cudaMemcpyHostToDevice, c.stream));
     // row CSR over the leaves' output slices (leaf order)
     std::vector<int64_t> cnt((size_t)n + 1, 0);
     for (auto& L : H->leaves)
@@ -1016,12 +1138,12 @@ void hmatrix_row_sums(Context& c, const Problem& p, int side, double2* out) {
 void hmatrix_gemv(Context& c, const HMatrixDev& H, cd alpha, const double2* x, cd beta, double2* b) {
     GmBatch none{};
     if (!H.leaves.empty()) {
-        hm_leaf_mv_kernel<<<(unsigned)H.leaves.size(), LEAF_THREADS, 0, c.stream>>>(
-            H.d_leaves.as<HLeaf>(), H.d_rows.as<int64_t>(), H.d_cols.as<int64_t>(), H.d_store.as<double2>(), none, 0,
+        hm_leaf_mv_kernel<<<(unsigned)H.leaves.size(), HMV_THREADS, 0, c.stream>>>(
+            H.d_leaves.as<HLeaf>(), H.d_order.as<int32_t>(), H.d_cols.as<int64_t>(), H.d_store.as<double2>(), none, 0,
             x, make_double2(alpha.re, alpha.im), const_cast<double2*>(H.d_y.as<double2>()));
         BEM_CHECK_LAUNCH(&c);
     }
-    hm_row_reduce_kernel<<<(unsigned)((H.n + 255) / 256), 256, 0, c.stream>>>(
+    hm_row_reduce_kernel<<<row_grid(H.n), ROW_THREADS, 0, c.stream>>>(
         H.n, H.d_rowptr.as<int64_t>(), H.d_rowent.as<int64_t>(), H.d_y.as<double2>(), none, 0,
         make_double2(beta.re, beta.im), b);
     BEM_CHECK_LAUNCH(&c);
@@ -1030,11 +1152,11 @@ void hmatrix_gemv(Context& c, const HMatrixDev& H, cd alpha, const double2* x, c
 // GMRES operator hook: W = H v, predicated on the (single) system's state.
 static void hm_apply_hook(Context& c, GmWorkspace& ws, int mode, void* user) {
     const HMatrixDev& H = *static_cast<const HMatrixDev*>(user);
-    hm_leaf_mv_kernel<<<(unsigned)H.leaves.size(), LEAF_THREADS, 0, c.stream>>>(
-        H.d_leaves.as<HLeaf>(), H.d_rows.as<int64_t>(), H.d_cols.as<int64_t>(), H.d_store.as<double2>(), ws.bt, mode,
+    hm_leaf_mv_kernel<<<(unsigned)H.leaves.size(), HMV_THREADS, 0, c.stream>>>(
+        H.d_leaves.as<HLeaf>(), H.d_order.as<int32_t>(), H.d_cols.as<int64_t>(), H.d_store.as<double2>(), ws.bt, mode,
         nullptr, make_double2(1.0, 0.0), const_cast<double2*>(H.d_y.as<double2>()));
     BEM_CHECK_LAUNCH(&c);
-    hm_row_reduce_kernel<<<(unsigned)((H.n + 255) / 256), 256, 0, c.stream>>>(
+    hm_row_reduce_kernel<<<row_grid(H.n), ROW_THREADS, 0, c.stream>>>(
         H.n, H.d_rowptr.as<int64_t>(), H.d_rowent.as<int64_t>(), H.d_y.as<double2>(), ws.bt, mode,
         make_double2(0.0, 0.0), ws.bt.W);
     BEM_CHECK_LAUNCH(&c);
