@@ -227,6 +227,10 @@ struct Context {
     DevBuf w_piv;     // the plain form's FP64 LU: row order, diagonal blocks' inverses
     DevBuf w_lu64;    // its trailing update's digit images
     int lu64_cluster = 0;  // largest cluster its panels run on (0: not asked yet)
+    // its second stream (created with the first factorization) and the events
+    // between the two
+    cudaStream_t lu64_side = nullptr;
+    cudaEvent_t lu64_ready = nullptr, lu64_done = nullptr;
     int gm_cluster = 0;    // the same for the Arnoldi step of the reference's form
     // results of the last bem_run
     std::vector<double> last_phi, last_vn;

@@ -18,11 +18,13 @@
 //          become U12 = L11^-1 A12 (FP64) and are split into digits; L21 is
 //          split by the same launch.
 //   gemm   A22 -= L21 U12 from the digits (tcgen05, FP16 operands, FP32
-//          accumulation that is exact), one FP64 subtraction per entry.
+//          accumulation that is exact), one FP64 subtraction per entry; the
+//          first tile of columns ahead of the others, which run beside the next
+//          block's panel.
 //
 // Device time of one factorization and solve, against one launch per column,
 // FP64 tiles for the trailing update and one thread per triangular block before:
-// n = 324 10.2 -> 1.35 ms, n = 2001 99 -> 10.9 ms, n = 6144 776 -> 74.5 ms.
+// n = 324 10.2 -> 1.4 ms, n = 2001 99 -> 10.4 ms, n = 6144 776 -> 57.9 ms.
 //
 // Beside the factors the row order and the inverses of the diagonal blocks are
 // kept; the substitutions run over the whole GPU (lu64_solve_kernel).
@@ -45,6 +47,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
 
 #include "cluster.cuh"
 #include "common.cuh"
@@ -762,7 +765,7 @@ __device__ __forceinline__ double sub_scaled_any(double c, int64_t T, int rexp, 
 }
 
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-    lu64_gemm_kernel(double* __restrict__ F, int64_t lda2, int m, int row_blocks, int col_tiles,
+    lu64_gemm_kernel(double* __restrict__ F, int64_t lda2, int m, int cols, int row_blocks, int col_tiles,
                      const unsigned char* __restrict__ Aimg, const unsigned char* __restrict__ Bimg,
                      const int* __restrict__ er, const int* __restrict__ ec, int* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -887,7 +890,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             const int r = rb * TM + 32 * quarter + lane, j0 = ct * TN + EPI_COLS * part;
             const bool rok = r < 2 * m;
-            const int nq = max(0, min(EPI_COLS, m - j0));
+            const int nq = max(0, min(EPI_COLS, cols - j0));
             const int rexp = rok ? er[r >> 1] : 0;  // (outside the matrix: any exponent in range)
             const int cexps = lane < nq ? ec[j0 + lane] : 0;
             double* p = F + (int64_t)j0 * lda2 + r;
@@ -1141,9 +1144,16 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
     RowMoves* mv = reinterpret_cast<RowMoves*>(reinterpret_cast<char*>(cexp) + c_bytes);
     double2* pinv = reinterpret_cast<double2*>(reinterpret_cast<char*>(mv) + v_bytes);
     BEM_CUDA(cudaMemsetAsync(cexp, 0x80, c_bytes, ctx.stream));  // below every exponent
+    if (!ctx.lu64_side) {
+        BEM_CUDA(cudaEventCreateWithFlags(&ctx.lu64_ready, cudaEventDisableTiming));
+        BEM_CUDA(cudaEventCreateWithFlags(&ctx.lu64_done, cudaEventDisableTiming));
+        BEM_CUDA(cudaStreamCreateWithFlags(&ctx.lu64_side, cudaStreamNonBlocking));
+    }
+    std::function<void()> beside;  // the part of the last update that runs beside this block's panels
     for (int64_t b0 = 0; b0 < n; b0 += NB) {
         const int nb = (int)std::min<int64_t>(NB, n - b0);
         const int64_t R = n - b0;
+        bool ahead = false;
         int cs = 1;  // CTAs of the panels' cluster: 32 rows each where the cluster reaches
         while (cs < ctx.lu64_cluster && (int64_t)cs * 32 < R) cs *= 2;
         auto rows_of = [&](int64_t rows) { return ((rows + cs - 1) / cs + 31) / 32 * 32; };
@@ -1156,6 +1166,11 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
             const int pw = (int)std::min<int64_t>(w, b0 + nb - c0), rpc = (int)rows_of(n - c0);
             launch_cluster(ctx, lu64_panel_kernel, cs, cs, PANEL_THREADS, sizeof(double2) * (size_t)rpc * pw, n, A, lda, c0,
                            pw, b0, nb, rpc, mv, cexp + b0, pinv, d_info, err);
+            if (beside) {  // (behind the panel in the order of submission)
+                beside();
+                beside = nullptr;
+                ahead = true;
+            }
             const int nc = (int)(b0 + nb - c0 - pw);
             if (nc > 0) {
                 lu64_mid_kernel<<<dim3((unsigned)((n - c0 - pw + 31) / 32), (unsigned)((nc + MID_COLS - 1) / MID_COLS)),
@@ -1163,6 +1178,7 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
                 BEM_CHECK_LAUNCH(&ctx);
             }
         }
+        if (ahead) BEM_CUDA(cudaStreamWaitEvent(ctx.stream, ctx.lu64_done, 0));
         const int64_t m = n - b0 - nb, rb = (m + 63) / 64, ct = (m + TN - 1) / TN;
         // columns per warp: a warp for every two columns while the SM quarters
         // (four per SM) outnumber the warps
@@ -1176,9 +1192,30 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
         BEM_CHECK_LAUNCH(&ctx);
         if (m <= 0) continue;
         const int64_t t0 = b0 + nb;
-        lu64_gemm_kernel<<<(unsigned)std::min<int64_t>(rb * ct, nsm), GEMM_THREADS, GEMM_SMEM, ctx.stream>>>(
-            reinterpret_cast<double*>(A + t0 * lda + t0), 2 * lda, (int)m, (int)rb, (int)ct, Aimg, Bimg, er, ec, err);
-        BEM_CHECK_LAUNCH(&ctx);
+        // column tiles first .. last of the update
+        auto update = [=, &ctx](int64_t first, int64_t last, int64_t sms, cudaStream_t stream) {
+            const int64_t cols = m - first * TN;
+            lu64_gemm_kernel<<<(unsigned)std::min<int64_t>(rb * (last - first), sms), GEMM_THREADS, GEMM_SMEM, stream>>>(
+                reinterpret_cast<double*>(A + (t0 + first * TN) * lda + t0), 2 * lda, (int)m, (int)cols, (int)rb,
+                (int)(last - first), Aimg, Bimg + first * (size_t)B_IMG, er, ec + first * TN, err);
+            BEM_CHECK_LAUNCH(&ctx);
+        };
+        if (ct < 2) {
+            update(0, ct, nsm, ctx.stream);
+            continue;
+        }
+        // The next panel needs the first tile of columns only: the others are
+        // updated beside it, on the SMs that its cluster leaves.  The panel comes
+        // first on the SMs because its stream goes straight on.  (One after the
+        // other, update and solve included: n = 1000 4.8 ms, 2001 11.3, 4000 32.7,
+        // 6144 73.7; this way 4.7, 10.4, 26.9, 57.9.)
+        update(0, 1, nsm, ctx.stream);
+        BEM_CUDA(cudaEventRecord(ctx.lu64_ready, ctx.stream));
+        BEM_CUDA(cudaStreamWaitEvent(ctx.lu64_side, ctx.lu64_ready, 0));
+        beside = [=, &ctx] {
+            update(1, ct, nsm - cs, ctx.lu64_side);
+            BEM_CUDA(cudaEventRecord(ctx.lu64_done, ctx.lu64_side));
+        };
     }
 }
 
