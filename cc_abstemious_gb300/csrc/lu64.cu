@@ -24,7 +24,7 @@
 //
 // Device time of one factorization and solve, against one launch per column,
 // FP64 tiles for the trailing update and one thread per triangular block before:
-// n = 324 10.2 -> 1.4 ms, n = 2001 99 -> 10.4 ms, n = 6144 776 -> 57.9 ms.
+// n = 324 10.2 -> 1.5 ms, n = 2001 99 -> 11.0 ms, n = 6144 776 -> 63.5 ms.
 //
 // Beside the factors the row order and the inverses of the diagonal blocks are
 // kept; the substitutions run over the whole GPU (lu64_solve_kernel).
@@ -34,11 +34,16 @@
 // in [-128, 128]; U12 likewise relative to the largest of its column.  Digit
 // products are integers <= 2^14, a sum over K = 64 (32 complex entries) of at
 // most seven of them stays below 2^23, so FP32 accumulation has no rounding at
-// all.  Of the 49 digit products the 28 of weight 256^-2 ... 256^-8 are formed,
-// in seven groups of equal weight; the groups are added in 64-bit integers and
-// rounded once to FP64.  What is left out is below 2^-54 of (largest of the
-// row) x (largest of the column): a chain of 32 FP64 multiply-adds rounds 32
-// times at 2^-53.  The columns of L21 and the rows of U12 are scaled against
+// all.  Of the 49 digit products the 34 of weight 256^-2 ... 256^-9 are formed,
+// in eight groups of equal weight; the groups are added in 64-bit integers and
+// rounded once to FP64.  What the splitting, the rounding and the products left
+// out lose is about 2^-54 of (largest of the row) x (largest of the column): a
+// chain of 32 FP64 multiply-adds rounds 64 times at 2^-54 of its partial sums.
+// (Without the group of weight 256^-9 the products left out were the largest
+// error, and x had half again to twice the error of FP64 elimination; the group
+// costs 9 % at n = 6144.  With it, geometric mean of the error of x over random
+// matrices, against FP64 tiles: n = 324 5.3e-14 / 9.4e-14, 1300 3.8e-13 / 7.0e-13,
+// 2001 1.4e-12 / 1.9e-12.)  The columns of L21 and the rows of U12 are scaled against
 // each other by the exponent of the column's largest entry, so that a matrix
 // whose rows or columns differ by orders of magnitude keeps that bound for
 // each of them.
@@ -65,6 +70,7 @@ namespace {
 
 constexpr int NB = 32;        // columns per block
 constexpr int SLICES = 7;     // digits per entry
+constexpr int GROUPS = SLICES + 1;  // groups of digit products of equal weight
 constexpr int TM = 128;       // tile rows (real): 64 complex rows
 constexpr int TN = 64;        // tile columns
 constexpr uint32_t A_SLICE = TM * 128, B_SLICE = TN * 128;  // 64 halves = 128 bytes per row
@@ -829,16 +835,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     ++nload;
                 }
                 ok = ok && mbar_wait_bounded(&bfull[st], (uint32_t)((it >> 1) & 1));
-                for (int g = SLICES; g >= 1 && ok; --g, ++idx) {
+                for (int g = GROUPS; g >= 1 && ok; --g, ++idx) {
+                    const int i0 = max(0, g - SLICES), i1 = min(g, SLICES);  // digits of A in this group
                     const int blk = idx % RING, use = idx / RING;
                     ok = use == 0 || mbar_wait_bounded(&tempty[blk], (uint32_t)((use - 1) & 1));
                     if (!ok) break;
                     tc_fence_after();
-                    for (int i = 0; i < g; ++i) {
+                    for (int i = i0; i < i1; ++i) {
                         const uint32_t as = tmem + TMEM_A + i * TMEM_A_SLICE, bd = base + st * B_IMG + (g - 1 - i) * B_SLICE;
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
-                            mma_f16(tmem + (uint32_t)(blk * TN), as + 8 * kk, desc_sw128(bd + kk * 32), (i | kk) ? 1u : 0u);
+                            mma_f16(tmem + (uint32_t)(blk * TN), as + 8 * kk, desc_sw128(bd + kk * 32),
+                                    i > i0 || kk ? 1u : 0u);
                     }
                     umma_commit(&tfull[blk]);
                 }
@@ -863,7 +871,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[k % RING]);
         };
-        for (int t = first; t < last && !*abort_flag; ++t, idx += SLICES) {
+        for (int t = first; t < last && !*abort_flag; ++t, idx += GROUPS) {
             const int rb = t / col_tiles, ct = t - rb * col_tiles;
             if (rb != rb_now) {
                 // this row block's slices into tensor memory (its MMAs have all
@@ -902,7 +910,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             int lo[EPI_COLS], mid[EPI_COLS];
             float v[8];
 #pragma unroll
-            for (int g = 0; g < 5; ++g) {
+            for (int g = 0; g < 6; ++g) {
                 const uint32_t a = arrived(idx + g);
 #pragma unroll
                 for (int h = 0; h < EPI_COLS / 8; ++h) {
@@ -910,16 +918,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int k = 8 * h + q;
-                        if (g == 0) lo[k] = (__float2int_rn(v[q]) + 128) >> 8;
-                        else if (g == 1) lo[k] += __float2int_rn(v[q]);
-                        else if (g == 2) lo[k] += __float2int_rn(v[q]) * 256;
-                        else if (g == 3) mid[k] = small_int(v[q]);
+                        if (g == 0) lo[k] = __float2int_rn(v[q]) + 32768;
+                        else if (g == 1) lo[k] = (lo[k] + __float2int_rn(v[q]) * 256) >> 16;
+                        else if (g == 2) lo[k] += __float2int_rn(v[q]);
+                        else if (g == 3) lo[k] += __float2int_rn(v[q]) * 256;
+                        else if (g == 4) mid[k] = small_int(v[q]);
                         else mid[k] += small_int(v[q]) * 256;
                     }
                 }
                 release(idx + g);
             }
-            const uint32_t a2 = arrived(idx + 5), a1 = arrived(idx + 6);
+            const uint32_t a2 = arrived(idx + 6), a1 = arrived(idx + 7);
             if (!ok) {
                 fail();
                 break;
@@ -940,8 +949,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     mid[k] = (int)(T >> 32);
                 }
             }
-            release(idx + 5);
             release(idx + 6);
+            release(idx + 7);
 #pragma unroll
             for (int h = 0; h < EPI_COLS / 4; ++h) {
                 double c[4], d[4];
@@ -993,8 +1002,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // block instead of two).  Waits are bounded (error word, then the ticket
 // carries on).  Four warps take 8 columns of a 32 x 32 block each; a block's
 // product is 8 complex multiply-adds of 4 x 65 clocks per warp, which with the
-// trip through L2 and the diagonal's product is the chain per block (about
-// 3 us; one cluster of 16 SMs walking the blocks took 14 to 24 us).
+// trip through L2 and the diagonal's three products is the chain per block
+// (one cluster of 16 SMs walking the blocks took 14 to 24 us per block).
+//
+// The inverse of a triangular block loses digits where the block is
+// ill-conditioned (twice the error of a substitution for random matrices), so its
+// product is corrected once by the residual against the block itself.  And the
+// sums over the blocks cancel against the right-hand side, so the blocks' products
+// are added without rounding error: as one running sum they made up most of the
+// error of x (n = 320: 1.7e-13 against 0.4e-13).
 constexpr int SOLVE_THREADS = 128;
 constexpr unsigned long long UNSET = ~0ull;
 
@@ -1002,6 +1018,13 @@ __device__ __forceinline__ bool is_unset(double2 v) {
     return (unsigned long long)__double_as_longlong(v.x) == UNSET ||
            (unsigned long long)__double_as_longlong(v.y) == UNSET;
 }
+// acc + low += v, the rounding error of acc + v kept in low (Knuth's two-sum).
+__device__ __forceinline__ void add_exactly(double& acc, double& low, double v) {
+    const double s = acc + v, t = s - acc;
+    low += (acc - (s - t)) + (v - t);
+    acc = s;
+}
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ double settled(double v) {
     return (unsigned long long)__double_as_longlong(v) == UNSET ? __longlong_as_double(0x7ff8000000000000ll) : v;
 }
@@ -1031,9 +1054,12 @@ __global__ void __launch_bounds__(SOLVE_THREADS) lu64_solve_kernel(int64_t n, co
                                                                    const int* __restrict__ order, double2* b, double2* z,
                                                                    double2* xr, int* __restrict__ counter,
                                                                    int* __restrict__ info, int* __restrict__ err) {
-    __shared__ double2 red[4][NB];
+    __shared__ double2 red[3][4][NB], ysum[NB];
     __shared__ int tk;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto sum = [&](int set, int row) {
+        return cadd(cadd(red[set][0][row], red[set][1][row]), cadd(red[set][2][row], red[set][3][row]));
+    };
     const int nblk = (int)((n + NB - 1) / NB);
     for (;;) {
         __syncthreads();
@@ -1047,12 +1073,18 @@ __global__ void __launch_bounds__(SOLVE_THREADS) lu64_solve_kernel(int64_t n, co
         const bool rok = r < n;
         const double2* y = fwd ? z : xr;
         const int steps = fwd ? rb : nblk - 1 - rb;
-        double2 acc = make_double2(0, 0);
-        // the diagonal block's inverse and the right-hand side, ahead of the waits
-        double2 d[8], rhs = make_double2(0, 0);
+        double2 acc = make_double2(0, 0), low = acc;
+        // the diagonal block, its inverse and the right-hand side, ahead of the waits
+        double2 d[8], e[8], rhs = make_double2(0, 0);
         const double2* D = Dinv + ((int64_t)rb * 2 + (fwd ? 0 : 1)) * (NB * NB) + (8 * warp) * NB + lane;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) d[i] = D[i * NB];
+        for (int i = 0; i < 8; ++i) {
+            const int col = 8 * warp + i;
+            const int64_t c = (int64_t)rb * NB + col;
+            d[i] = D[i * NB];
+            e[i] = rok && c < n && (fwd ? col < lane : col >= lane) ? A[c * lda + r]
+                                                                    : make_double2(fwd && col == lane ? 1.0 : 0.0, 0);
+        }
         if (warp == 0 && fwd && rok) rhs = b[order[r]];
         for (int i = 0; i < steps; ++i) {
             const int k = fwd ? i : nblk - 1 - i;
@@ -1072,9 +1104,14 @@ __global__ void __launch_bounds__(SOLVE_THREADS) lu64_solve_kernel(int64_t n, co
                 }
             }
             __syncwarp();
-            block_product(acc, a, xv);
+            double2 part = make_double2(0, 0);
+            block_product(part, a, xv);
+            add_exactly(acc.x, low.x, part.x);
+            add_exactly(acc.y, low.y, part.y);
         }
-        red[warp][lane] = acc;
+        if (finite_bits(low.x)) acc.x += low.x;
+        if (finite_bits(low.y)) acc.y += low.y;
+        red[0][warp][lane] = acc;
         if (!fwd && warp == 0 && rok) {
             rhs = ld_relaxed(z + r);
             for (unsigned it = 0; is_unset(rhs); ++it) {
@@ -1088,16 +1125,26 @@ __global__ void __launch_bounds__(SOLVE_THREADS) lu64_solve_kernel(int64_t n, co
             if (u.x == 0.0 && u.y == 0.0) atomicCAS(info, 0, (int)(r + 1));
         }
         __syncthreads();
-        __shared__ double2 ysum[NB];
-        if (warp == 0)
-            ysum[lane] = csub(rhs, cadd(cadd(red[0][lane], red[1][lane]), cadd(red[2][lane], red[3][lane])));
+        if (warp == 0) ysum[lane] = csub(rhs, sum(0, lane));
+        __syncthreads();
+        // y = D^-1 (right-hand side), then once more with what D y leaves of it
+        const int c8 = 8 * warp + (lane & 7);
+        acc = make_double2(0, 0);
+        block_product(acc, d, ysum[c8]);
+        red[1][warp][lane] = acc;
         __syncthreads();
         acc = make_double2(0, 0);
-        block_product(acc, d, lane < 8 ? ysum[8 * warp + lane] : make_double2(0, 0));
-        red[warp][lane] = acc;
+        block_product(acc, e, sum(1, c8));
+        red[2][warp][lane] = acc;
+        __syncthreads();
+        acc = make_double2(0, 0);
+        block_product(acc, d, csub(ysum[c8], sum(2, c8)));
+        red[0][warp][lane] = acc;
         __syncthreads();
         if (warp == 0 && rok) {
-            double2 v = cadd(cadd(red[0][lane], red[1][lane]), cadd(red[2][lane], red[3][lane]));
+            double2 v = sum(1, lane);
+            const double2 f = sum(0, lane);
+            if (finite_bits(f.x) && finite_bits(f.y)) v = cadd(v, f);
             v = make_double2(settled(v.x), settled(v.y));
             st_relaxed((fwd ? z : xr) + r, v);
             if (!fwd) b[r] = v;  // every forward block has been read by now

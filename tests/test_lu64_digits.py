@@ -1,11 +1,12 @@
 """The trailing update of the FP64 LU (csrc/lu64.cu) restated with Python
 integers: entries split into seven digits of eight bits relative to the largest
-of their row (L21) or column (U12), the 28 digit products of the highest
+of their row (L21) or column (U12), the 34 digit products of the highest
 weights, sums kept as integers.  The bound checked is the one the kernel
-claims: every group of products stays below 2^24 (exact in FP32 accumulation)
-and the product is within 2^-52 of (largest of the row) x (largest of the
-column) x K / 4, a quarter of which is the rounding of the last group and the
-rest the products left out."""
+claims: every group of products stays below 2^24 (exact in FP32 accumulation),
+the two lowest groups fit 32-bit integers together, and the product is within
+(K / 2 + 1) 2^-54 of (largest of the row) x (largest of the column): half a unit
+2^-55 from the splitting of either factor, half a unit 2^-54 from the rounding
+of the lowest groups, less than that from the products left out."""
 import numpy as np
 import pytest
 
@@ -46,11 +47,13 @@ def test_digit_products(kind):
         ea, eb = exponent(a), exponent(b)
         da, db = [digits(x, ea) for x in a], [digits(x, eb) for x in b]
         G = [sum(da[k][s] * db[k][g - s] for k in range(K) for s in range(g + 1)) for g in range(S)]
+        G.append(sum(da[k][s] * db[k][7 - s] for k in range(K) for s in range(1, S)))
         assert max(abs(x) for x in G) < 2 ** 24
-        T = sum(G[g] << (8 * (5 - g)) for g in range(6)) + ((G[6] + 128) >> 8)
+        assert abs(G[6] * 256 + G[7] + 32768) < 2 ** 31
+        T = sum(G[g] << (8 * (5 - g)) for g in range(6)) + ((G[6] * 256 + G[7] + 32768) >> 16)
         assert abs(T) < 2 ** 62
         from fractions import Fraction
         exact = sum(Fraction(x) * Fraction(y) for x, y in zip(a, b))
         got = Fraction(T) * Fraction(2) ** (ea + eb - 54)
-        bound = Fraction(K, 4) * Fraction(2) ** (ea + eb - 52)
+        bound = (Fraction(K, 2) + 1) * Fraction(2) ** (ea + eb - 54)
         assert abs(got - exact) <= bound
