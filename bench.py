@@ -336,9 +336,7 @@ def main():
         ctx.check(ctx.lib.bem_run(ctx.h, pd.h, form, precond, bem._ptr(sc), bem._ptr(inc), reps, check))
 
     if args.profile_only:
-        # the library's per-stage timing runs GMRES iteration by iteration:
-        # every kernel is its own launch (a profiler sees them, as it does not
-        # inside the solve graph's device-side loop)
+        # the library's per-stage timing runs GMRES iteration by iteration
         ctx.set_profiling(True)
         run_mixed()
         torch.cuda.synchronize()

@@ -356,6 +356,7 @@ BEM_API void bem_ctx_destroy(bem_ctx* ctx) {
         cudaStreamSynchronize(ctx->c.lu64_side);
         cudaStreamDestroy(ctx->c.lu64_side);
     }
+    if (ctx->c.progress) cudaFreeHost(ctx->c.progress);
     if (ctx->c.lu64_ready) cudaEventDestroy(ctx->c.lu64_ready);
     if (ctx->c.lu64_done) cudaEventDestroy(ctx->c.lu64_done);
     delete ctx;

@@ -2,7 +2,7 @@
 // per body and one frequency at a time (analysis.rs:87-111); here every
 // frequency of every body is assembled by one multi-body launch and all
 // systems are solved by one ragged batched GMRES (systems of different sizes
-// side by side, CUDA-graph captured), so small bodies do not leave the GPU
+// side by side, launched as CUDA graphs), so small bodies do not leave the GPU
 // idle.  Bodies are grouped into chunks whose operators fit a share of the
 // free device memory.
 #include <algorithm>
@@ -206,7 +206,7 @@ void solve_chunk(Context& c, std::vector<BodyPlan*>& bodies, bem_precond precond
     std::vector<GmState> st;
     {
         BatchStage bs(c, "batch_gmres");
-        gm_run(c, ws, c.profiling ? 0 : 4, cap);
+        gm_run(c, ws, 2, cap);
         gm_read_states(c, ws, st);
     }
     // ---- surface unknowns and field points

@@ -231,6 +231,7 @@ struct Context {
     // between the two
     cudaStream_t lu64_side = nullptr;
     cudaEvent_t lu64_ready = nullptr, lu64_done = nullptr;
+    int* progress = nullptr;  // rounds of the running GMRES solve, written by the device (mapped host memory)
     int gm_cluster = 0;    // the same for the Arnoldi step of the reference's form
     // results of the last bem_run
     std::vector<double> last_phi, last_vn;

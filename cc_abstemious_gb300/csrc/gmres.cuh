@@ -146,12 +146,7 @@ struct GmWorkspace {
     // dense operator's n^2 entries)
     double mv_bytes = 0;
     const char* mv_stage = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
-    int graph_chunk = 0, graph_rounds = 0;
-    bool graph_loop = false;  // graph_exec is the whole solve (device-side loop)
-    DevBuf rounds;            // rounds the solve graph ran
-    int64_t launches_per_graph = 0;
-    ~GmWorkspace();
+    DevBuf rounds;  // finished rounds of gm_run
 };
 
 void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const void* A, int64_t lda,

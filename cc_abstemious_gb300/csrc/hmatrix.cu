@@ -1176,7 +1176,7 @@ GmresResult gmres_hmatrix(Context& c, const HMatrixDev& H, int64_t max_it, doubl
     BEM_CUDA(cudaMemcpyAsync(ws.bt.B, x, sizeof(double2) * n, cudaMemcpyDeviceToDevice, c.stream));
     BEM_CUDA(cudaMemcpyAsync(ws.anorm, &H.norm, sizeof(double), cudaMemcpyHostToDevice, c.stream));
     gm_init(c, ws, tol, restarts);
-    gm_run(c, ws, 0, restarts * (int64_t)m + 1);
+    gm_run(c, ws, 1, restarts * (int64_t)m + 1);
     std::vector<GmState> st;
     gm_read_states(c, ws, st);
     BEM_CUDA(cudaMemcpyAsync(x, ws.bt.X, sizeof(double2) * n, cudaMemcpyDeviceToDevice, c.stream));

@@ -245,7 +245,7 @@ static void run_mixed_range(Context& c, Problem& p, int64_t F0, int64_t nf, bem_
             precond = hmixed_block_jacobi(c, ws, Hm) ? BEM_PRECOND_BLOCK_JACOBI : BEM_PRECOND_NONE;
         else if (precond != BEM_PRECOND_NONE)
             precond = precond_setup(c, p, ws, precond, ks_sys.data());
-        gm_run(c, ws, c.profiling ? 0 : 4, restarts * (int64_t)m + 1);
+        gm_run(c, ws, 2, restarts * (int64_t)m + 1);
         gm_read_states(c, ws, st);
         int64_t mv = 0;
         for (auto& x : st) mv += x.num_mv;
