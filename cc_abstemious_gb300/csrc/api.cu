@@ -352,13 +352,13 @@ BEM_API void bem_ctx_destroy(bem_ctx* ctx) {
         cudaStreamSynchronize(ctx->c.stream);
         cudaStreamDestroy(ctx->c.stream);
     }
-    if (ctx->c.lu64_side) {
-        cudaStreamSynchronize(ctx->c.lu64_side);
-        cudaStreamDestroy(ctx->c.lu64_side);
+    if (ctx->c.side) {
+        cudaStreamSynchronize(ctx->c.side);
+        cudaStreamDestroy(ctx->c.side);
     }
     if (ctx->c.progress) cudaFreeHost(ctx->c.progress);
-    if (ctx->c.lu64_ready) cudaEventDestroy(ctx->c.lu64_ready);
-    if (ctx->c.lu64_done) cudaEventDestroy(ctx->c.lu64_done);
+    if (ctx->c.forked) cudaEventDestroy(ctx->c.forked);
+    if (ctx->c.joined) cudaEventDestroy(ctx->c.joined);
     delete ctx;
 }
 

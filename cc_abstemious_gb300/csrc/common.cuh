@@ -227,10 +227,27 @@ struct Context {
     DevBuf w_piv;     // the plain form's FP64 LU: row order, diagonal blocks' inverses
     DevBuf w_lu64;    // its trailing update's digit images
     int lu64_cluster = 0;  // largest cluster its panels run on (0: not asked yet)
-    // its second stream (created with the first factorization) and the events
-    // between the two
-    cudaStream_t lu64_side = nullptr;
-    cudaEvent_t lu64_ready = nullptr, lu64_done = nullptr;
+    // a second stream for work beside that of `stream` (created when first
+    // needed) and the events between the two
+    cudaStream_t side = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
+    void need_side() {
+        if (side) return;
+        BEM_CUDA(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+        BEM_CUDA(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
+        BEM_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    }
+    // what `side` runs from here on follows what `stream` has been given
+    void fork() {
+        need_side();
+        BEM_CUDA(cudaEventRecord(forked, stream));
+        BEM_CUDA(cudaStreamWaitEvent(side, forked, 0));
+    }
+    // what `stream` runs from here on follows what `side` has been given
+    void join() {
+        BEM_CUDA(cudaEventRecord(joined, side));
+        BEM_CUDA(cudaStreamWaitEvent(stream, joined, 0));
+    }
     int* progress = nullptr;  // rounds of the running GMRES solve, written by the device (mapped host memory)
     int gm_cluster = 0;    // the same for the Arnoldi step of the reference's form
     // results of the last bem_run

@@ -193,8 +193,9 @@ __device__ __forceinline__ double wsum(double v) {
 // argmax of |v[t]| over t not excluded; first index wins ties (aca.rs:256-268).
 // Moduli (hypot, about 25 FP64 instructions) only of the entries whose square
 // is within a few rounding errors of the largest square, which decides the
-// others.
-__device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t len, double* sh, int64_t* shi) {
+// others.  The winner's is returned beside its index (-1 where there is none).
+__device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t len, double* sh, int64_t* shi,
+                                double& modulus) {
     const long long inf = 0x7ff0000000000000ll;
     auto square = [&](int64_t t) {  // as the bits of a non-negative double; -1: excluded or NaN
         if (excl[t]) return -1ll;
@@ -236,13 +237,18 @@ __device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t le
             int64_t oi = __shfl_down_sync(0xffffffffu, bi, o);
             if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
         }
-        if (l == 0) shi[32] = bi;
+        if (l == 0) {
+            shi[32] = bi;
+            sh[41] = best;
+        }
     }
     __syncthreads();
+    modulus = sh[41];
     return shi[32];
 }
 
 constexpr int LEAF_THREADS = 256;
+constexpr int ACA_RMAX = 256;  // largest rank of a compressed leaf
 constexpr int JACOBI_SMEM = 32;  // ranks up to this run the Jacobi sweeps in shared memory
 
 // Dense (inadmissible) leaves: one CTA per leaf, entries column-major m x n.
@@ -288,8 +294,22 @@ __device__ __forceinline__ double bnsq(const double2* a, int64_t len, double* sh
     return bsum(acc, sh);
 }
 
+// The warp that does a leaf's single-warp work: a different one from CTA to CTA,
+// since a warp's number decides the SM quarter whose FP64 pipe it uses.
+__device__ __forceinline__ int lead_warp(int warps) {
+    return (int)((blockIdx.x * 0x9E3779B1u) >> 20) & (warps - 1);
+}
+
 // Partially pivoted ACA (aca.rs:57-136) of every admissible leaf.
-__global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restrict__ leaves,
+//
+// FP64 instructions bound it, and in a small leaf those that are not entries:
+// moduli, quotients and roots cost 600 to 1600 clocks of an SM quarter per warp
+// however few lanes want them.  So they are gathered: the moduli of the norm
+// estimate one lane per earlier rank, the pivot's quotient and the roots once per
+// leaf, by one warp that differs from leaf to leaf.  (1534 leaves of n = 2560: 3.7
+// ms with every warp doing them, 2.8 this way.)
+constexpr int ACA_THREADS = 128;
+__global__ void __launch_bounds__(ACA_THREADS, 4) hm_aca_kernel(HLeaf* __restrict__ leaves,
                                                               const int32_t* __restrict__ list,
                                                               const int64_t* __restrict__ rows,
                                                               const int64_t* __restrict__ cols, GenParams g,
@@ -298,10 +318,12 @@ __global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restri
     __shared__ double sh[48];
     __shared__ int64_t shi[33];
     __shared__ DevRng rng;
-    __shared__ int64_t s_iref, s_jref, s_istar, s_jstar;
+    __shared__ int64_t s_iref, s_jref;
     __shared__ double s_total;
     __shared__ int s_stop;
-    __shared__ double s_prod[256];  // one per earlier rank (kmax <= ACA_RMAX = 256)
+    __shared__ double2 s_f, s_du[ACA_RMAX], s_dv[ACA_RMAX];  // one per rank (kmax <= ACA_RMAX)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = ACA_THREADS / 32, lead = lead_warp(nw);
+    const double limit = tol / 50.0;
     HLeaf& L = leaves[list[blockIdx.x]];
     const int64_t m = L.m, n = L.n;
     const int64_t nr = m < n ? m : n;
@@ -331,26 +353,29 @@ __global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restri
             if (threadIdx.x == 0) atomicOr(err, 8);
             break;
         }
-        int64_t jstar = bargmax_excl(riref, jex, n, sh, shi);
-        double jval = hypot(riref[jstar].x, riref[jstar].y);
-        int64_t istar = bargmax_excl(rjref, iex, m, sh, shi);
-        double ival = hypot(rjref[istar].x, rjref[istar].y);
+        double jval, ival, unused;
+        int64_t jstar = bargmax_excl(riref, jex, n, sh, shi, jval);
+        int64_t istar = bargmax_excl(rjref, iex, m, sh, shi, ival);
         if (ival > jval) {
             aca_res_row(g, L, rows, cols, U, V, rank, istar, ristar);
-            jstar = bargmax_excl(ristar, jex, n, sh, shi);
+            jstar = bargmax_excl(ristar, jex, n, sh, shi, unused);
             aca_res_col(g, L, rows, cols, U, V, rank, jstar, rjstar);
         } else {
             aca_res_col(g, L, rows, cols, U, V, rank, jstar, rjstar);
-            istar = bargmax_excl(rjstar, iex, m, sh, shi);
+            istar = bargmax_excl(rjstar, iex, m, sh, shi, unused);
             aca_res_row(g, L, rows, cols, U, V, rank, istar, ristar);
         }
-        const z2 piv = ristar[jstar];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            iex[istar] = 1;
-            jex[jstar] = 1;
+        if (warp == lead) {  // 1 / pivot, a part per lane
+            const z2 piv = ristar[jstar];
+            const double den = piv.x * piv.x + piv.y * piv.y, part = (lane ? -piv.y : piv.x) / den;
+            if (lane < 2) reinterpret_cast<double*>(&s_f)[lane] = part;
+            if (lane == 0) {
+                iex[istar] = 1;
+                jex[jstar] = 1;
+            }
         }
-        const z2 f = cdiv(make_double2(1.0, 0.0), piv);
+        __syncthreads();
+        const z2 f = s_f;
         double2* uk = U + (size_t)k * m;
         double2* vk = V + (size_t)k * n;
         for (int64_t t = threadIdx.x; t < n; t += blockDim.x) vk[t] = cmul(ristar[t], f);
@@ -358,31 +383,41 @@ __global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restri
         __syncthreads();
         rank = (int)k + 1;
         // update_norm_estimate (aca.rs:224-241): the products with every
-        // earlier rank one warp each, summed in rank order by one thread
-        double nk = bnsq(uk, m, sh) * bnsq(vk, n, sh);
-        {
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-            for (int t = warp; t < k; t += nw) {
-                const double2* ut = U + (size_t)t * m;
-                const double2* vt = V + (size_t)t * n;
-                z2 du = make_double2(0, 0), dv = make_double2(0, 0);
+        // earlier rank and the new rank's norms one warp each, the moduli one lane
+        // each, summed in rank order
+        for (int t = warp; t <= k; t += nw) {
+            const double2* ut = U + (size_t)t * m;
+            const double2* vt = V + (size_t)t * n;
+            z2 du = make_double2(0, 0), dv = make_double2(0, 0);
+            if (t < k) {
                 for (int64_t i = lane; i < m; i += 32) cfma(du, ut[i], uk[i]);
                 for (int64_t j = lane; j < n; j += 32) cfma(dv, vt[j], vk[j]);
-                du = wsum2(du);
-                dv = wsum2(dv);
-                if (lane == 0) s_prod[t] = 2.0 * hypot(du.x, du.y) * hypot(dv.x, dv.y);
+            } else {
+                for (int64_t i = lane; i < m; i += 32) du.x = fma(uk[i].x, uk[i].x, fma(uk[i].y, uk[i].y, du.x));
+                for (int64_t j = lane; j < n; j += 32) dv.x = fma(vk[j].x, vk[j].x, fma(vk[j].y, vk[j].y, dv.x));
+            }
+            wsum4(du, dv);
+            if (lane == 0) {
+                s_du[t] = du;
+                s_dv[t] = dv;
             }
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (warp == lead) {
+            for (int t = lane; t < k; t += 32)
+                s_du[t].x = 2.0 * hypot(s_du[t].x, s_du[t].y) * hypot(s_dv[t].x, s_dv[t].y);
+            __syncwarp();
+            const double nk = s_du[k].x * s_dv[k].x;
             double add = 0;
-            for (int t = 0; t < k; ++t) add += s_prod[t];
-            s_total += nk;
-            s_total += add;
-            double step = sqrt(nk) / sqrt(s_total);
-            s_stop = step < tol / 50.0;
-            s_istar = istar;
-            s_jstar = jstar;
+            for (int t = 0; t < k; ++t) add += s_du[t].x;
+            const double total = s_total + nk + add;
+            __syncwarp();
+            const double root = sqrt(lane ? total : nk);
+            const double step = __shfl_sync(0xffffffffu, root, 0) / __shfl_sync(0xffffffffu, root, 1);
+            if (lane == 0) {
+                s_total = total;
+                s_stop = step < limit;
+                }
         }
         __syncthreads();
         if (s_stop) break;
@@ -439,68 +474,120 @@ __global__ void __launch_bounds__(LEAF_THREADS, 2) hm_aca_kernel(HLeaf* __restri
 // one-sided Jacobi, truncation at s < tol * cumulative sum (+1, at least 1),
 // then U <- Q_u W Sigma and V <- Q_v Z with Z = (V^H)^T (plain transpose, the
 // factors pair as u v^T).
-__device__ void house_qr_dev(double2* A, int64_t m, int r, double2* R, double2* tau) {
+//
+// A leaf's CTA has four warps, one per SM quarter; both factors are reduced in the
+// same loop, so that the serial part of a reflector (a root and a quotient, lanes
+// side by side) is paid once for the two.
+constexpr int RC_THREADS = 128, RC_WARPS = RC_THREADS / 32;
+
+// x -= tau v (v^H x) for two columns at once (q may be missing), rows k .. m of a
+// warp: one pass over v, and the two sums share their additions.
+__device__ __forceinline__ void reflect_two(const double2* __restrict__ v, double2* __restrict__ p,
+                                            double2* __restrict__ q, int64_t k, int64_t m, double tau, int lane) {
+    z2 d = make_double2(0, 0), e = d;
+    if (q) {
+#pragma unroll 2
+        for (int64_t i = k + lane; i < m; i += 32) {
+            const z2 a = cconj(v[i]);
+            cfma(d, a, p[i]);
+            cfma(e, a, q[i]);
+        }
+        wsum4(d, e);
+        d = cscale(d, -tau);
+        e = cscale(e, -tau);
+#pragma unroll 2
+        for (int64_t i = k + lane; i < m; i += 32) {
+            const z2 a = v[i];
+            z2 x = p[i], y = q[i];
+            cfma(x, a, d);
+            cfma(y, a, e);
+            p[i] = x;
+            q[i] = y;
+        }
+    } else {
+        for (int64_t i = k + lane; i < m; i += 32) cfma(d, cconj(v[i]), p[i]);
+        d = cscale(wsum2(d), -tau);
+        for (int64_t i = k + lane; i < m; i += 32) cfma(p[i], v[i], d);
+    }
+}
+
+__device__ void house_qr_dev(double2* A0, int64_t m0, double2* R0, double2* tau0, double2* A1, int64_t m1, double2* R1,
+                             double2* tau1, int r, int lead) {
     // A: m x r column-major; on exit the reflectors v_k = x - alpha e_k are
-    // kept in A below and on the diagonal.  Warp 0 forms column k's reflector
-    // (|v_k|^2 = 2 |x| (|x| + |x_0|), no second reduction), every warp applies
-    // it to its share of the later columns: two barriers per k.
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __shared__ double s_tau;
+    // kept in A below and on the diagonal.  One warp per factor forms column k's
+    // reflector (|v_k|^2 = 2 |x| (|x| + |x_0|), no second reduction), every warp
+    // applies them to its share of the later columns: two barriers per k.
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mine = (warp - lead) & (RC_WARPS - 1);
+    __shared__ double s_tau[2];
     for (int k = 0; k < r; ++k) {
-        double2* a = A + (size_t)k * m;
-        if (warp == 0) {
+        if (mine < 2) {
+            double2* a = (mine ? A1 : A0) + (size_t)k * (mine ? m1 : m0);
+            const int64_t m = mine ? m1 : m0;
             const z2 x0 = a[k];
             double nx2 = 0;
             for (int64_t i = k + lane; i < m; i += 32) nx2 = fma(a[i].x, a[i].x, fma(a[i].y, a[i].y, nx2));
-            const double nx = sqrt(wsum(nx2)), ax0 = sqrt(cnorm2(x0));
-            const double inv0 = ax0 == 0 ? 0.0 : 1.0 / ax0;
-            const z2 ph = ax0 == 0 ? make_double2(1.0, 0.0) : make_double2(x0.x * inv0, x0.y * inv0);
+            nx2 = wsum(nx2);
+            const double root = sqrt(lane ? cnorm2(x0) : nx2);
+            const double nx = __shfl_sync(0xffffffffu, root, 0), ax0 = __shfl_sync(0xffffffffu, root, 1);
+            const double half = nx * (nx + ax0);
+            const double part = (lane == 0 ? x0.x : lane == 1 ? x0.y : 1.0) / (lane < 2 ? ax0 : half);
+            z2 ph = make_double2(__shfl_sync(0xffffffffu, part, 0), __shfl_sync(0xffffffffu, part, 1));
+            double tk = __shfl_sync(0xffffffffu, part, 2);
+            if (ax0 == 0) ph = make_double2(1.0, 0.0);
+            if (half == 0) tk = 0.0;
             const z2 alpha = make_double2(-ph.x * nx, -ph.y * nx);
-            const double half = nx * (nx + ax0), tk = half == 0 ? 0.0 : 1.0 / half;
             __syncwarp();
             if (lane == 0) {
                 a[k] = csub(x0, alpha);
-                R[(size_t)k * r + k] = alpha;
-                tau[k] = make_double2(tk, 0.0);
-                s_tau = tk;
+                (mine ? R1 : R0)[(size_t)k * r + k] = alpha;
+                (mine ? tau1 : tau0)[k] = make_double2(tk, 0.0);
+                s_tau[mine] = tk;
             }
         }
         __syncthreads();
-        const double tk = s_tau;
-        for (int j = k + 1 + warp; j < r; j += nw) {
-            double2* c = A + (size_t)j * m;
-            z2 d = make_double2(0, 0);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(d, cconj(a[i]), c[i]);
-            d = cscale(wsum2(d), -tk);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(c[i], a[i], d);
+        const int later = r - k - 1, pairs = (later + 1) / 2;
+        for (int t = warp; t < 2 * pairs; t += RC_WARPS) {
+            const bool second = t >= pairs;
+            const int64_t m = second ? m1 : m0;
+            const int j = k + 1 + 2 * (second ? t - pairs : t);
+            double2* A = second ? A1 : A0;
+            reflect_two(A + (size_t)k * m, A + (size_t)j * m, j + 1 < r ? A + (size_t)(j + 1) * m : nullptr, k, m,
+                        s_tau[second], lane);
         }
         __syncthreads();
     }
     // R above the diagonal lives in rows < k of columns k
-    for (int t = threadIdx.x; t < r * r; t += blockDim.x) {
+    for (int t = threadIdx.x; t < r * r; t += RC_THREADS) {
         const int i = t % r, j = t / r;
-        if (i != j) R[t] = i < j ? A[(size_t)j * m + i] : make_double2(0, 0);
+        if (i == j) continue;
+        R0[t] = i < j ? A0[(size_t)j * m0 + i] : make_double2(0, 0);
+        R1[t] = i < j ? A1[(size_t)j * m1 + i] : make_double2(0, 0);
     }
     __syncthreads();
 }
 
-// out (m x c) = Q [B; 0] where Q = H_0 ... H_{r-1} (reflectors in A), B r x c.
-// A warp carries its columns through all reflectors; the columns do not meet.
-__device__ void house_apply_dev(const double2* A, int64_t m, int r, const double2* tau, const double2* B, int c,
-                                double2* out) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int j = warp; j < c; j += nw) {
-        double2* o = out + (size_t)j * m;
-        for (int64_t i = lane; i < m; i += 32) o[i] = i < r ? B[(size_t)j * r + i] : make_double2(0, 0);
+// out (m x c) = Q [B; 0] where Q = H_0 ... H_{r-1} (reflectors in A), B r x c,
+// for both factors.  A warp carries its columns through all reflectors; the
+// columns do not meet.
+__device__ void house_apply_dev(const double2* A0, int64_t m0, const double2* tau0, const double2* B0, double2* out0,
+                                const double2* A1, int64_t m1, const double2* tau1, const double2* B1, double2* out1,
+                                int r, int c) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pairs = (c + 1) / 2;
+    for (int t = warp; t < 2 * pairs; t += RC_WARPS) {
+        const bool second = t >= pairs;
+        const int j = 2 * (second ? t - pairs : t);
+        const int64_t m = second ? m1 : m0;
+        const double2 *A = second ? A1 : A0, *tau = second ? tau1 : tau0, *b = (second ? B1 : B0) + (size_t)j * r;
+        double2 *o = (second ? out1 : out0) + (size_t)j * m, *p = j + 1 < c ? o + m : nullptr;
+        for (int64_t i = lane; i < m; i += 32) {
+            o[i] = i < r ? b[i] : make_double2(0, 0);
+            if (p) p[i] = i < r ? b[r + i] : make_double2(0, 0);
+        }
         __syncwarp();
         for (int k = r - 1; k >= 0; --k) {
-            const double2* v = A + (size_t)k * m;
             const double tk = tau[k].x;
             if (tk == 0.0) continue;
-            z2 d = make_double2(0, 0);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(d, cconj(v[i]), o[i]);
-            d = cscale(wsum2(d), -tk);
-            for (int64_t i = k + lane; i < m; i += 32) cfma(o[i], v[i], d);
+            reflect_two(A + (size_t)k * m, o, p, k, m, tk, lane);
             __syncwarp();
         }
     }
@@ -513,14 +600,15 @@ __device__ void house_apply_dev(const double2* A, int64_t m, int r, const double
 // finds no pair further than 1e-15 from orthogonal.
 //
 // Bound by FP64 issue (65 clocks per warp instruction however few lanes are
-// active), so a pair takes only as many lanes as fill the warps (16 columns:
-// one warp, four lanes per pair) and the rotation's angle comes from FP32: it
+// active), so a pair takes only as many lanes as fill the warps (18 columns:
+// one warp, three lanes per pair; more warps only for the largest ranks, which
+// would be the last to finish) and the rotation's angle comes from FP32: it
 // only has to be near, the next sweep corrects it; what is kept to FP64 is that
 // the rotation is unitary (its cosine and the phase, each one FP32 seed and a
-// third-order correction).  The right factor is not accumulated; the caller
-// forms it from W Sigma and the original matrix.  2560 triangles, leaf 32, eta 4:
-// the whole recompression 24.7 -> 7.8 ms, with the QR's reflectors formed by one
-// warp and the reductions' additions halved.
+// third-order correction).  The columns' norms follow the rotations and are
+// summed anew in every sweep.  The right factor is not accumulated; the caller
+// forms it from W Sigma and the original matrix.  2560 triangles, leaf 32, eta 4,
+// 1534 leaves with ranks up to 38: the whole recompression 24.7 -> 3.8 ms.
 // 1 / sqrt(v) for 0 < v (normal numbers).
 __device__ __forceinline__ double near_rsqrt(double v) {
     const int e = (((__double2hiint(v) >> 20) & 0x7ff) - 1023) & ~1;  // even
@@ -529,22 +617,41 @@ __device__ __forceinline__ double near_rsqrt(double v) {
     return fma(s * c, fma(0.375, c, 0.5), s);
 }
 
-__device__ void jacobi_dev(double2* M, int r, double* S, int* perm) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+__device__ void jacobi_dev(double2* M, int r, double* S, int* perm, int lead) {
+    const int lane = threadIdx.x & 31, nw = RC_WARPS, warp = ((threadIdx.x >> 5) - lead) & (nw - 1);
     const int rr = r + (r & 1), pairs = rr / 2;  // players of the round robin (index r: a bye when r is odd)
-    const int warps = r <= 16 ? 1 : r <= 32 ? 2 : r <= 48 ? 4 : 8;
-    int lpp = 32;  // lanes per pair
-    while (lpp > 1 && lpp * pairs > 32 * warps) lpp >>= 1;
+    const int warps = r <= 24 ? 1 : r <= 32 ? 2 : 4;
+    int lpp = 32;  // lanes per pair, any number: groups do not reach over warps
+    while (lpp > 1 && 32 / lpp * warps < pairs) --lpp;
     __shared__ int s_turned;
+    __shared__ double s_n[ACA_RMAX];  // squared norms of the columns
     if (warp < warps) {
         auto together = [&]() {
             if (warps == 1) __syncwarp();
             else asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
         };
-        const int groups = 32 * warps / lpp, grp = (warp * 32 + lane) / lpp, g = lane & (lpp - 1);
+        const int per = 32 / lpp, groups = per * warps, first = lane / lpp * lpp;
+        const int grp = lane < per * lpp ? warp * per + lane / lpp : 1 << 20, g = lane - first;
+        // sum over a group's lanes, in one order in all of them
+        auto group_sum = [&](double v) {
+            double t = __shfl_sync(0xffffffffu, v, first);
+            for (int o = 1; o < lpp; ++o) t += __shfl_sync(0xffffffffu, v, (first + o) & 31);
+            return t;
+        };
         for (int sweep = 0; sweep < 60 && r > 1; ++sweep) {
             together();
-            if (threadIdx.x == 0) s_turned = 0;
+            if (warp == 0 && lane == 0) s_turned = 0;
+            for (int c0 = 0; c0 < r; c0 += groups) {
+                const int c = c0 + grp;
+                double a = 0;
+                if (c < r)
+                    for (int i = g; i < r; i += lpp) {
+                        const z2 x = M[(size_t)c * r + i];
+                        a = fma(x.x, x.x, fma(x.y, x.y, a));
+                    }
+                a = group_sum(a);
+                if (c < r && g == 0) s_n[c] = a;
+            }
             together();
             for (int step = 0; step < rr - 1; ++step) {
                 for (int p0 = 0; p0 < pairs; p0 += groups) {
@@ -556,21 +663,11 @@ __device__ void jacobi_dev(double2* M, int r, double* S, int* perm) {
                     const bool on = pi < pairs && q < r;  // (q = r: the bye)
                     double2* up = M + (size_t)p * r;
                     double2* uq = M + (size_t)q * r;
-                    double a = 0, b = 0;
+                    const double a = on ? s_n[p] : 0.0, b = on ? s_n[q] : 0.0;
                     z2 cc = make_double2(0, 0);
                     if (on)
-                        for (int i = g; i < r; i += lpp) {
-                            const z2 x = up[i], y = uq[i];
-                            a = fma(x.x, x.x, fma(x.y, x.y, a));
-                            b = fma(y.x, y.x, fma(y.y, y.y, b));
-                            cfma(cc, cconj(x), y);
-                        }
-                    for (int o = 1; o < lpp; o <<= 1) {
-                        a += __shfl_xor_sync(0xffffffffu, a, o);
-                        b += __shfl_xor_sync(0xffffffffu, b, o);
-                        cc.x += __shfl_xor_sync(0xffffffffu, cc.x, o);
-                        cc.y += __shfl_xor_sync(0xffffffffu, cc.y, o);
-                    }
+                        for (int i = g; i < r; i += lpp) cfma(cc, cconj(up[i]), uq[i]);
+                    cc = make_double2(group_sum(cc.x), group_sum(cc.y));
                     const double n2 = cnorm2(cc);
                     const bool turn = on && n2 > 1e-290 && n2 > 1e-30 * (a * b);
                     if (!__any_sync(0xffffffffu, turn)) continue;
@@ -578,11 +675,16 @@ __device__ void jacobi_dev(double2* M, int r, double* S, int* perm) {
                     if (!turn) continue;
                     // tan of the angle from FP32, everything relative to max(a, b)
                     const int e = ((__double2hiint(fmax(a, b)) >> 20) & 0x7ff) - 1023;
-                    const double ri = near_rsqrt(n2);
-                    const float d = near_float(b, e) - near_float(a, e), f = 2.0f * near_float(n2 * ri, e);
+                    const double ri = near_rsqrt(n2), mod = n2 * ri;
+                    const float d = near_float(b, e) - near_float(a, e), f = 2.0f * near_float(mod, e);
                     const double t = (double)copysignf(__fdividef(f, fmaxf(fabsf(d) + sqrtf(fmaf(d, d, f * f)), 1e-37f)), d);
                     const double cs = near_rsqrt(fma(t, t, 1.0)), sn = cs * t;
                     const z2 se = cscale(cc, ri * sn);
+                    if (g == 0) {  // the norms after this rotation, whatever its angle
+                        const double t2 = t * t, c2 = cs * cs, tm = 2.0 * t * mod;
+                        s_n[p] = fmax(fma(t2, b, a - tm) * c2, 0.0);
+                        s_n[q] = fmax(fma(t2, a, b + tm) * c2, 0.0);
+                    }
                     for (int i = g; i < r; i += lpp) {
                         const z2 x = up[i], y = uq[i];
                         up[i] = make_double2(fma(cs, x.x, -fma(se.x, y.x, se.y * y.y)),
@@ -613,7 +715,7 @@ __device__ void jacobi_dev(double2* M, int r, double* S, int* perm) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __restrict__ leaves,
+__global__ void __launch_bounds__(RC_THREADS, 5) hm_recompress_kernel(HLeaf* __restrict__ leaves,
                                                                      const int32_t* __restrict__ list,
                                                                      double2* __restrict__ store,
                                                                      double2* __restrict__ scr,
@@ -638,8 +740,8 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
     double2* outV = outU + (size_t)m * r; // n x r
     double* S = reinterpret_cast<double*>(outV + (size_t)n * r);
     int* perm = reinterpret_cast<int*>(S + r);
-    house_qr_dev(U, m, r, Ru, tauu);
-    house_qr_dev(V, n, r, Rv, tauv);
+    const int lead = lead_warp(RC_WARPS);
+    house_qr_dev(U, m, Ru, tauu, V, n, Rv, tauv, r, lead);
     // RR = R_u R_v^T
     for (int t = threadIdx.x; t < r * r; t += blockDim.x) {
         int i = t % r, j = t / r;
@@ -649,7 +751,7 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
         M[(size_t)j * r + i] = acc;
     }
     __syncthreads();
-    jacobi_dev(M, r, S, perm);
+    jacobi_dev(M, r, S, perm, lead);
     // truncation (aca.rs:162-171)
     __shared__ int s_keep;
     if (threadIdx.x == 0) {
@@ -670,8 +772,6 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
     // U_new = Q_u (W Sigma)
     for (int t = 0; t < keep; ++t)
         for (int i = threadIdx.x; i < r; i += blockDim.x) B[(size_t)t * r + i] = M[(size_t)perm[t] * r + i];
-    __syncthreads();
-    house_apply_dev(U, m, r, tauu, B, keep, outU);
     // V_new = Q_v Z with Z the transpose of Sigma^-1 W^H (R_u R_v^T) =
     // Sigma^-2 (W Sigma)^H (R_u R_v^T)
     for (int t = threadIdx.x; t < keep * r; t += blockDim.x) {
@@ -680,10 +780,10 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
         const double sv = S[perm[c]], s2 = sv > 0 ? 1.0 / (sv * sv) : 0.0;
         z2 acc = make_double2(0, 0);
         for (int l = 0; l < r; ++l) cfma(acc, cconj(wt[l]), RR[(size_t)i * r + l]);
-        B[t] = cscale(acc, s2);
+        Rv[t] = cscale(acc, s2);  // (R_v is done with)
     }
     __syncthreads();
-    house_apply_dev(V, n, r, tauv, B, keep, outV);
+    house_apply_dev(U, m, tauu, B, outU, V, n, tauv, Rv, outV, r, keep);
     for (int t = 0; t < keep; ++t) {
         for (int64_t i = threadIdx.x; i < m; i += blockDim.x) U[(size_t)t * m + i] = outU[(size_t)t * m + i];
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) V[(size_t)t * n + i] = outV[(size_t)t * n + i];
@@ -691,7 +791,7 @@ __global__ void __launch_bounds__(LEAF_THREADS) hm_recompress_kernel(HLeaf* __re
     __syncthreads();
     // calculate_norm_estimate (aca.rs:212-222): |u_a|^2 |v_a|^2 and twice the
     // products of every pair of ranks, one warp per pair
-    __shared__ double s_tot[LEAF_THREADS / 32];
+    __shared__ double s_tot[RC_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     double sum = 0;
     for (int t = warp; t < keep * (keep + 1) / 2; t += nw) {
@@ -899,8 +999,6 @@ static GenParams gen_params(const Problem& p, int side) {
     return g;
 }
 
-constexpr int ACA_RMAX = 256;  // also the size of the ACA kernel's s_prod
-
 // The cluster tree and block leaves of a problem's collocation points (they
 // depend on the geometry, the leaf size and eta only, not on the frequency),
 // built on the device.
@@ -915,6 +1013,14 @@ static std::shared_ptr<HTrees> build_trees(Context& c, const Problem& p) {
     T->bl = forest_block_leaves(c, *T->F, p.in.hm_eta);
     return T;
 }
+
+// A leaf whose recompression is more than this share of an SM's is launched first
+// and keeps most others off its SM by the shared memory that it asks for, since the
+// largest leaf is the last to finish (1534 leaves: 5.7 ms without; shares of 0.1,
+// 0.2 and 0.35 all 3.9 ms, 0.9 4.9; with 60 KB 5.1, with 150 and 200 KB, which
+// leave it less L1 cache, 4.4 and 5.4).
+constexpr double RC_ALONE = 0.2;
+constexpr int RC_ALONE_SMEM = 100 * 1024;
 
 template <class Work>
 static std::vector<int32_t> heaviest_first(size_t count, Work work) {
@@ -1003,7 +1109,7 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
     if (!adm_list.empty()) {
         int* err = device_err(c);
         BEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), c.stream));
-        hm_aca_kernel<<<(unsigned)adm_list.size(), LEAF_THREADS, 0, c.stream>>>(
+        hm_aca_kernel<<<(unsigned)adm_list.size(), ACA_THREADS, 0, c.stream>>>(
             dl, d_adm.as<int32_t>(), H->d_rows.as<int64_t>(), H->d_cols.as<int64_t>(), g, H->d_store.as<double2>(),
             H->d_scratch.as<double2>(), p.in.hm_aca_tol, err);
         BEM_CHECK_LAUNCH(&c);
@@ -1013,13 +1119,12 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
         c.sync();
         require(herr == 0, "ACA rank exceeded the storage cap of " + std::to_string(ACA_RMAX),
                 BEM_ERR_NOT_CONVERGED);
-        std::stable_sort(adm_list.begin(), adm_list.end(), [&](int32_t a, int32_t b) {
-            auto work = [&](int32_t l) {
-                const HLeaf& L = H->leaves[(size_t)l];
-                return (int64_t)L.rank * L.rank * (L.m + L.n + 8 * L.rank);
-            };
-            return work(a) > work(b);
-        });
+        // FP64 clocks of a leaf's recompression, about
+        auto work = [&](int32_t l) {
+            const HLeaf& L = H->leaves[(size_t)l];
+            return (double)L.rank * L.rank * (8.0 * (double)(L.m + L.n) + 64.0 * L.rank);
+        };
+        std::stable_sort(adm_list.begin(), adm_list.end(), [&](int32_t a, int32_t b) { return work(a) > work(b); });
         BEM_CUDA(cudaMemcpyAsync(d_adm.p, adm_list.data(), sizeof(int32_t) * adm_list.size(), cudaMemcpyHostToDevice,
                                  c.stream));
         // recompression scratch sized by the ranks just found
@@ -1035,10 +1140,29 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
         d_off.ensure(sizeof(int64_t) * off.size());
         d_scr2.ensure(sizeof(double2) * (size_t)std::max<int64_t>(tot, 1));
         BEM_CUDA(cudaMemcpyAsync(d_off.p, off.data(), sizeof(int64_t) * off.size(), cudaMemcpyHostToDevice, c.stream));
-        hm_recompress_kernel<<<(unsigned)adm_list.size(), LEAF_THREADS, 0, c.stream>>>(
-            dl, d_adm.as<int32_t>(), H->d_store.as<double2>(), d_scr2.as<double2>(), d_off.as<int64_t>(),
-            p.in.hm_aca_tol);
-        BEM_CHECK_LAUNCH(&c);
+        // the largest leaves apart (RC_ALONE)
+        int sms = 0;
+        BEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
+        double total = 0;
+        for (int32_t l : adm_list) total += work(l);
+        size_t alone = 0;
+        while (alone < adm_list.size() && alone < (size_t)sms / 2 && work(adm_list[alone]) > RC_ALONE * total / sms) ++alone;
+        auto recompress = [&](size_t first, size_t last, size_t smem, cudaStream_t stream) {
+            if (first == last) return;
+            hm_recompress_kernel<<<(unsigned)(last - first), RC_THREADS, smem, stream>>>(
+                dl, d_adm.as<int32_t>() + first, H->d_store.as<double2>(), d_scr2.as<double2>(),
+                d_off.as<int64_t>() + first, p.in.hm_aca_tol);
+            BEM_CHECK_LAUNCH(&c);
+        };
+        if (alone) {
+            BEM_CUDA(cudaFuncSetAttribute(hm_recompress_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RC_ALONE_SMEM));
+            c.fork();
+            recompress(0, alone, RC_ALONE_SMEM, c.stream);  // (goes straight on: ahead of the others)
+            recompress(alone, adm_list.size(), 0, c.side);
+            c.join();
+        } else {
+            recompress(0, adm_list.size(), 0, c.stream);
+        }
         c.sync();
     }
     BEM_CUDA(cudaMemcpyAsync(H->leaves.data(), dl, sizeof(HLeaf) * nl, cudaMemcpyDeviceToHost, c.stream));

@@ -1191,11 +1191,7 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
     RowMoves* mv = reinterpret_cast<RowMoves*>(reinterpret_cast<char*>(cexp) + c_bytes);
     double2* pinv = reinterpret_cast<double2*>(reinterpret_cast<char*>(mv) + v_bytes);
     BEM_CUDA(cudaMemsetAsync(cexp, 0x80, c_bytes, ctx.stream));  // below every exponent
-    if (!ctx.lu64_side) {
-        BEM_CUDA(cudaEventCreateWithFlags(&ctx.lu64_ready, cudaEventDisableTiming));
-        BEM_CUDA(cudaEventCreateWithFlags(&ctx.lu64_done, cudaEventDisableTiming));
-        BEM_CUDA(cudaStreamCreateWithFlags(&ctx.lu64_side, cudaStreamNonBlocking));
-    }
+    ctx.need_side();
     std::function<void()> beside;  // the part of the last update that runs beside this block's panels
     for (int64_t b0 = 0; b0 < n; b0 += NB) {
         const int nb = (int)std::min<int64_t>(NB, n - b0);
@@ -1225,7 +1221,7 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
                 BEM_CHECK_LAUNCH(&ctx);
             }
         }
-        if (ahead) BEM_CUDA(cudaStreamWaitEvent(ctx.stream, ctx.lu64_done, 0));
+        if (ahead) ctx.join();
         const int64_t m = n - b0 - nb, rb = (m + 63) / 64, ct = (m + TN - 1) / TN;
         // columns per warp: a warp for every two columns while the SM quarters
         // (four per SM) outnumber the warps
@@ -1257,11 +1253,9 @@ void lu_factor_fp64(Context& ctx, int64_t n, double2* A, int64_t lda, void* aux,
         // other, update and solve included: n = 1000 4.8 ms, 2001 11.3, 4000 32.7,
         // 6144 73.7; this way 4.7, 10.4, 26.9, 57.9.)
         update(0, 1, nsm, ctx.stream);
-        BEM_CUDA(cudaEventRecord(ctx.lu64_ready, ctx.stream));
-        BEM_CUDA(cudaStreamWaitEvent(ctx.lu64_side, ctx.lu64_ready, 0));
+        ctx.fork();
         beside = [=, &ctx] {
-            update(1, ct, nsm - cs, ctx.lu64_side);
-            BEM_CUDA(cudaEventRecord(ctx.lu64_done, ctx.lu64_side));
+            update(1, ct, nsm - cs, ctx.side);
         };
     }
 }
