@@ -976,6 +976,7 @@ struct LuData {
         Kind kind;
         int ks, kw, woff, yoff, nchunks;
         Seg seg;
+        bool side;  // on the second stream, beside the step's DIAG
     };
     std::vector<Launch> plan;
     // preconditioner application: tickets, and a counter + row flags
@@ -1229,24 +1230,51 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
     // k .. k + j - 1 at once (K = 256 j); then its diagonal block and panels.
     // After the group, one K = 256 LU_GROUP update of the rest with every
     // step's panels side by side: A22 is read and written once per group.
-    auto plan = [&](LuData::Kind kind, int ks, int kw, int woff, int yoff, int nchunks,
-                    const std::vector<Entry>& e) {
-        LuData::Launch l{kind, ks, kw, woff, yoff, nchunks, add_segment(*d, e)};
+    //
+    // A step's diagonal blocks take one SM each for about 0.1 ms.  Where they are
+    // few, the update before them is cut: the tile that holds the diagonal block
+    // first, then DIAG and, beside it on the other SMs, the rest of the update.
+    // The column panel's embedding does not need the diagonal block either.  (Two
+    // operators of n = 40960, 320 steps, 33 ms of DIAG with 150 SMs idle: whole
+    // solve 540 -> 522 ms; 96 operators of up to 5000, the embedding alone beside
+    // DIAG: 51.7 -> 49.3 ms.)
+    int nsm = 0;
+    BEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    int64_t nfact = 0;
+    for (int s = 0; s < nsys; ++s) nfact += owner[(size_t)s] == s;
+    const bool cut = nfact <= nsm / 8;
+    auto plan = [&](LuData::Kind kind, int ks, int kw, int woff, int yoff, int nchunks, const std::vector<Entry>& e,
+                    bool side = false) {
+        LuData::Launch l{kind, ks, kw, woff, yoff, nchunks, add_segment(*d, e), side};
         if (l.seg.ctas) d->plan.push_back(l);
     };
     for (int k = 0; k < d->nblk_max; k += G) {
         const int64_t ktw = (int64_t)(k + 1) * LB;  // trailing origin of the group: W row 0
         for (int j = 0; j < G; ++j) {
             const int st = k + j;
-            std::vector<Entry> thin, diag, expd, l21, u12, copy;
+            // the update before this step: within the group, or the last group's
+            // of everything right of and below it
+            const int kg = j > 0 ? k : k - G, jg = j > 0 ? j : G;
+            std::vector<Entry> head, rest, diag, expd, l21, u12, copy;
             for (int s = 0; s < nsys; ++s) {
                 const LuSys& L = d->sys[(size_t)s];
                 if (L.nblk <= st || owner[(size_t)s] != s) continue;  // factored once per operator
                 const int64_t kts = (int64_t)(st + 1) * LB, mts = L.n - kts, mtw = L.n - ktw;
-                if (j > 0) {
-                    const int64_t c0 = (int64_t)st * LB;
-                    thin.push_back(trail_entry(s, 2 * (j - 1) * LB, 2 * mtw, c0, std::min<int64_t>(c0 + LB, L.n)));
-                    thin.push_back(trail_entry(s, 2 * (j - 1) * LB, 2 * j * LB, c0 + LB, L.n));
+                if (st > 0) {
+                    const int64_t c0 = (int64_t)st * LB, r0 = 2 * (jg - 1) * LB, r1 = 2 * (L.n - (int64_t)(kg + 1) * LB);
+                    // (a whole tile of columns where the update reaches that far)
+                    const int64_t rd = std::min<int64_t>(r0 + 2 * LB, r1),
+                                  c1 = std::min<int64_t>(c0 + (j > 0 ? LB : GN), L.n);
+                    if (cut) {
+                        head.push_back(trail_entry(s, r0, rd, c0, c1));
+                        rest.push_back(trail_entry(s, rd, r1, c0, c1));
+                        rest.push_back(trail_entry(s, r0, j > 0 ? rd : r1, c1, L.n));
+                    } else if (j > 0) {
+                        head.push_back(trail_entry(s, r0, r1, c0, c1));
+                        head.push_back(trail_entry(s, r0, rd, c1, L.n));
+                    } else {
+                        head.push_back(trail_entry(s, r0, r1, c0, L.n));
+                    }
                 }
                 diag.push_back(Entry{s, 1, 0, 0, 0, 0, 0});
                 if (mts <= 0) continue;  // the system's last block
@@ -1255,21 +1283,15 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
                 u12.push_back(Entry{s, 2 * ((mts + GN - 1) / GN), 0, 0, 0, kts, L.n});
                 copy.push_back(Entry{s, (mts + 31) / 32, 0, 0, 0, 0, 0});
             }
-            plan(LuData::TRAIL, st, k, 0, 0, GCHUNKS16 * j, thin);
+            const int ks = j > 0 ? st : kg + G - 1;
+            plan(LuData::TRAIL, ks, kg, 0, 0, GCHUNKS16 * jg, head);
             plan(LuData::DIAG, st, k, 0, 0, 0, diag);
-            plan(LuData::EXPAND, st, k, 2 * LB * j, 0, 0, expd);
+            plan(LuData::TRAIL, ks, kg, 0, 0, GCHUNKS16 * jg, rest, true);
+            plan(LuData::EXPAND, st, k, 2 * LB * j, 0, 0, expd, true);
             plan(LuData::L21, st, k, 2 * LB * j, 0, GCHUNKS, l21);
             plan(LuData::U12, st, k, 0, 2 * LB * j, GCHUNKS, u12);
             plan(LuData::COPY, st, k, 0, 2 * LB * j, 0, copy);
         }
-        std::vector<Entry> rest;
-        for (int s = 0; s < nsys; ++s) {
-            const LuSys& L = d->sys[(size_t)s];
-            const int64_t c0 = (int64_t)(k + G) * LB;
-            if (owner[(size_t)s] != s || c0 >= L.n) continue;
-            rest.push_back(trail_entry(s, 2 * (G - 1) * LB, 2 * (L.n - ktw), c0, L.n));
-        }
-        plan(LuData::TRAIL, k + G - 1, k, 0, 0, GCHUNKS16 * G, rest);
     }
     // substitution tickets: forward rows by ascending block, then backward
     // rows by descending block, the groups interleaved.  A group is up to
@@ -1327,8 +1349,6 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
     BEM_CUDA(cudaFuncSetAttribute(lu_gemm_kernel<G_L21>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
     const LuSys* sys = d->sysbuf.as<LuSys>();
     const LuWork* wk = d->work.as<LuWork>();
-    int nsm = 0;
-    BEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));  // persistent grids
     // with profiling: CUDA events around every launch, summed per kind
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float tsum[6] = {0, 0, 0, 0, 0, 0};  // per launch kind
@@ -1336,43 +1356,49 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
         BEM_CUDA(cudaEventCreate(&ev0));
         BEM_CUDA(cudaEventCreate(&ev1));
     }
-    auto persistent = [&](int64_t ctas) { return (unsigned)std::min<int64_t>(ctas, nsm); };
+    // persistent grids; on the second stream they leave the diagonal blocks' SMs
+    auto persistent = [&](int64_t ctas, bool side) {
+        return (unsigned)std::min<int64_t>(ctas, side ? nsm - nfact : nsm);
+    };
     // tile raster of the trailing updates (super-blocks of sb_r x sb_c tiles)
     // (keyed by the largest operator and the number of factored operators)
-    int64_t nfact = 0, nmax = 0;
-    for (int s = 0; s < nsys; ++s) {
-        nfact += owner[(size_t)s] == s;
-        nmax = std::max(nmax, d->sys[(size_t)s].n);
-    }
+    int64_t nmax = 0;
+    for (int s = 0; s < nsys; ++s) nmax = std::max(nmax, d->sys[(size_t)s].n);
     const int sb_r = std::max(1, std::min(65535, c.tuning.pick("lu_gemm_trail", "sb_r", nmax, nfact, 8)));
     const int sb_c = std::max(1, std::min(65535, c.tuning.pick("lu_gemm_trail", "sb_c", nmax, nfact, 32)));
     const int raster = (sb_r << 16) | sb_c;
+    bool open = false;  // work on the second stream
     for (const LuData::Launch& l : d->plan) {
         const LuData::Seg& sg = l.seg;
+        const bool side = l.side && open;
+        if (open && !side) c.join();
+        open = side || (l.kind == LuData::DIAG && !c.profiling);
+        if (open && !side) c.fork();  // before DIAG, which goes straight on
+        const cudaStream_t stream = side ? c.side : c.stream;
         if (c.profiling) BEM_CUDA(cudaEventRecord(ev0, c.stream));
         switch (l.kind) {
             case LuData::DIAG:
-                lu_diag_kernel<<<(unsigned)sg.ctas, DIAG_THREADS, diag_smem, c.stream>>>(sys, wk + sg.off, l.ks,
+                lu_diag_kernel<<<(unsigned)sg.ctas, DIAG_THREADS, diag_smem, stream>>>(sys, wk + sg.off, l.ks,
                                                                                  d->info.as<int>());
                 break;
             case LuData::EXPAND:
-                lu_expand_kernel<<<(unsigned)sg.ctas, 256, expand_smem, c.stream>>>(sys, wk + sg.off, sg.count, l.ks,
+                lu_expand_kernel<<<(unsigned)sg.ctas, 256, expand_smem, stream>>>(sys, wk + sg.off, sg.count, l.ks,
                                                                                     l.kw);
                 break;
             case LuData::L21:
-                lu_gemm_kernel<G_L21><<<persistent(sg.ctas), GTHREADS, G_SMEM, c.stream>>>(
+                lu_gemm_kernel<G_L21><<<persistent(sg.ctas, side), GTHREADS, G_SMEM, stream>>>(
                     sys, wk + sg.off, sg.count, l.ks, l.kw, l.nchunks, l.woff, l.yoff, sg.ctas, raster, err);
                 break;
             case LuData::U12:
-                lu_gemm_kernel<G_U12><<<persistent(sg.ctas), GTHREADS, G_SMEM, c.stream>>>(
+                lu_gemm_kernel<G_U12><<<persistent(sg.ctas, side), GTHREADS, G_SMEM, stream>>>(
                     sys, wk + sg.off, sg.count, l.ks, l.kw, l.nchunks, l.woff, l.yoff, sg.ctas, raster, err);
                 break;
             case LuData::COPY:
-                lu_copy_u12_kernel<<<(unsigned)sg.ctas, 256, 0, c.stream>>>(sys, wk + sg.off, sg.count, l.ks,
+                lu_copy_u12_kernel<<<(unsigned)sg.ctas, 256, 0, stream>>>(sys, wk + sg.off, sg.count, l.ks,
                                                                             l.yoff);
                 break;
             case LuData::TRAIL:
-                lu_gemm_kernel<G_TRAIL><<<persistent(sg.ctas), GTHREADS, G_SMEM, c.stream>>>(
+                lu_gemm_kernel<G_TRAIL><<<persistent(sg.ctas, side), GTHREADS, G_SMEM, stream>>>(
                     sys, wk + sg.off, sg.count, l.ks, l.kw, l.nchunks, l.woff, l.yoff, sg.ctas, raster, err);
                 break;
         }
@@ -1385,6 +1411,7 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
             tsum[(int)l.kind] += ms;
         }
     }
+    if (open) c.join();
     if (c.profiling) {
         // algorithmic work: 8 n^3 / 3 complex flop per factored operator
         double fl = 0;
