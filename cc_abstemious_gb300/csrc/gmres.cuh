@@ -23,6 +23,7 @@ struct GmSys {
     int64_t tile0;  // first CTA of this system in the flattened mat-vec grid
     int rb, cb;     // row blocks, column chunks
     int64_t tile64; // first CTA of this system in the flattened grid of 64-row blocks
+    int mate;       // another system with the same operator (-1: none), to share its reads
 };
 
 struct GmBatch {
@@ -51,6 +52,7 @@ struct GmBatch {
     int gs_chunks = 0;
     int gs_rows = 0;     // rows per chunk
     int tpr = 1;         // tickets per row block
+    int mates = 0;       // ragged: some systems have mates
     int64_t ntiles64 = 0;  // ragged: CTAs of the flattened grid of 64-row blocks
     // split FP64 operators (refined form): every system's FP32 matrix (the
     // operator rounded to FP32, leading dimension lda) is followed, split_lo

@@ -46,3 +46,24 @@ def test_mixed_sizes(n, precond, form):
     for rep in a.reports:
         assert rep["flag"] == 1
         assert 0 <= rep["rel_err_vs_lu"] < 1e-6, rep
+
+
+@pytest.mark.parametrize("waves", [2, 3])
+@pytest.mark.parametrize("n", [2570, 3100])
+def test_waves_share_an_operator(n, waves):
+    """Sizes and counts at which the mixed form's products take the wide tiles, two
+    right-hand sides per pass and, with three, one left over (8 or 12 systems of 36
+    or 49 tiles): every wave to the form's accuracy, and converged by itself."""
+    inp = workloads.perturbed_sphere_input(tempfile.mkdtemp(prefix="bem_waves_"), n, n, [1.0, 2.0, 3.0, 4.0], tol=1e-8)
+    inp["incident_wave"] = {"PlaneWave": {"direction": [0.0, 0.0, 1.0], "amplitude": [1.0, 0.0]}}
+    inp["additional_incident_waves"] = [
+        {"SphericalWave": {"origin": [0.0, 0.0, 3.0], "amplitude": [0.5, 0.2]}},
+        {"PlaneWave": {"direction": [1.0, 1.0, 0.0], "amplitude": [0.0, 1.0]}}][:waves - 1]
+    a = bem.Analysis(bem.Context.default())
+    a.set_input(inp)
+    a.run(form="mixed", check_vs_lu=True)
+    reports = [rep for r in a.reports_by_rhs for rep in r]
+    assert len(reports) == 4 * waves
+    for rep in reports:
+        assert rep["flag"] == 1
+        assert 0 <= rep["rel_err_vs_lu"] < 1e-6, rep
