@@ -179,11 +179,11 @@ struct Asm32Smem {
 // One 64 x 64 tile (row tile ti, column tile tj) of every system of a body;
 // the squared Frobenius norm partial of system s goes to
 // norm_part[s * norm_stride + tile_index].
-template <int WITH_RHS>
+template <int WITH_RHS, bool TWIN>
 __device__ __forceinline__ void assemble32_tile(int64_t n, int64_t npad, const float* __restrict__ g32,
                                                 const double* __restrict__ geo, const Asm32Params& prm,
-                                                float2* __restrict__ A, int64_t ld, size_t mat_stride,
-                                                double2* __restrict__ part, size_t part_stride,
+                                                float2* __restrict__ A, float2* __restrict__ twin, int64_t ld,
+                                                size_t mat_stride, double2* __restrict__ part, size_t part_stride,
                                                 double* __restrict__ norm_part, size_t norm_stride,
                                                 size_t tile_index, int ti, int tj, int* __restrict__ err,
                                                 Asm32Smem& sm) {
@@ -243,6 +243,7 @@ __device__ __forceinline__ void assemble32_tile(int64_t n, int64_t npad, const f
                 cfma(a, be, g);
                 float2 af = make_float2((float)a.x, (float)a.y);
                 A[s * mat_stride + j * ld + i] = af;
+                if (TWIN && twin) twin[s * mat_stride + j * ld + i] = af;
                 nrm[s] += af.x * af.x + af.y * af.y;
                 if (WITH_RHS) {
                     z2 ga = make_double2(prm.s[s].gamma.x, prm.s[s].gamma.y);
@@ -289,6 +290,7 @@ __device__ __forceinline__ void assemble32_tile(int64_t n, int64_t npad, const f
                     af = make_float2(af.x + b2.x, af.y + b2.y);
                 }
                 A[s * mat_stride + j * ld + i] = af;
+                if (TWIN && twin) twin[s * mat_stride + j * ld + i] = af;
                 nrm[s] += af.x * af.x + af.y * af.y;
                 if (WITH_RHS) {
                     float2 r1 = fmul(S.gamma, h), r2 = fmul(S.delta, g);
@@ -335,13 +337,16 @@ __device__ __forceinline__ void assemble32_tile(int64_t n, int64_t npad, const f
 
 // MINB: CTAs per SM the register allocation must allow (tuned per size:
 // more CTAs hide latency, fewer registers per thread cost spills and ILP).
-template <int WITH_RHS, int MINB = 3>
+// TWIN: with a second copy, for the LU's working copy (a copy of its own took 2.5
+// of 49 ms for 96 operators of up to 5000; the branch on its pointer would cost
+// assemblies without one 6 %).
+template <int WITH_RHS, int MINB = 3, bool TWIN = false>
 __global__ void __launch_bounds__(ASM_THREADS, MINB) assemble32_kernel(
     int64_t n, int64_t npad, const float* __restrict__ g32, const double* __restrict__ geo, Asm32Params prm,
-    float2* __restrict__ A, int64_t ld, size_t mat_stride, double2* __restrict__ part, size_t part_stride,
-    double* __restrict__ norm_part, int* __restrict__ err) {
+    float2* __restrict__ A, float2* __restrict__ twin, int64_t ld, size_t mat_stride, double2* __restrict__ part,
+    size_t part_stride, double* __restrict__ norm_part, int* __restrict__ err) {
     __shared__ __align__(128) Asm32Smem sm;
-    assemble32_tile<WITH_RHS>(n, npad, g32, geo, prm, A, ld, mat_stride, part, part_stride, norm_part,
+    assemble32_tile<WITH_RHS, TWIN>(n, npad, g32, geo, prm, A, twin, ld, mat_stride, part, part_stride, norm_part,
                               (size_t)gridDim.x * gridDim.y, (size_t)blockIdx.y * gridDim.x + blockIdx.x,
                               (int)blockIdx.y, (int)blockIdx.x, err, sm);
 }
@@ -354,6 +359,7 @@ struct Body32 {
     const float* g32;
     const double* geo;
     float2* A;          // system s of the body at A + s * mat_stride
+    float2* twin;       // a second copy of the same layout (nullptr: none)
     int64_t ld;
     size_t mat_stride;
     double* norm_part;  // nsys x ntiles^2 partials
@@ -361,6 +367,7 @@ struct Body32 {
     int ntiles, pad;
 };
 
+template <bool TWIN>
 __global__ void __launch_bounds__(ASM_THREADS, 3) assemble32_multi_kernel(const Body32* __restrict__ bodies,
                                                                       int nbodies,
                                                                       const Asm32Params* __restrict__ prms,
@@ -383,7 +390,7 @@ __global__ void __launch_bounds__(ASM_THREADS, 3) assemble32_multi_kernel(const 
     __syncthreads();
     const int64_t local = t - B.tile0;
     const int ti = (int)(local / B.ntiles), tj = (int)(local % B.ntiles);
-    assemble32_tile<0>(B.n, B.npad, B.g32, B.geo, prm, B.A, B.ld, B.mat_stride, nullptr, 0, B.norm_part,
+    assemble32_tile<0, TWIN>(B.n, B.npad, B.g32, B.geo, prm, B.A, B.twin, B.ld, B.mat_stride, nullptr, 0, B.norm_part,
                        (size_t)B.ntiles * B.ntiles, (size_t)local, ti, tj, err, sm);
 }
 
@@ -439,7 +446,8 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(ASM_THREADS, 2) assemble_ff_kernel(int64_t n, int64_t npad,
                                                                     const float* __restrict__ g32,
                                                                     const double* __restrict__ geo, AsmFFParams prm,
-                                                                    float2* __restrict__ A, int64_t ld, size_t stride,
+                                                                    float2* __restrict__ A, float2* __restrict__ twin,
+                                                                    int64_t ld, size_t stride,
                                                                     size_t plane, double* __restrict__ norm_part,
                                                                     int* __restrict__ err) {
     __shared__ __align__(128) Asm32Smem sm;
@@ -489,6 +497,7 @@ __global__ void __launch_bounds__(ASM_THREADS, 2) assemble_ff_kernel(int64_t n, 
                 cfma(a, prm.s[s].beta_d, g);
                 const float hx = __double2float_rn(a.x), hy = __double2float_rn(a.y);
                 A[s * stride + o] = make_float2(hx, hy);
+                if (!SPLIT && twin) twin[s * stride + o] = make_float2(hx, hy);
                 if (SPLIT)
                     A[s * stride + o + plane] =
                         make_float2(__double2float_rn(a.x - (double)hx), __double2float_rn(a.y - (double)hy));
@@ -536,6 +545,7 @@ __global__ void __launch_bounds__(ASM_THREADS, 2) assemble_ff_kernel(int64_t n, 
             cff a = S.alpha_one ? h : S.alpha * h;
             if (!S.beta_zero) a = a + S.beta * g;
             A[s * stride + o] = make_float2(a.re.h, a.im.h);
+            if (!SPLIT && twin) twin[s * stride + o] = make_float2(a.re.h, a.im.h);
             if (SPLIT) A[s * stride + o + plane] = make_float2(a.re.l, a.im.l);
             nrm[s] += a.re.h * a.re.h + a.im.h * a.im.h;
         }
@@ -562,8 +572,9 @@ static ff host_ff(double v) {
 }
 
 void assemble_system_split(Context& ctx, const Problem& p, const double* ks, const cd* alphas, const cd* betas,
-                           int nsys, float2* A, int64_t ld, size_t plane, double* norms, bool remainder) {
+                           int nsys, float2* A, int64_t ld, size_t plane, double* norms, bool remainder, float2* twin) {
     require(plane == (size_t)ld * p.n, "split assembly: planes must be ld * n entries");
+    require(!twin || !remainder, "split assembly: a second copy of the rounded form only");
     int* err = device_err(ctx);
     BEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx.stream));
     const int ntiles = (int)(p.geo.npad / TILE);
@@ -608,11 +619,13 @@ void assemble_system_split(Context& ctx, const Problem& p, const double* ks, con
         const size_t stride = remainder ? 2 * plane : plane;
         if (remainder)
             assemble_ff_kernel<true><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-                p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, A + (size_t)s0 * stride, ld, stride, plane,
+                p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, A + (size_t)s0 * stride,
+                twin ? twin + (size_t)s0 * stride : nullptr, ld, stride, plane,
                 ctx.w_norm.as<double>(), err);
         else
             assemble_ff_kernel<false><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-                p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, A + (size_t)s0 * stride, ld, stride, plane,
+                p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, A + (size_t)s0 * stride,
+                twin ? twin + (size_t)s0 * stride : nullptr, ld, stride, plane,
                 ctx.w_norm.as<double>(), err);
         BEM_CHECK_LAUNCH(&ctx);
         finish_norms(ctx, ctx.w_norm.as<double>(), nparts, prm.nsys, norms + s0);
@@ -622,7 +635,7 @@ void assemble_system_split(Context& ctx, const Problem& p, const double* ks, con
 
 void assemble_system_fp32_body(Context& ctx, const Problem& p, const double* ks, const cd* alphas, const cd* betas,
                                const cd* gammas, const cd* deltas, int nsys, float2* A, int64_t ld, size_t mat_stride,
-                               double2* rowsum, size_t vec_stride, double* norms) {
+                               double2* rowsum, size_t vec_stride, double* norms, float2* twin) {
     int* err = device_err(ctx);
     BEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx.stream));
     const float P1 = 1.5703125f;  // 201/128: n * P1 exact for n < 2^16
@@ -651,13 +664,15 @@ void assemble_system_fp32_body(Context& ctx, const Problem& p, const double* ks,
         }
         dim3 grid((unsigned)ntiles, (unsigned)ntiles);
         float2* As = A + (size_t)s0 * mat_stride;
+        float2* Ts = twin ? twin + (size_t)s0 * mat_stride : nullptr;
         double* np_ = nbuf.as<double>();
         if (rowsum) {
             size_t pstride = (size_t)ntiles * p.geo.npad;
             ctx.w_part.ensure(sizeof(double2) * pstride * prm.nsys);
             double2* part = ctx.w_part.as<double2>();
-            assemble32_kernel<1><<<grid, ASM_THREADS, 0, ctx.stream>>>(p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0),
-                                                                       prm, As, ld, mat_stride, part, pstride, np_,
+            auto kernel = Ts ? assemble32_kernel<1, 3, true> : assemble32_kernel<1>;
+            kernel<<<grid, ASM_THREADS, 0, ctx.stream>>>(p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0),
+                                                                       prm, As, Ts, ld, mat_stride, part, pstride, np_,
                                                                        err);
             BEM_CHECK_LAUNCH(&ctx);
             for (int s = 0; s < prm.nsys; ++s)
@@ -665,15 +680,22 @@ void assemble_system_fp32_body(Context& ctx, const Problem& p, const double* ks,
                                     rowsum + (size_t)(s0 + s) * vec_stride);
         } else {
             const int minb = ctx.tuning.pick("assemble32", "min_ctas", p.n, nsys, 3);
-            if (minb == 2)
+            if (Ts)
+                assemble32_kernel<0, 3, true><<<grid, ASM_THREADS, 0, ctx.stream>>>(
+                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, Ts, ld, mat_stride, nullptr, 0, np_,
+                    err);
+            else if (minb == 2)
                 assemble32_kernel<0, 2><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, ld, mat_stride, nullptr, 0, np_, err);
+                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, Ts, ld, mat_stride, nullptr, 0, np_,
+                    err);
             else if (minb == 4)
                 assemble32_kernel<0, 4><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, ld, mat_stride, nullptr, 0, np_, err);
+                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, Ts, ld, mat_stride, nullptr, 0, np_,
+                    err);
             else
                 assemble32_kernel<0, 3><<<grid, ASM_THREADS, 0, ctx.stream>>>(
-                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, ld, mat_stride, nullptr, 0, np_, err);
+                    p.n, p.geo.npad, p.geo.arr32(0), p.geo.arr(0), prm, As, Ts, ld, mat_stride, nullptr, 0, np_,
+                    err);
             BEM_CHECK_LAUNCH(&ctx);
         }
         if (norms) {
@@ -739,6 +761,7 @@ void assemble_fp32_multi(Context& ctx, const std::vector<BodyAsm32>& bodies, dou
             e.g32 = p.geo.arr32(0);
             e.geo = p.geo.arr(0);
             e.A = b.A + (size_t)s0 * b.mat_stride;
+            e.twin = b.twin ? b.twin + (size_t)s0 * b.mat_stride : nullptr;
             e.ld = b.ld;
             e.mat_stride = b.mat_stride;
             e.norm_part = reinterpret_cast<double*>(parts);  // offset for now
@@ -773,7 +796,9 @@ void assemble_fp32_multi(Context& ctx, const std::vector<BodyAsm32>& bodies, dou
     int* err = device_err(ctx);
     BEM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx.stream));
     require(tiles < (int64_t)INT32_MAX, "multi-body assembly: too many tiles");
-    assemble32_multi_kernel<<<(unsigned)tiles, ASM_THREADS, 0, ctx.stream>>>(
+    // (all bodies of a batch have a second copy or none has)
+    auto multi = ent[0].twin ? assemble32_multi_kernel<true> : assemble32_multi_kernel<false>;
+    multi<<<(unsigned)tiles, ASM_THREADS, 0, ctx.stream>>>(
         reinterpret_cast<const Body32*>(mb), (int)nent, reinterpret_cast<const Asm32Params*>(mb + o_prm), err);
     BEM_CHECK_LAUNCH(&ctx);
     if (norms) {

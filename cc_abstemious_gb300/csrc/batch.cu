@@ -117,7 +117,14 @@ void solve_chunk(Context& c, std::vector<BodyPlan*>& bodies, bem_precond precond
     const size_t nsys = ns.size();
     c.w_mat.ensure(sizeof(float2) * ent);
     float2* A = c.w_mat.as<float2>();
+    // the LU preconditioner's working copy is written by the assembly
+    float2* twin = nullptr;
+    if (precond == BEM_PRECOND_LU) {
+        c.w_lu_F.ensure(sizeof(float2) * ent);
+        twin = c.w_lu_F.as<float2>();
+    }
     GmWorkspace ws;
+    ws.factors_seeded = twin != nullptr;
     ws.mem_pool = &c.w_gm;
     ws.z_pool = &c.w_gmz;
     gm_prepare_ragged(c, ws, ns, lds, aoff, mmax, A, true);
@@ -149,10 +156,10 @@ void solve_chunk(Context& c, std::vector<BodyPlan*>& bodies, bem_precond precond
             if (B.need_rowsum) {
                 assemble_system_fp32_body(c, *B.p, B.ks.data(), B.al.data(), B.be.data(), B.ga.data(), B.de.data(),
                                           B.nf, A + aoff[s0], B.ld, (size_t)B.ld * B.n, rowsum + L[s0].v_off,
-                                          (size_t)B.n, ws.anorm + s0);
+                                          (size_t)B.n, ws.anorm + s0, twin ? twin + aoff[s0] : nullptr);
             } else {
                 multi.push_back(BodyAsm32{B.p, B.nf, B.ks.data(), B.al.data(), B.be.data(), A + aoff[s0], B.ld,
-                                          (size_t)B.ld * B.n});
+                                          (size_t)B.ld * B.n, twin ? twin + aoff[s0] : nullptr});
                 multi_sys0.push_back(s0);
             }
         }

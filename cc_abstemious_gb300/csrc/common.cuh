@@ -290,12 +290,16 @@ void assemble_system_fp64(Context& ctx, const Problem& p, double2* A, int64_t ld
 // e^{ik r} by recurrence for evenly spaced wavenumbers; systems 2 * plane
 // float2 apart; norms[s] = ||A_s||_F.  remainder false: the FP32 roundings
 // alone (the operator rounded once from its float-float value), systems
-// `plane` float2 apart.
+// `plane` float2 apart.  twin: a second copy of the same layout, written beside
+// the first (also below); the assembly is bound by arithmetic, a copy of the
+// operators afterwards by memory.
 void assemble_system_split(Context& ctx, const Problem& p, const double* ks, const cd* alphas, const cd* betas,
-                           int nsys, float2* A, int64_t ld, size_t plane, double* norms, bool remainder = true);
+                           int nsys, float2* A, int64_t ld, size_t plane, double* norms, bool remainder = true,
+                           float2* twin = nullptr);
 void assemble_system_fp32_body(Context& ctx, const Problem& p, const double* ks, const cd* alphas,
                                const cd* betas, const cd* gammas, const cd* deltas, int nsys, float2* A,
-                               int64_t ld, size_t mat_stride, double2* rowsum, size_t vec_stride, double* norms);
+                               int64_t ld, size_t mat_stride, double2* rowsum, size_t vec_stride, double* norms,
+                               float2* twin = nullptr);
 // Several bodies, each with nsys frequencies (LHS operator only), in one
 // launch; norms[g] = ||A_g||_F for the systems in body-major order.
 struct BodyAsm32 {
@@ -306,6 +310,7 @@ struct BodyAsm32 {
     float2* A;  // system s at A + s * mat_stride
     int64_t ld;
     size_t mat_stride;
+    float2* twin;  // second copy, of the same layout (nullptr: none)
 };
 void assemble_fp32_multi(Context& ctx, const std::vector<BodyAsm32>& bodies, double* norms);
 void evaluate_field32_batch(Context& ctx, const Problem& p, const double* ks, int nsys, const double2* phi,

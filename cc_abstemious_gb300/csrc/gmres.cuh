@@ -148,6 +148,7 @@ struct GmWorkspace {
     // dense operator's n^2 entries)
     double mv_bytes = 0;
     const char* mv_stage = nullptr;
+    bool factors_seeded = false;  // the LU's buffer holds a copy of the operators already
     DevBuf rounds;  // finished rounds of gm_run
 };
 

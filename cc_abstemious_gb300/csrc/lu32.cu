@@ -1107,6 +1107,7 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
     }
     // the factors, block inverses and panel workspace live in grow-only
     // buffers of the context
+    require(!ws.factors_seeded || c.w_lu_F.bytes >= sizeof(float2) * entries, "LU: working copy too small", BEM_ERR_CUDA);
     c.w_lu_F.ensure(sizeof(float2) * entries);
     c.w_lu_D.ensure(sizeof(float2) * std::max<size_t>(dm, 1));
     c.w_lu_W.ensure(sizeof(float) * std::max<size_t>(wsz, 4));
@@ -1117,7 +1118,9 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
     std::vector<double> anorm((size_t)nsys);
     BEM_CUDA(cudaMemcpyAsync(anorm.data(), ws.anorm, sizeof(double) * nsys, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
-    if (ws.bt.split_lo) {
+    if (ws.factors_seeded) {
+        // the assembly has left a copy there
+    } else if (ws.bt.split_lo) {
         // one copy per distinct operator (several right-hand sides share one)
         for (int s = 0; s < nsys; ++s) {
             bool first = true;
@@ -1248,6 +1251,9 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
         LuData::Launch l{kind, ks, kw, woff, yoff, nchunks, add_segment(*d, e), side};
         if (l.seg.ctas) d->plan.push_back(l);
     };
+    // U12's copy into the factors waits for the next step's DIAG as well
+    std::vector<Entry> late;
+    int late_ks = 0, late_kg = 0, late_y = 0;
     for (int k = 0; k < d->nblk_max; k += G) {
         const int64_t ktw = (int64_t)(k + 1) * LB;  // trailing origin of the group: W row 0
         for (int j = 0; j < G; ++j) {
@@ -1288,11 +1294,16 @@ void lu_precond_setup(Context& c, GmWorkspace& ws) {
             plan(LuData::DIAG, st, k, 0, 0, 0, diag);
             plan(LuData::TRAIL, ks, kg, 0, 0, GCHUNKS16 * jg, rest, true);
             plan(LuData::EXPAND, st, k, 2 * LB * j, 0, 0, expd, true);
+            plan(LuData::COPY, late_ks, late_kg, 0, late_y, 0, late, true);
             plan(LuData::L21, st, k, 2 * LB * j, 0, GCHUNKS, l21);
             plan(LuData::U12, st, k, 0, 2 * LB * j, GCHUNKS, u12);
-            plan(LuData::COPY, st, k, 0, 2 * LB * j, 0, copy);
+            late = copy;
+            late_ks = st;
+            late_kg = k;
+            late_y = 2 * LB * j;
         }
     }
+    plan(LuData::COPY, late_ks, late_kg, 0, late_y, 0, late);
     // substitution tickets: forward rows by ascending block, then backward
     // rows by descending block, the groups interleaved.  A group is up to
     // TS_MAXR consecutive systems sharing one operator (several right-hand

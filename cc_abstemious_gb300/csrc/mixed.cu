@@ -166,6 +166,14 @@ static void run_mixed_range(Context& c, Problem& p, int64_t F0, int64_t nf, bem_
         ws.mv_bytes = 16.0 * (double)n * (double)n;
     }
 
+    // the LU preconditioner's working copy, written by the assembly
+    auto twin = [&]() -> float2* {
+        if (precond != BEM_PRECOND_LU) return nullptr;
+        c.w_lu_F.ensure(sizeof(float2) * mstride * nf);
+        ws.factors_seeded = true;
+        return c.w_lu_F.as<float2>();
+    };
+
     if (hier) {
         EventTimer t(c);
         Hm = hmixed_build(c, p, F0, nf, (int)R);
@@ -204,7 +212,7 @@ static void run_mixed_range(Context& c, Problem& p, int64_t F0, int64_t nf, bem_
         // refined form's assembly without the remainder plane)
         EventTimer t(c);
         assemble_system_split(c, p, ks.data(), al.data(), be.data(), (int)nf, A32, ld, mstride,
-                              R == 1 ? ws.anorm : normf, false);
+                              R == 1 ? ws.anorm : normf, false, twin());
         if (R > 1) {
             repeat_norms_kernel<<<(unsigned)((ns + 127) / 128), 128, 0, c.stream>>>(normf, (int)R, (int)ns, ws.anorm);
             BEM_CHECK_LAUNCH(&c);
@@ -214,7 +222,7 @@ static void run_mixed_range(Context& c, Problem& p, int64_t F0, int64_t nf, bem_
         // the assembly kernel also writes ||A_f||_F for the stopping test
         EventTimer t(c);
         assemble_system_fp32_body(c, p, ks.data(), al.data(), be.data(), ga.data(), de.data(), (int)nf, A32, ld,
-                                  mstride, need_rowsum ? rowsum : nullptr, (size_t)n, R == 1 ? ws.anorm : normf);
+                                  mstride, need_rowsum ? rowsum : nullptr, (size_t)n, R == 1 ? ws.anorm : normf, twin());
         if (R > 1) {
             repeat_norms_kernel<<<(unsigned)((ns + 127) / 128), 128, 0, c.stream>>>(normf, (int)R, (int)ns, ws.anorm);
             BEM_CHECK_LAUNCH(&c);
