@@ -224,6 +224,8 @@ struct Context {
     // every mixed solve)
     DevBuf w_gm, w_gmz, w_lu_F, w_lu_D, w_lu_W, w_lu_P, w_lu_H;
     DevBuf w_upload;  // mesh staging of problem construction
+    DevBuf w_tree[18];  // the cluster and block tree builds' work arrays, an H-matrix build's lists
+    DevBuf w_rounds;    // finished rounds of the running GMRES solve
     DevBuf w_piv;     // the plain form's FP64 LU: row order, diagonal blocks' inverses
     DevBuf w_lu64;    // its trailing update's digit images
     int lu64_cluster = 0;  // largest cluster its panels run on (0: not asked yet)

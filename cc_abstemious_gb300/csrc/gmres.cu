@@ -1685,12 +1685,12 @@ void gm_run(Context& ctx, GmWorkspace& ws, int chunk, int64_t max_total_iteratio
     BEM_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), ctx.progress, 0));
     volatile int* seen = ctx.progress;
     *seen = 1;  // round 0, open (nothing of an earlier run is in flight)
-    ws.rounds.ensure(sizeof(int));
-    BEM_CUDA(cudaMemsetAsync(ws.rounds.p, 0, sizeof(int), ctx.stream));
+    ctx.w_rounds.ensure(sizeof(int));
+    BEM_CUDA(cudaMemsetAsync(ctx.w_rounds.p, 0, sizeof(int), ctx.stream));
     gm_launch_start(ctx, ws);
     auto launch_round = [&] {
         for (int c = 0; c < chunk; ++c) gm_launch_iteration(ctx, ws, nullptr, nullptr);
-        gm_progress_kernel<<<1, 128, 0, ctx.stream>>>(ws.bt.st, ws.bt.nsys, ws.rounds.as<int>(), dev);
+        gm_progress_kernel<<<1, 128, 0, ctx.stream>>>(ws.bt.st, ws.bt.nsys, ctx.w_rounds.as<int>(), dev);
         BEM_CHECK_LAUNCH(&ctx);
     };
     struct Graph {
@@ -1749,6 +1749,7 @@ GmresResult gmres_dense_fp64(Context& ctx, int64_t n, const double2* A, int64_t 
     int m = (int)std::ceil(std::sqrt((double)max_it));
     int64_t restarts = max_it / m;
     GmWorkspace ws;
+    ws.mem_pool = &ctx.w_gm;
     gm_prepare(ctx, ws, 1, n, m, A, lda, 0, false, true);
     BEM_CUDA(cudaMemcpyAsync(ws.bt.B, x, sizeof(double2) * n, cudaMemcpyDeviceToDevice, ctx.stream));
     gm_matrix_norms(ctx, ws);

@@ -149,7 +149,6 @@ struct GmWorkspace {
     double mv_bytes = 0;
     const char* mv_stage = nullptr;
     bool factors_seeded = false;  // the LU's buffer holds a copy of the operators already
-    DevBuf rounds;  // finished rounds of gm_run
 };
 
 void gm_prepare(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, int m, const void* A, int64_t lda,

@@ -1089,7 +1089,7 @@ std::unique_ptr<HMatrixDev> hmatrix_build(Context& c, const Problem& p, int side
         if (H->leaves[(size_t)b].adm) adm_list.push_back(b);
     for (size_t b = 0; b < nl; ++b)
         if (!H->leaves[b].adm) dense_list.push_back((int32_t)b);
-    DevBuf d_adm, d_dense;
+    DevBuf &d_adm = c.w_tree[16], &d_dense = c.w_tree[17];
     d_adm.ensure(sizeof(int32_t) * std::max<size_t>(adm_list.size(), 1));
     d_dense.ensure(sizeof(int32_t) * std::max<size_t>(dense_list.size(), 1));
     BEM_CUDA(cudaMemcpyAsync(d_adm.p, adm_list.data(), sizeof(int32_t) * adm_list.size(), cudaMemcpyHostToDevice,
@@ -1294,6 +1294,7 @@ GmresResult gmres_hmatrix(Context& c, const HMatrixDev& H, int64_t max_it, doubl
     int m = (int)std::ceil(std::sqrt((double)max_it));
     int64_t restarts = max_it / m;
     GmWorkspace ws;
+    ws.mem_pool = &c.w_gm;
     gm_prepare(c, ws, 1, n, m, nullptr, n, 0, false, true);
     ws.hook = hm_apply_hook;
     ws.hook_user = const_cast<HMatrixDev*>(&H);

@@ -438,7 +438,9 @@ void build_forest_dev(Context& c, Forest& F, const DevBuf& d_xyz) {
     const int nb = F.nbodies;
     const int64_t total = F.pt0[(size_t)nb];
     const int cap = (int)std::min<int64_t>(2 * total + 2 * nb + 2, INT32_MAX);
-    DevBuf d_nodes, d_scratch, d_front, d_next, d_split, d_cnt, d_pt0;
+    // (kept by the context: an allocation and its release take longer than a level)
+    DevBuf &d_nodes = c.w_tree[0], &d_scratch = c.w_tree[1], &d_front = c.w_tree[2], &d_next = c.w_tree[3],
+           &d_split = c.w_tree[4], &d_cnt = c.w_tree[5], &d_pt0 = c.w_tree[6];
     d_nodes.ensure(sizeof(TreeNode) * (size_t)cap);
     F.d_perm.ensure(sizeof(int64_t) * (size_t)std::max<int64_t>(total, 1));
     d_scratch.ensure(sizeof(int64_t) * (size_t)std::max<int64_t>(total, 1));
@@ -557,7 +559,7 @@ std::shared_ptr<Forest> build_forest(Context& c, int nb, const double* const* pt
     for (int b = 0; b < nb; ++b)
         for (int64_t i = 0; i < npts[b]; ++i)
             for (int d = 0; d < 3; ++d) h[(size_t)(3 * (F->pt0[(size_t)b] + i) + d)] = pts[b][stride * i + d];
-    DevBuf d_xyz;
+    DevBuf& d_xyz = c.w_tree[7];
     d_xyz.ensure(sizeof(double) * h.size());
     BEM_CUDA(cudaMemcpyAsync(d_xyz.p, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, c.stream));
     build_forest_dev(c, *F, d_xyz);
@@ -578,7 +580,7 @@ std::shared_ptr<Forest> build_forest(Context& c, const std::vector<const Problem
         F->pt0.push_back(F->pt0.back() + p.n);
     }
     const int64_t total = F->pt0.back();
-    DevBuf d_xyz, d_g;
+    DevBuf &d_xyz = c.w_tree[7], &d_g = c.w_tree[8];
     d_xyz.ensure(sizeof(double) * (size_t)(3 * std::max<int64_t>(total, 1)));
     d_g.ensure(sizeof(BodyGeo) * (size_t)nb);
     BEM_CUDA(cudaMemcpyAsync(d_g.p, g.data(), sizeof(BodyGeo) * nb, cudaMemcpyHostToDevice, c.stream));
@@ -594,7 +596,8 @@ std::shared_ptr<Forest> build_forest(Context& c, const std::vector<const Problem
 std::vector<BlockLeaf> forest_block_leaves(Context& c, const Forest& F, double eta) {
     TreeTimer timer(c, "block_tree");
     const int nb = F.nbodies;
-    DevBuf d_nodes, d_pr, d_kind, d_cb, d_cnt, d_off, d_ctr, d_out;
+    DevBuf &d_nodes = c.w_tree[0], &d_pr = c.w_tree[9], &d_kind = c.w_tree[10], &d_cb = c.w_tree[11],
+           &d_cnt = c.w_tree[12], &d_off = c.w_tree[13], &d_ctr = c.w_tree[14], &d_out = c.w_tree[15];
     // the block tree reads boxes, diameters and sons only
     d_nodes.ensure(sizeof(TreeNode) * F.nodes.size());
     BEM_CUDA(cudaMemcpyAsync(d_nodes.p, F.nodes.data(), sizeof(TreeNode) * F.nodes.size(), cudaMemcpyHostToDevice,
