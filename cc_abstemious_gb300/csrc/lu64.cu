@@ -10,8 +10,8 @@
 // columns, per block:
 //
 //   panel  a thread-block cluster holds the block's columns in its shared
-//          memory and factors them column by column; one hardware cluster
-//          barrier per column.  A tall block is cut into narrower panels that
+//          memory and factors them column by column; one exchange of stores
+//          counted on barriers per column.  A tall block is cut into narrower panels that
 //          fit, and the rest of the block's columns take a panel's update over
 //          the whole GPU (lu64_mid_kernel).
 //   rows   the columns right of the block take the block's row exchanges,
@@ -689,8 +689,8 @@ __global__ void __launch_bounds__(ROWS_THREADS) lu64_rows_kernel(
 // finish with one FP64 subtraction per entry while the next tile's MMAs run.
 //
 // Why: with both operands in shared memory an MMA of 128 x 64 took 91 clocks
-// and one of 128 x 128 took 165 (operand reads), a tile's 112 MMAs more than
-// its epilogue; and with all of shared memory taken by operands the epilogue's
+// and one of 128 x 128 took 165 (operand reads), a tile's MMAs more than its
+// epilogue; and with all of shared memory taken by operands the epilogue's
 // register spills went to L2.  The epilogue's floor is the FP64 pipe: 8192
 // subtractions a tile at two per clock.
 constexpr int GEMM_THREADS = 576, GEMM_EPI = GEMM_THREADS - 64, EPI_COLS = 16;
