@@ -516,29 +516,6 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return sh[32];
 }
 
-__device__ __forceinline__ double2 block_sum2(double2 v, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-    }
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) { sh[2 * w] = v.x; sh[2 * w + 1] = v.y; }
-    __syncthreads();
-    if (w == 0) {
-        int nw = blockDim.x >> 5;
-        v.x = l < nw ? sh[2 * l] : 0.0;
-        v.y = l < nw ? sh[2 * l + 1] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-            v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-        }
-        if (l == 0) { sh[64] = v.x; sh[65] = v.y; }
-    }
-    __syncthreads();
-    return make_double2(sh[64], sh[65]);
-}
-
 __device__ double vec_norm(const double2* v, int64_t n, double* sh) {
     double s = 0;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += v[i].x * v[i].x + v[i].y * v[i].y;

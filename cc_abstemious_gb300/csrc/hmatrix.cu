@@ -156,12 +156,6 @@ __device__ __forceinline__ double bsum(double v, double* sh) {
     return sh[40];
 }
 
-__device__ __forceinline__ z2 bsum2(z2 v, double* sh) {
-    double a = bsum(v.x, sh);
-    double b = bsum(v.y, sh);
-    return make_double2(a, b);
-}
-
 // Sum of a complex value over the 32 lanes of a warp (every lane gets it).
 // The parts part ways in the first step: five FP64 additions, not ten (each
 // occupies the FP64 pipe of the SM quarter for 65 clocks).
