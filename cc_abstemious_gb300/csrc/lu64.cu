@@ -356,12 +356,13 @@ __global__ void __launch_bounds__(PANEL_THREADS, 1)
             mblk.exchange(sh + j, sh + p, lane);
         }
     }
-    if (warp == 0 && rank == 0 && lane < w) pinv[c0 - b0 + lane] = sinv[lane];
     if (!worker && rank == 0) {
         mown.store(&own, lane);
         mblk.store(moves, lane);
     }
     cl.sync();
+    // (behind the barrier: the last column's reciprocal is thread 0's)
+    if (warp == 0 && rank == 0 && lane < w) pinv[c0 - b0 + lane] = sinv[lane];
     if (worker) {
         // the factored panel, and the largest entry of each column of L21
         const int below = (int)(b0 + nb - c0) - row0;

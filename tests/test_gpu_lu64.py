@@ -75,3 +75,13 @@ def test_non_finite_entries_end_in_non_finite_results(value):
     assert not np.all(np.isfinite(x))
     A, b = matrix(150, 2)
     assert backward(A, bem.solve_lu(A, b), b) <= 16 * 158 * U
+
+
+@pytest.mark.parametrize("n", [2, 31, 33, 95, 545, 1057])
+def test_repeated_solves_are_bit_identical(n):
+    """The panels' CTAs and warps hand results to one another; every hand-over has
+    its barrier, so that a solve does not depend on which of them is ahead."""
+    A, b = matrix(n, 5 * n)
+    x = bem.solve_lu(A, b)
+    for _ in range(10):
+        assert np.array_equal(bem.solve_lu(A, b), x)
