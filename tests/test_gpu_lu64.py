@@ -85,3 +85,63 @@ def test_repeated_solves_are_bit_identical(n):
     x = bem.solve_lu(A, b)
     for _ in range(10):
         assert np.array_equal(bem.solve_lu(A, b), x)
+
+
+def rowwise(A, x, b):
+    """Largest |b - A x|_i / (|A| |x|)_i, which for partial pivoting is a small
+    multiple of n u whatever the scale of row i or of the columns."""
+    return float(np.max(np.abs(A @ x - b) / (np.abs(A) @ np.abs(x))))
+
+
+@pytest.mark.parametrize("scale", [1e6, 1e9, 1e12])
+@pytest.mark.parametrize("count", [1, 15, 17, 24, 31, 56])
+@pytest.mark.parametrize("n", [300, 1100, 2100])
+def test_a_few_rows_of_another_scale(n, count, scale):
+    """The large rows are the first pivots and end inside a block; where its panels
+    are narrower than it, the rows exchanged by a later panel leave the columns
+    of an earlier one small."""
+    A, b = matrix(n, n + count)
+    rows = np.random.default_rng(count).permutation(n)[:count]
+    A[rows] *= scale
+    b[rows] *= scale
+    assert rowwise(A, bem.solve_lu(A, b), b) <= 16 * (n + 8) * U
+
+
+@pytest.mark.parametrize("count", [17, 24, 56])
+@pytest.mark.parametrize("n", [300, 1100, 2100])
+def test_a_few_columns_of_another_scale(n, count):
+    A, b = matrix(n, 2 * n + count)
+    A[:, np.random.default_rng(count).permutation(n)[:count]] *= 1e9
+    assert rowwise(A, bem.solve_lu(A, b), b) <= 16 * (n + 8) * U
+
+
+@pytest.mark.parametrize("n", [300, 1100, 1500])
+def test_rows_over_many_decades(n):
+    A, b = matrix(n, n + 5)
+    d = 10.0 ** np.random.default_rng(n).uniform(-9, 9, n)
+    A, b = d[:, None] * A, d * b
+    assert rowwise(A, bem.solve_lu(A, b), b) <= 16 * (n + 8) * U
+
+
+@pytest.mark.parametrize("n", [12833, 25665])
+def test_panels_of_eight_and_of_four_columns(n):
+    """Above 12800 and 25600 rows the cluster's shared memory holds panels of 8 and
+    of 4 columns; twenty-four rows a billion times the others, as above."""
+    import torch
+    ctx = bem.Context()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    At = torch.randn(n, n, dtype=torch.complex128, device="cuda", generator=g)  # its transpose, column-major
+    b = torch.randn(n, dtype=torch.complex128, device="cuda", generator=g)
+    rows = torch.randperm(n, device="cuda", generator=g)[:24]
+    At[:, rows] *= 1e9
+    b[rows] *= 1e9
+    x = b.clone()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.bem_solve_lu(ctx.h, n, At.data_ptr(), n, x.data_ptr(), 1))
+    size = torch.empty(n, dtype=torch.float64, device="cuda")
+    for i in range(0, n, 2048):
+        size[i:i + 2048] = x.abs() @ At[:, i:i + 2048].abs()
+    r = ((x @ At - b).abs() / size).max().item()
+    del At, size, ctx
+    torch.cuda.empty_cache()
+    assert r <= 16 * (n + 8) * U
