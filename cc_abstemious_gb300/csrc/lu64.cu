@@ -75,8 +75,9 @@ constexpr int TM = 128;       // tile rows (real): 64 complex rows
 constexpr int TN = 64;        // tile columns
 constexpr uint32_t A_SLICE = TM * 128, B_SLICE = TN * 128;  // 64 halves = 128 bytes per row
 constexpr uint32_t A_IMG = SLICES * A_SLICE, B_IMG = SLICES * B_SLICE;
-constexpr int EXP_NONE = -(1 << 20);  // exponent of zero
-constexpr int EXP_BAD = 1 << 20;      // row or column with an infinity or a NaN
+constexpr int EXP_NONE = -(1 << 20);  // exponent of zero; the sum of any two exponents
+// with an EXP_BAD among them is far outside the range of numbers
+constexpr int EXP_BAD = 1 << 22;      // row or column with an infinity or a NaN
 
 // ---------------------------------------------------------------------------
 // Row exchanges of one block (or of one panel): position top0 + t (t < 32)

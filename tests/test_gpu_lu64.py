@@ -145,3 +145,19 @@ def test_panels_of_eight_and_of_four_columns(n):
     del At, size, ctx
     torch.cuda.empty_cache()
     assert r <= 16 * (n + 8) * U
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1j * np.inf])
+@pytest.mark.parametrize("first,last", [(40, 41), (40, 44), (92, 96), (32, 96)])
+def test_zeros_of_l21_meet_non_finite_columns_of_u12(first, last, value):
+    """0 x infinity is NaN in elimination: rows of L21 that are zero throughout carry
+    it into the trailing matrix, and from there into every unknown (four columns at
+    a time in the kernel: alone, in a whole group of four, everywhere)."""
+    A, b = matrix(96, 9)
+    A[32:, :32] = 0
+    A[3, first:last] = value
+    try:
+        x = bem.solve_lu(A, b)
+    except bem.BemError:
+        return
+    assert not np.isfinite(x).any()
