@@ -347,6 +347,10 @@ __global__ void __launch_bounds__(ACA_THREADS, 4) hm_aca_kernel(HLeaf* __restric
             if (threadIdx.x == 0) atomicOr(err, 8);
             break;
         }
+        // (read here, barriers ahead of the updates below: a warp that read them
+        // there could find thread 0's new ones, take the other branch and part
+        // ways with the rest of the CTA)
+        const int64_t iref = s_iref, jref = s_jref;
         double jval, ival, unused;
         int64_t jstar = bargmax_excl(riref, jex, n, sh, shi, jval);
         int64_t istar = bargmax_excl(rjref, iex, m, sh, shi, ival);
@@ -416,9 +420,9 @@ __global__ void __launch_bounds__(ACA_THREADS, 4) hm_aca_kernel(HLeaf* __restric
         __syncthreads();
         if (s_stop) break;
         // reference row / column updates
-        if (s_iref == istar) {
+        if (iref == istar) {
             if (threadIdx.x == 0) {
-                int64_t v = s_iref;
+                int64_t v = iref;
                 if (iex[v]) {
                     v = rng_uniform_incl(rng, (uint32_t)(nr - 1));
                     for (int64_t t = 0; t < nr - 1; ++t) {
@@ -431,13 +435,13 @@ __global__ void __launch_bounds__(ACA_THREADS, 4) hm_aca_kernel(HLeaf* __restric
             __syncthreads();
             aca_res_row(g, L, rows, cols, U, V, rank, s_iref, riref);
         } else {
-            const z2 c = uk[s_iref];
+            const z2 c = uk[iref];
             for (int64_t t = threadIdx.x; t < n; t += blockDim.x) cfma(riref[t], cneg(c), vk[t]);
             __syncthreads();
         }
-        if (s_jref == jstar) {
+        if (jref == jstar) {
             if (threadIdx.x == 0) {
-                int64_t v = s_jref;
+                int64_t v = jref;
                 if (jex[v]) {
                     v = rng_uniform_incl(rng, (uint32_t)(nr - 1));
                     for (int64_t t = 0; t < nr - 1; ++t) {
@@ -450,7 +454,7 @@ __global__ void __launch_bounds__(ACA_THREADS, 4) hm_aca_kernel(HLeaf* __restric
             __syncthreads();
             aca_res_col(g, L, rows, cols, U, V, rank, s_jref, rjref);
         } else {
-            const z2 c = vk[s_jref];
+            const z2 c = vk[jref];
             for (int64_t t = threadIdx.x; t < m; t += blockDim.x) cfma(rjref[t], cneg(c), uk[t]);
             __syncthreads();
         }
