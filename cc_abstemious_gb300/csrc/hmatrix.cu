@@ -625,8 +625,10 @@ __device__ void jacobi_dev(double2* M, int r, double* S, int* perm, int lead) {
     __shared__ double s_n[ACA_RMAX];  // squared norms of the columns
     if (warp < warps) {
         auto together = [&]() {
-            if (warps == 1) __syncwarp();
-            else asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
+            // (a warp whose pairs have not all turned comes here in parts; the
+            // barrier wants it whole)
+            __syncwarp();
+            if (warps > 1) asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
         };
         const int per = 32 / lpp, groups = per * warps, first = lane / lpp * lpp;
         const int grp = lane < per * lpp ? warp * per + lane / lpp : 1 << 20, g = lane - first;

@@ -1,11 +1,15 @@
 """Building an H-matrix (csrc/hmatrix.cu): pivots of the compression, recompression."""
+import tempfile
+
 import numpy as np
 import pytest
 
 from conftest import sphere_input
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 bem = pytest.importorskip("cc_abstemious_gb300")
+from cc_abstemious_gb300 import workloads  # noqa: E402
 
 
 def test_repeated_builds_are_bit_identical():
@@ -23,3 +27,39 @@ def test_repeated_builds_are_bit_identical():
         got = (H.stats(), H.gemv(0.7 - 0.2j, x, 0.3 + 0.1j, b))
         first = first or got
         assert got[0] == first[0] and np.array_equal(got[1], first[1])
+
+
+@pytest.mark.parametrize("n,ka,leaf,eta,tol,ranks", [
+    (500, 1.0, 30, 4.0, 1e-6, [12, 13, 20, 21, 29]),
+    (900, 2.0, 33, 2.0, 1e-8, [23, 24, 25, 26, 31, 32, 33, 34]),   # both sides of 24 and of 32
+    (700, 6.0, 40, 4.0, 1e-10, [15, 28, 32, 42, 49]),
+    (700, 3.0, 60, 4.0, 1e-13, [29, 30, 47, 49]),                   # leaves of full rank, down to rounding
+    (1400, 15.0, 150, 6.0, 1e-9, [61, 83, 84, 90]),                 # above 64, odd and even
+])
+def test_compressed_leaves(n, ka, leaf, eta, tol, ranks):
+    """Every compressed leaf against its dense block and the ranks against the oracle's,
+    at the ranks where the recompression takes other numbers of warps (24 / 25, 32 / 33),
+    device instead of shared memory (32 / 33) and a bye in its pairing (odd ranks).
+
+    The iteration ends at steps of tol / 50; what the truncation drops are singular
+    values below tol times the sum of the larger ones, at most r of them: within
+    (4 + r) tol of the block's norm."""
+    inp = workloads.perturbed_sphere_input(tempfile.mkdtemp(prefix="bem_hb_"), 3, n, [ka])
+    inp["solver"] = {"Hierarchical": {"tolerance": 1e-6, "max_iterations": 1000, "leaf_size": leaf, "eta": eta,
+                                      "aca_tolerance": tol}}
+    P = O.Problem(inp)
+    H, G = P.dense_surface()
+    al, be = P.lhs_factors()
+    A = al * H + be * G
+    pd = bem.PreData.from_dict(inp, ctx=bem.Context.default())
+    built = bem.HMatrix(pd, bem.EqnSide.LHS)
+    F, bl = built.to_full(), O.block_list(P.cpts, leaf, eta)
+    seen = []
+    for i in np.flatnonzero(bl["admissible"]):
+        ix = np.ix_(bl["rows"][bl["row_off"][i]:bl["row_off"][i + 1]], bl["cols"][bl["col_off"][i]:bl["col_off"][i + 1]])
+        r = O.aca(A[ix], tol)[0].shape[1]
+        seen.append(r)
+        assert np.linalg.norm(F[ix] - A[ix]) <= (4 + r) * tol * np.linalg.norm(A[ix])
+    assert built.stats()["admissible"] == len(seen)
+    assert abs(built.stats()["rank_sum"] - sum(seen)) <= max(2, sum(seen) // 200)
+    assert set(ranks) <= set(seen)
