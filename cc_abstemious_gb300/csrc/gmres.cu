@@ -1033,7 +1033,8 @@ __global__ void __launch_bounds__(MG_THREADS) gm_arnoldi_kernel(GmBatch bt, int 
         for (int l = tid; l < rows; l += MG_THREADS) qk1[l] = make_double2(w[l].x * sc, w[l].y * sc);
         if (*t.chk) gm_add_correction(bt, g, t.y, k, l0, l1);
     }
-    if (!ok && tid == 0) {  // a wait ran out: the system ends as not converged
+    if (!ok && tid == 0) {  // a wait ran out: the system ends here, gm_require_waits reports it
+        st.gave_up = 1;
         st.done = 1;
         __threadfence();
     }
@@ -1122,6 +1123,7 @@ __global__ void gm_init_kernel(GmBatch bt, const double* anorm, double tol, int6
         st.check = 0;
         st.done = 0;
         st.converged = 0;
+        st.gave_up = 0;
         st.num_mv = 0;
         st.iterations = 0;
         st.restarts = 0;
@@ -1578,6 +1580,7 @@ void gm_read_states(Context& ctx, GmWorkspace& ws, std::vector<GmState>& out) {
     out.resize(ws.bt.nsys);
     BEM_CUDA(cudaMemcpyAsync(out.data(), ws.bt.st, sizeof(GmState) * ws.bt.nsys, cudaMemcpyDeviceToHost, ctx.stream));
     ctx.sync();
+    gm_require_waits(out.data(), out.size());
 }
 
 // One iteration at a time; the Krylov mat-vec of every iteration is timed with

@@ -9,8 +9,16 @@ enum { MV_START = 0, MV_Q = 1, MV_CHECK = 2 };
 struct GmState {
     double anorm, bnorm, tol, xnorm, error;
     int k, need_start, check, done, converged, m;  // m: this system's restart length (<= batch m)
+    int gave_up;  // a bounded wait of one of its kernels ran out (done is set with it)
     long long num_mv, iterations, restarts, max_restarts;
 };
+
+// A wait that ran out is a failure of the device, not of the iteration.
+inline void gm_require_waits(const GmState* st, size_t count) {
+    for (size_t s = 0; s < count; ++s)
+        require(!st[s].gave_up, "a bounded device-side wait gave up (GMRES, system " + std::to_string(s) + ")",
+                BEM_ERR_TIMEOUT);
+}
 
 // Per-system layout of a ragged batch (systems of different sizes).
 struct GmSys {

@@ -89,6 +89,7 @@ BEM_API bem_status bem_gmres_solve_noalloc(bem_ctx* ctx, int64_t n, const bem_cp
             BEM_CUDA(cudaStreamSynchronize(c.stream));
             if (st.done) break;
         }
+        gm_require_waits(&st, 1);
         BEM_CUDA(cudaMemcpyAsync(x, ws.bt.X, sizeof(double2) * n, cudaMemcpyDeviceToDevice, c.stream));
         BEM_CUDA(cudaStreamSynchronize(c.stream));
         if (report) {
