@@ -1350,16 +1350,7 @@ void gm_prepare_ragged(Context& ctx, GmWorkspace& ws, const std::vector<int64_t>
         npmax = std::max(npmax, d.n_pad);
     }
     BEM_CUDA(cudaDeviceGetAttribute(&ws.sms, cudaDevAttrMultiProcessorCount, ctx.device));
-    // systems in pairs where they share an operator
-    int mates = 0;
-    for (int s = 0; s < nsys; ++s) sys[s].mate = -1;
-    for (int s = 0; s < nsys; ++s)
-        for (int o = s + 1; o < nsys && sys[s].mate < 0; ++o)
-            if (sys[o].mate < 0 && sys[o].a_off == sys[s].a_off && sys[o].n == sys[s].n && sys[o].lda == sys[s].lda) {
-                sys[s].mate = o;
-                sys[o].mate = s;
-                mates = 1;
-            }
+    const int mates = gm_pair_systems(sys);
     GmBatch& bt = ws.bt;
     bt.mates = mates;
     bt.nsys = nsys;

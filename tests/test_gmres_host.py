@@ -43,3 +43,52 @@ def reported(tmp_path_factory):
 def test_a_wait_that_ran_out_is_not_reported_as_non_convergence(reported, states, status):
     """c: converged, n: out of iterations, w: a kernel's wait gave up (BEM_ERR_TIMEOUT = 7)."""
     assert reported(*states) == [str(status)]
+
+
+@pytest.fixture(scope="module")
+def pairs(tmp_path_factory):
+    """argv: the systems' operators as 'offset,n,lda'; or 'time', their number and how
+    many of them share one operator: prints milliseconds."""
+    return compiled(tmp_path_factory.mktemp("pairs"), """
+    const bool time = argc > 1 && argv[1][0] == 't';
+    std::vector<GmSys> sys((size_t)(time ? atoi(argv[2]) : argc - 1));
+    for (size_t s = 0; s < sys.size(); ++s) {
+        long long off = 0, n = 100, ld = 128;
+        if (time) off = (long long)(s / (size_t)atoi(argv[3])) * 12800;
+        else sscanf(argv[s + 1], "%lld,%lld,%lld", &off, &n, &ld);
+        sys[s].a_off = (size_t)off;
+        sys[s].n = n;
+        sys[s].lda = ld;
+    }
+    const auto t0 = std::chrono::steady_clock::now();
+    const int any = gm_pair_systems(sys);
+    const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (time) return 0 * printf("%f", ms);
+    printf("%d", any);
+    for (const GmSys& d : sys) printf(" %d", d.mate);""")
+
+
+def reference_pairs(systems):
+    """The first later system with the same operator that has no mate yet."""
+    mate = [-1] * len(systems)
+    for s in range(len(systems)):
+        for o in range(s + 1, len(systems)):
+            if mate[s] < 0 and mate[o] < 0 and systems[s] == systems[o]:
+                mate[s], mate[o] = o, s
+    return mate
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_pairs_of_systems_that_share_an_operator(pairs, seed):
+    import random
+    rng = random.Random(seed)
+    systems = [(rng.randrange(1 + seed) * 640, 100 + rng.randrange(2), 128) for _ in range(rng.randrange(1, 40))]
+    mate = reference_pairs(systems)
+    assert pairs(*["%d,%d,%d" % s for s in systems]) == [str(v) for v in [int(max(mate) >= 0)] + mate]
+
+
+@pytest.mark.parametrize("share", [1, 3, 20000])
+def test_pairing_of_many_systems_is_not_quadratic(pairs, share):
+    """20000 systems: every one against every other takes 200 million comparisons, a
+    third of a second."""
+    assert min(float(pairs("time", 20000, share)[0]) for _ in range(3)) < 60
