@@ -34,4 +34,15 @@ __host__ __device__ __forceinline__ c2 fmul(c2 a, c2 b) {
 }
 __host__ __device__ __forceinline__ c2 fscale(c2 a, float s) { return make_float2(a.x * s, a.y * s); }
 
+// Sum over eight lanes, the parts in the first two of them (they part ways in the
+// first step: three additions).
+__device__ __forceinline__ double sum8_parts(z2 v) {
+    const bool odd = threadIdx.x & 1;
+    double s = odd ? v.y : v.x;
+    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    return s;
+}
+
 }  // namespace bem

@@ -4,16 +4,17 @@
 //
 // One iteration is the fixed launch sequence
 //   [precondition] -> apply(Q) -> Gram-Schmidt and rotations -> apply(CHECK) -> check
-// after one apply(START) -> start, where every kernel reads the per-system state and returns immediately when
-// it has nothing to do.  The host therefore launches ahead of the device, which
-// tells it when every system is done.
+// after one start (with an apply(START) before it in the reference form), where
+// every kernel reads the per-system state and returns immediately when it has
+// nothing to do.  The host therefore launches ahead of the device, which tells it
+// when every system is done.
 //
 // Operator: FP64 matrix (plain form, bit-for-bit the reference arithmetic up
 // to summation order) or FP32 matrix with FP64 vectors and compensated
 // products/sums (mixed form).  Arnoldi, Givens rotations, the small
 // triangular solve and the stopping test are FP64: the reference form keeps
-// its single-CTA modified Gram-Schmidt, the mixed and refined forms
-// orthogonalise across the whole GPU (classical Gram-Schmidt twice).
+// modified Gram-Schmidt, on one thread-block cluster per system, the mixed and
+// refined forms orthogonalise across the whole GPU (classical Gram-Schmidt twice).
 #include <mutex>
 
 #include "cluster.cuh"
@@ -34,13 +35,6 @@ constexpr int TICKETS = MV_ROWS / SMALL_ROWS;
 constexpr int AR_THREADS = 1024;
 // dynamic shared memory of the Arnoldi kernels
 constexpr size_t AR_SMEM_CAP = 200 * 1024;
-
-__device__ __forceinline__ bool mv_active(const GmState& s, int mode) {
-    if (s.done) return false;
-    if (mode == MV_START) return s.need_start != 0;
-    if (mode == MV_Q) return s.need_start == 0 && s.check == 0;
-    return s.check != 0;  // MV_CHECK
-}
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
@@ -106,14 +100,11 @@ __global__ void __launch_bounds__(MV_THREADS) gm_apply_kernel(GmBatch bt, int mo
         by = blockIdx.y;
     }
     GmState& st = bt.st[s];
-    if (!mv_active(st, mode)) return;
-    // outside the reference-faithful mode the first cycle starts from x = 0,
-    // so its residual is b itself: no product needed
-    if (mode == MV_START && !bt.ref_dotc && st.restarts == 0) return;
+    if (!gm_apply_active(st, mode)) return;
     int s2 = -1;
     if (NV == 2) {
         const int mate = bt.sys[s].mate;
-        if (mate >= 0 && mv_active(bt.st[mate], mode)) {
+        if (mate >= 0 && gm_apply_active(bt.st[mate], mode)) {
             if (mate < s) return;  // the mate's CTA does both
             s2 = mate;
         }
@@ -328,7 +319,7 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) gm_apply_small_kernel(GmBatc
         bx = blockIdx.x;
         by = blockIdx.y;
     }
-    if (!gm_apply_active(bt, bt.st[s], mode)) return;
+    if (!gm_apply_active(bt.st[s], mode)) return;
     const GmView g = gm_view(bt, s);
     const int64_t n = g.n, lda = g.lda;
     const double2* kv = bt.Z ? bt.Z : bt.Q;
@@ -542,7 +533,7 @@ __global__ void __launch_bounds__(AR_THREADS) gm_start_kernel(GmBatch bt) {
     const double2* b = bt.B + g.v;
     const double2* W = bt.W + g.v;
     double2* Q = bt.Q + g.q;
-    const bool zero_x = !bt.ref_dotc && st.restarts == 0;  // x = 0: A x not formed
+    const bool zero_x = !bt.ref_dotc;  // x = 0, and the reference's A x is not formed
     double acc = 0;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
         double2 r = zero_x ? b[i] : csub(b[i], W[i]);
@@ -587,14 +578,9 @@ __device__ __forceinline__ bool gm_arnoldi_active(const GmState& st) {
     return !(st.done || st.need_start || st.check);
 }
 
-// Sum over the eight lanes of a group (every lane gets it): the parts part ways
-// in the first step, three additions.
+// Sum over the eight lanes of a group; every lane gets it.
 __device__ __forceinline__ double2 sum8(double2 v) {
-    const bool odd = threadIdx.x & 1;
-    double s = odd ? v.y : v.x;
-    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    const double s = sum8_parts(v);
     const int base = threadIdx.x & 24;
     return make_double2(__shfl_sync(0xffffffffu, s, base), __shfl_sync(0xffffffffu, s, base + 1));
 }
@@ -1298,7 +1284,7 @@ size_t gm_prepare_external(Context& ctx, GmWorkspace& ws, int nsys, int64_t n, i
     bt.X = reinterpret_cast<double2*>(base + oX);
     bt.B = reinterpret_cast<double2*>(base + oB);
     bt.Q = reinterpret_cast<double2*>(base + oQ);
-    bt.gs_part = nullptr;  // caller memory: the single-CTA Gram-Schmidt
+    bt.gs_part = nullptr;  // (the reference form only)
     bt.gs_norm = nullptr;
     bt.gs_chunks = 0;
     bt.W = reinterpret_cast<double2*>(base + oW);
@@ -1467,22 +1453,20 @@ void gm_init_each(Context& ctx, GmWorkspace& ws, const std::vector<double>& tol,
     ctx.sync();  // the host arrays are pageable and owned by the caller
 }
 
-// Finer tiles where they were the faster ones.  FP64: at every size (us per
-// product, wide -> finer: n = 2048 263 -> 39, 6144 312 -> 269, 16384 1820 -> 1749;
-// the wide tiles remain for caller-provided memory, which has no room for the
-// tickets).  FP32: below 1.5 wide tiles per SM (Krylov products, us of eight, wide ->
-// finer: 36 tiles 295 -> 92, 144 384 -> 373, 196 751 -> 568, 288 822 -> 870, 1152
-// 2447 -> 3069; beyond, memory bounds them and the longer columns of the wide
-// tiles read it better).
-
 static void launch_apply(Context& ctx, GmWorkspace& ws, int mode) {
     if (ws.hook) {
         ws.hook(ctx, ws, mode, ws.hook_user);
         return;
     }
     const GmBatch& bt = ws.bt;
-    // (hooks and launches alike read the sizes from ws.bt: the same for every
-    // mode of a solve, so the three modes sum in one order)
+    // Finer tiles where they were the faster ones.  FP64: at every size (us per
+    // product, wide -> finer: n = 2048 263 -> 39, 6144 312 -> 269, 16384 1820 ->
+    // 1749; the wide tiles remain for caller-provided memory, which has no room for
+    // the tickets).  FP32: below 1.5 wide tiles per SM (Krylov products, us of eight,
+    // wide -> finer: 36 tiles 295 -> 92, 144 384 -> 373, 196 751 -> 568, 288 822 ->
+    // 870, 1152 2447 -> 3069; beyond, memory bounds them and the longer columns of
+    // the wide tiles read it better).  One choice for all products of a solve, so
+    // that they sum in one order.
     const int64_t tiles = bt.sys ? bt.ntiles : (int64_t)ws.rb * ws.cb * bt.nsys;
     const bool small = bt.tpr == TICKETS && (!ws.fp32 || 2 * tiles < 3 * ws.sms);
     const dim3 grid = bt.sys ? dim3((unsigned)(small ? bt.ntiles64 : bt.ntiles))

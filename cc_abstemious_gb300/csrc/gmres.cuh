@@ -77,9 +77,8 @@ struct GmBatch {
     double2* small;     // per-system Hessenberg / rotations
     GmState* st;
     double2* Z;         // flexible right preconditioning: Z[:, k] = M Q[:, k] (nullptr: none)
-    // Gram-Schmidt of the mixed / refined forms across the whole GPU (null:
-    // the single-CTA modified Gram-Schmidt of the reference form): per system,
-    // partial dot products of every row chunk with the basis (gs_chunks x
+    // Gram-Schmidt of the mixed / refined forms across the whole GPU (null: the
+    // reference form's, on a cluster per system): per system, partial dot products of every row chunk with the basis (gs_chunks x
     // (m + 1)) and partial squared norms (gs_chunks)
     double2* gs_part = nullptr;
     double* gs_norm = nullptr;
@@ -96,9 +95,9 @@ struct GmBatch {
 };
 
 // Whether the operator application of `mode` has work for a system.
-__device__ __forceinline__ bool gm_apply_active(const GmBatch& bt, const GmState& s, int mode) {
+__device__ __forceinline__ bool gm_apply_active(const GmState& s, int mode) {
     if (s.done) return false;
-    if (mode == MV_START) return s.need_start != 0 && !(!bt.ref_dotc && s.restarts == 0);
+    if (mode == MV_START) return s.need_start != 0;  // (the reference form only)
     if (mode == MV_Q) return s.need_start == 0 && s.check == 0;
     return s.check != 0;  // MV_CHECK
 }

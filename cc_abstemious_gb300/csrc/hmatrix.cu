@@ -843,16 +843,6 @@ __global__ void hm_dense_norm_kernel(HLeaf* __restrict__ leaves, const int32_t* 
 // products alone take 173 us; now 276 us.)
 constexpr int HMV_THREADS = 128, HMV_WARPS = HMV_THREADS / 32, HMV_CHUNK = 512;
 
-// Sum over eight lanes, the parts in the first two of them.
-__device__ __forceinline__ double sum8_parts(double2 v) {
-    const bool odd = threadIdx.x & 1;
-    double s = odd ? v.y : v.x;
-    s += __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    return s;
-}
-
 // out[i] (+)= sum over k < nc of M[k m + i] c[k], M column-major in device
 // memory, c and `part` (HMV_THREADS entries) in shared memory; the whole CTA.
 __device__ __forceinline__ void leaf_columns(const double2* __restrict__ M, int64_t m, int nc, const double2* c,
@@ -900,7 +890,7 @@ __global__ void __launch_bounds__(HMV_THREADS) hm_leaf_mv_kernel(const HLeaf* __
     const double2* x = xin;
     if (bt.st) {
         const GmState& st = bt.st[0];
-        if (!gm_apply_active(bt, st, mode)) return;
+        if (!gm_apply_active(st, mode)) return;
         x = (mode == MV_Q) ? bt.Q + (size_t)st.k * bt.n : bt.X;
     }
     const HLeaf L = leaves[order[blockIdx.x]];
@@ -970,7 +960,7 @@ __global__ void __launch_bounds__(ROW_THREADS) hm_row_reduce_kernel(int64_t n, c
                                                                     int mode, z2 beta, double2* __restrict__ out) {
     if (bt.st) {
         const GmState& st = bt.st[0];
-        if (!gm_apply_active(bt, st, mode)) return;
+        if (!gm_apply_active(st, mode)) return;
     }
     const int64_t i = (blockIdx.x * (int64_t)ROW_THREADS + threadIdx.x) / ROW_LANES;
     const int l8 = threadIdx.x & (ROW_LANES - 1);

@@ -190,7 +190,7 @@ __device__ __forceinline__ const double2* hm_operand(const GmBatch& bt, const Gm
 __global__ void hmx_gather_kernel(HmDev h, GmBatch bt, int mode) {
     const int s = blockIdx.y;
     const GmState& st = bt.st[s];
-    if (!gm_apply_active(bt, st, mode)) return;
+    if (!gm_apply_active(st, mode)) return;
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= h.n) return;
     const double2 x = hm_operand(bt, st, s, mode)[h.perm[q]];
@@ -207,7 +207,7 @@ constexpr int PJ_WARPS = 8;
 template <int EXACT>
 __global__ void __launch_bounds__(PJ_WARPS * 32) hmx_project_kernel(HmDev h, GmBatch bt, int mode) {
     const int s = blockIdx.y;
-    if (!gm_apply_active(bt, bt.st[s], mode)) return;
+    if (!gm_apply_active(bt.st[s], mode)) return;
     const int op = s / h.R;
     const int64_t q = (int64_t)blockIdx.x * PJ_WARPS + (threadIdx.x >> 5);
     if (q >= h.nproj[op]) return;
@@ -244,7 +244,7 @@ constexpr int RW_ROWS = 64, RW_WARPS = 8, RW_THREADS = RW_WARPS * 32;
 template <int EXACT>
 __global__ void __launch_bounds__(RW_THREADS) hmx_rows_kernel(HmDev h, GmBatch bt, int mode) {
     const int s = blockIdx.y;
-    if (!gm_apply_active(bt, bt.st[s], mode)) return;
+    if (!gm_apply_active(bt.st[s], mode)) return;
     __shared__ float4 red[RW_WARPS][RW_ROWS];
     const int64_t ch = blockIdx.x;
     const int rc = h.ch_rc[ch], op = s / h.R;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(RW_THREADS) hmx_rows_kernel(HmDev h, GmBatch b
 // W[rows of cluster rc] = the cluster's chunk partials, added in chunk order.
 __global__ void __launch_bounds__(RW_ROWS) hmx_reduce_kernel(HmDev h, GmBatch bt, int mode) {
     const int s = blockIdx.y;
-    if (!gm_apply_active(bt, bt.st[s], mode)) return;
+    if (!gm_apply_active(bt.st[s], mode)) return;
     const int rc = blockIdx.x, i = threadIdx.x;
     const int64_t rs = h.rc_start[rc];
     if (i >= (int)(h.rc_start[rc + 1] - rs)) return;
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(256) hmx_bj_invert_kernel(HmDev h, const int32
 __global__ void __launch_bounds__(BJ_MAX) hmx_bj_apply_kernel(HmDev h, const float2* __restrict__ Minv, GmBatch bt) {
     const int s = blockIdx.y, rc = blockIdx.x;
     const GmState& st = bt.st[s];
-    if (!gm_apply_active(bt, st, MV_Q)) return;
+    if (!gm_apply_active(st, MV_Q)) return;
     __shared__ double2 qs[BJ_MAX];
     const GmView g = gm_view(bt, s);
     const double2* qv = bt.Q + g.q + (size_t)st.k * g.n;

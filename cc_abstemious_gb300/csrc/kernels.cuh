@@ -41,6 +41,12 @@ __device__ __forceinline__ double wide(float f) {
     const int b = __float_as_int(f);
     return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + ((1023 - 127) << 20)), b << 29);
 }
+// Any float: by the conversion where the exponent is that of zero, a subnormal, an
+// infinity or a NaN.
+__device__ __forceinline__ double wide_any(float f) {
+    const unsigned e = (__float_as_uint(f) >> 23) & 0xff;
+    return e == 0 || e == 0xff ? (double)f : wide(f);
+}
 
 // inv = 1 / sqrt(v) and root = sqrt(v): the FP32 seed and one third-order
 // correction shared by both, seven FP64 instructions (a square root and a

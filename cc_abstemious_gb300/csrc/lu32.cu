@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(TS_THREADS, R == TS_MAXR ? 1 : 2) lu_trsv_kern
             qr[r] = nullptr;
             if (r < T.nrhs) {
                 const GmState& st = bt.st[T.sys + r];
-                act[r] = gm_apply_active(bt, st, MV_Q);
+                act[r] = gm_apply_active(st, MV_Q);
                 const GmView g = gm_view(bt, T.sys + r);
                 zr[r] = bt.Z + g.q + (size_t)st.k * g.n;
                 qr[r] = bt.Q + g.q + (size_t)st.k * g.n;

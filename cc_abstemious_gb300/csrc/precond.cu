@@ -268,14 +268,6 @@ __global__ void __launch_bounds__(256) pc_diag_inverse_kernel(const T* __restric
 // instructions, now 8).
 constexpr int PC_APPLY_THREADS = 256, PC_APPLY_ROWS = 32;
 
-// A float as a double, without the conversion instruction where it is normal.
-__device__ __forceinline__ double pc_wide(float f) {
-    const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xff;
-    if (e == 0 || e == 0xff) return (double)f;
-    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023 - 127) << 20))),
-                            (int)(b << 29));
-}
-
 __device__ __forceinline__ void pc_block_apply(int c, int half, const int64_t* cl_off, const int64_t* cl_idx,
                                                const int32_t* nb_off, const int32_t* nb_d, const int64_t* nb_blk,
                                                const float2* Ms, const double2* q, double2* z, int use_offdiag) {
@@ -304,7 +296,7 @@ __device__ __forceinline__ void pc_block_apply(int c, int half, const int64_t* c
         const int jn = min(CPW, bd - j0);
 #pragma unroll
         for (int j = 0; j < CPW; ++j)
-            if (j < jn) cfma(acc, make_double2(pc_wide(m[j].x), pc_wide(m[j].y)), qs[warp][j]);
+            if (j < jn) cfma(acc, make_double2(wide_any(m[j].x), wide_any(m[j].y)), qs[warp][j]);
     }
     sums[warp][lane] = acc;
     __syncthreads();
@@ -321,7 +313,7 @@ __device__ __forceinline__ void pc_block_apply(int c, int half, const int64_t* c
 __global__ void __launch_bounds__(PC_APPLY_THREADS) pc_apply_gmres_kernel(PcDev pc, GmBatch bt) {
     const int s = blockIdx.y;
     const GmState& st = bt.st[s];
-    if (!gm_apply_active(bt, st, MV_Q)) return;
+    if (!gm_apply_active(st, MV_Q)) return;
     const int c = pc_leaf(pc, s, blockIdx.x >> 1);
     if (c < 0) return;
     const GmView g = gm_view(bt, s);
