@@ -707,11 +707,7 @@ __device__ void jacobi_dev(double2* M, int r, double* S, int* perm, int lead) {
         if (lane == 0) S[j] = sqrt(v);
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < r; j += blockDim.x) {
-        int at = 0;
-        for (int i = 0; i < r; ++i) at += S[i] > S[j] || (S[i] == S[j] && i < j);
-        perm[at] = j;
-    }
+    for (int j = threadIdx.x; j < r; j += blockDim.x) perm[descending_rank(S, r, j)] = j;
     __syncthreads();
 }
 

@@ -1,10 +1,30 @@
 // Hierarchical matrices: cluster / block trees, ACA and the H-matrix mat-vec.
 #pragma once
+#include <cstring>
 #include <memory>
 
 #include "common.cuh"
 
 namespace bem {
+
+// Place of singular value j among r in descending order, equal ones in theirs.
+// By the bits of the values, which order NaNs too: over all j the places are a
+// permutation for any values (the leaves of an operator with NaNs or with a
+// block of zeros, which has no pivot, end in NaNs).
+__host__ __device__ inline int descending_rank(const double* S, int r, int j) {
+    auto key = [&](int i) {
+        long long b;
+        memcpy(&b, S + i, sizeof(b));
+        return b & 0x7fffffffffffffffll;
+    };
+    const long long kj = key(j);
+    int at = 0;
+    for (int i = 0; i < r; ++i) {
+        const long long ki = key(i);
+        at += ki > kj || (ki == kj && i < j);
+    }
+    return at;
+}
 
 struct HMatrixDev;
 
