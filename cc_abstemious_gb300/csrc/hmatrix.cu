@@ -187,33 +187,35 @@ __device__ __forceinline__ double wsum(double v) {
 // argmax of |v[t]| over t not excluded; first index wins ties (aca.rs:256-268).
 // Moduli (hypot, about 25 FP64 instructions) only of the entries whose square
 // is within a few rounding errors of the largest square, which decides the
-// others.  The winner's is returned beside its index (-1 where there is none).
+// others.  The winner's is returned beside its index.  Where every entry that is
+// not excluded is a NaN, the first of them (modulus -1): the index addresses the
+// leaf's rows and columns and is always one of them.
 __device__ int64_t bargmax_excl(const double2* v, const int8_t* excl, int64_t len, double* sh, int64_t* shi,
                                 double& modulus) {
     const long long inf = 0x7ff0000000000000ll;
-    auto square = [&](int64_t t) {  // as the bits of a non-negative double; -1: excluded or NaN
-        if (excl[t]) return -1ll;
-        const long long k = __double_as_longlong(cnorm2(v[t]));
+    auto square = [&](int64_t t) {  // as the bits of a non-negative double; -1: NaN, -2: excluded
+        if (excl[t]) return -2ll;
+        const long long k = __double_as_longlong(cnorm2(v[t])) & 0x7fffffffffffffffll;
         return k > inf ? -1ll : k;
     };
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    long long top = -1;
+    long long top = -2;
     for (int64_t t = threadIdx.x; t < len; t += blockDim.x) top = max(top, square(t));
     for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
     __syncthreads();
     if (l == 0) shi[w] = top;
     __syncthreads();
-    top = l < nw ? (long long)shi[l] : -1ll;
+    top = l < nw ? (long long)shi[l] : -2ll;
     for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
     // 2^-47 below the largest (zero where squares underflow: every entry)
-    const long long floor_ = top < 0 ? 0 : top < (64ll << 52) ? 0 : top == inf ? inf : top - 64;
+    const long long floor_ = top < 0 ? -1 : top < (64ll << 52) ? 0 : top == inf ? inf : top - 64;
     double best = -1.0;
     int64_t bi = len;
     for (int64_t t = threadIdx.x; t < len; t += blockDim.x) {
         const long long k = square(t);
-        if (k < 0 || k < floor_) continue;
-        const double a = hypot(v[t].x, v[t].y);
-        if (best < a) { best = a; bi = t; }
+        if (k < floor_) continue;
+        const double a = k < 0 ? -1.0 : hypot(v[t].x, v[t].y);
+        if (best < a || bi == len) { best = a; bi = t; }
     }
     for (int o = 16; o > 0; o >>= 1) {
         double ob = __shfl_down_sync(0xffffffffu, best, o);

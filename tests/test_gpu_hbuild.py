@@ -63,3 +63,59 @@ def test_compressed_leaves(n, ka, leaf, eta, tol, ranks):
     assert built.stats()["admissible"] == len(seen)
     assert abs(built.stats()["rank_sum"] - sum(seen)) <= max(2, sum(seen) // 200)
     assert set(ranks) <= set(seen)
+
+
+def flat_box(path, m):
+    """A cube of 6 m^2 quads with flat faces: between two elements of a face the
+    classical kernel's derivative along the normal is exactly zero."""
+    from cc_abstemious_gb300 import meshgen
+    nodes, cells = [], []
+    t = np.linspace(-1.0, 1.0, m + 1)
+    for axis in range(3):
+        for side in (-1.0, 1.0):
+            base = len(nodes)
+            for i in range(m + 1):
+                for j in range(m + 1):
+                    p = np.zeros(3)
+                    p[axis], p[(axis + 1) % 3], p[(axis + 2) % 3] = side, t[i], t[j]
+                    nodes.append(p)
+            for i in range(m):
+                for j in range(m):
+                    q = base + i * (m + 1) + j
+                    c = [q, q + m + 1, q + m + 2, q + 1]
+                    cells.append(c if side > 0 else c[::-1])
+    meshgen.write_vtk(path, np.array(nodes), np.array(cells), 9)
+
+
+@pytest.mark.parametrize("form", ["plain", "mixed"])
+def test_blocks_of_zeros_end_in_no_result_and_nothing_sticks(tmp_path, form):
+    """A block of zeros has no pivot (the reference divides by it and ends in an index
+    out of range): no result is claimed, and the next build is what it was."""
+    good = workloads.perturbed_sphere_input(str(tmp_path), 4, 400, [2.0])
+    good["solver"] = {"Hierarchical": {"tolerance": 1e-6, "max_iterations": 1000, "leaf_size": 8, "eta": 4.0}}
+    path = str(tmp_path / "box.vtk")
+    flat_box(path, 8)
+    flat = workloads.base_input(path, [100.0], method="Classical", solver=good["solver"],
+                                field_points=np.array([[3.0, 0.0, 0.0]]))
+    P = O.Problem(flat)
+    A, bl = P.dense_surface()[0], O.block_list(P.cpts, 8, 4.0)
+    blocks = [np.ix_(bl["rows"][bl["row_off"][i]:bl["row_off"][i + 1]], bl["cols"][bl["col_off"][i]:bl["col_off"][i + 1]])
+              for i in np.flatnonzero(bl["admissible"])]
+    assert any(not A[ix].any() for ix in blocks)
+    ctx = bem.Context.default()
+
+    def solve(inp):
+        a = bem.Analysis(ctx)
+        a.set_input(inp)
+        a.run(form=form)
+        return a.get_result()[0].scattered, a.reports[0]
+
+    first = solve(good)
+    for _ in range(2):
+        try:
+            got, rep = solve(flat)
+        except bem.BemError:
+            continue
+        assert rep["flag"] == 2 or not np.isfinite(got).all()
+    again = solve(good)
+    assert np.array_equal(first[0], again[0]) and again[1]["flag"] == 1
